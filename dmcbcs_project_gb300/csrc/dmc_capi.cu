@@ -122,7 +122,8 @@ struct dmc_ctx {
     dmc_system_desc sd;
     dmc_run_desc rd;
     DevParams P;
-    SmemLayout L;
+    SmemLayout L;           // the mixed walker kernel's layout; it decides the grid
+    SmemLayout L64;         // the FP64 walker kernel's, for the same grid
     int device = 0, nsm = 0, grid = 0, cap = 0, n3 = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -134,6 +135,9 @@ struct dmc_ctx {
     DevBuf<KVecMP> kv_mp;
     DevBuf<TabUDmp> tud_mp;
     DevBuf<TabSSmp> tss_mp;
+    DevBuf<TabPoly> tpoly;          // FP64 walker path: tables by grid interval
+    DevBuf<PhiFix> phi;             // and the pair function's fixed-point coefficients
+    DevBuf<long long> phi_oct;
     int precision = DMC_PREC_FP64;
     DevBuf<unsigned long long> jumpA, jumpC;
     DevBuf<double> gscratch;
@@ -312,6 +316,78 @@ void fill_params(dmc_ctx* c)
     }
 }
 
+// The FP64 walker path's pair function (PhiFix): amplitudes A(n) of the
+// shells' octant vectors, in units of a power of two above the sum of their
+// magnitudes, so that no partial sum leaves the fixed-point range.  A sum
+// that is not finite (an amplitude that is not) makes the units NaN.
+int upload_phi(dmc_ctx* c)
+{
+    const Setup& S = c->S;
+    int n2max = 0, M = 0;
+    for (const KVec& K : S.kv) {
+        n2max = std::max(n2max, K.n[0] * K.n[0] + K.n[1] * K.n[1] + K.n[2] * K.n[2]);
+        for (int k = 0; k < 3; ++k) M = std::max(M, std::abs(K.n[k]));
+    }
+    std::vector<double> a(n2max + 1, 0.0);   // vorb by |n|^2
+    for (const KVec& K : S.kv) a[K.n[0] * K.n[0] + K.n[1] * K.n[1] + K.n[2] * K.n[2]] = S.vorb[K.shell - 1];
+    auto amp = [&](int x, int y, int z) {
+        const int n2 = x * x + y * y + z * z;
+        return n2 > n2max ? 0.0 : a[n2] * (1 << ((x != 0) + (y != 0) + (z != 0)));
+    };
+    double sum = 0.0, suml = 0.0;
+    for (int x = 0; x <= M; ++x)
+        for (int y = 0; y <= M; ++y)
+            for (int z = 0; z <= M; ++z) {
+                sum += std::fabs(amp(x, y, z));
+                suml += (x * x + y * y + z * z) * std::fabs(amp(x, y, z));
+            }
+    auto unit = [](double v) {   // the power of two above v
+        int e = 0;
+        if (!(v > 0.0) || !std::isfinite(v)) return 1.0;
+        std::frexp(v, &e);
+        return std::ldexp(1.0, e);
+    };
+    const double sc = unit(sum), sl = unit(suml), one = 4611686018427387904.0;   // 2^62
+    const bool fin = std::isfinite(sum) && std::isfinite(suml);
+    auto fix = [&](double v, double u) { return fin ? (long long)std::llrint(v / u * one) : 0ll; };
+    PhiFix F;
+    std::memset(&F, 0, sizeof F);
+    F.M = M;
+    while ((1 << F.kM) < M) ++F.kM;
+    F.fast = n2max <= 6;
+    const double kap = 2.0 * 3.14159265358979323846 / S.el;
+    std::vector<long long> oct(1, 0);
+    if (F.fast) {
+        double b[7] = {0, 0, 0, 0, 0, 0, 0};
+        for (int m = 0; m <= n2max; ++m) b[m] = a[m];
+        const double w[7] = {1, 8, 16, 8, 8, 32, 32};   // symmetric sums in quarters where they exceed one
+        for (int m = 0; m < 7; ++m) F.f[m] = fix(w[m] * b[m], sc);
+        for (int m = 1; m < 7; ++m) F.f[6 + m] = fix(w[m] * m * b[m], sl);
+        const double g1[5] = {2 * b[1], 8 * b[2], 8 * b[3], 8 * b[5], 16 * b[6]}, g2[3] = {2 * b[4], 8 * b[5], 8 * b[6]};
+        for (int m = 0; m < 5; ++m) F.f[13 + m] = fix(g1[m], sc);
+        for (int m = 0; m < 3; ++m) F.f[18 + m] = fix(g2[m], sc);
+    } else {
+        const size_t n3 = (size_t)(M + 1) * (M + 1) * (M + 1);
+        oct.assign(2 * n3, 0);
+        size_t q = 0;
+        for (int x = 0; x <= M; ++x)
+            for (int y = 0; y <= M; ++y)
+                for (int z = 0; z <= M; ++z, ++q) {
+                    oct[q] = fix(amp(x, y, z), sc);
+                    oct[n3 + q] = fix((x * x + y * y + z * z) * amp(x, y, z), sl);
+                }
+    }
+    const double bad = fin ? 1.0 : std::nan("");
+    F.sphi = bad * sc / one;
+    F.sgrad = bad * -kap * sc / one * (F.fast ? 4.0 : (double)(1 << F.kM));
+    F.slap = bad * -kap * kap * sl / one;
+    CK(c->phi.alloc(1));
+    CK(cudaMemcpy(c->phi.p, &F, sizeof F, cudaMemcpyHostToDevice));
+    CK(c->phi_oct.alloc(oct.size()));
+    CK(cudaMemcpy(c->phi_oct.p, oct.data(), oct.size() * sizeof(long long), cudaMemcpyHostToDevice));
+    return DMC_OK;
+}
+
 int upload_kv(dmc_ctx* c)
 {
     std::vector<KVecDev> kv(c->S.nk);
@@ -342,7 +418,7 @@ int upload_kv(dmc_ctx* c)
     CK(c->kv_mp.alloc(km.size()));
     CK(cudaMemcpy(c->kv_mp.p, km.data(), km.size() * sizeof(KVecMP), cudaMemcpyHostToDevice));
     c->P.vorb1 = c->S.vorb[0];
-    return DMC_OK;
+    return upload_phi(c);
 }
 
 int upload_tables(dmc_ctx* c)
@@ -359,6 +435,23 @@ int upload_tables(dmc_ctx* c)
     CK(c->tss.alloc(nt));
     CK(cudaMemcpy(c->tud.p, ud.data(), nt * sizeof(TabUD), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c->tss.p, ss.data(), nt * sizeof(TabSS), cudaMemcpyHostToDevice));
+    // FP64 walker path: the cubic through points i-1 .. i+2 in t = position - i,
+    // from differences (an interval's own points give no cancellation)
+    std::vector<TabPoly> tp(nt);
+    std::memset(tp.data(), 0, nt * sizeof(TabPoly));
+    const std::vector<double>* src[7] = {&S.btab, &S.dbtab, &S.d2btab, &S.vtab[0], &S.utab[0], &S.dutab[0], &S.d2utab[0]};
+    for (int i = 1; i + 2 < nt; ++i)
+        for (int k = 0; k < 7; ++k) {
+            const double* T = src[k]->data() + i - 1;
+            const double d1 = T[2] - T[1];
+            const double a3 = ((T[3] - T[0]) - 3.0 * d1) / 6.0, a2 = ((T[0] - T[1]) + d1) / 2.0;
+            tp[i].c[k][0] = T[1];
+            tp[i].c[k][1] = (d1 - a2) - a3;
+            tp[i].c[k][2] = a2;
+            tp[i].c[k][3] = a3;
+        }
+    CK(c->tpoly.alloc(nt));
+    CK(cudaMemcpy(c->tpoly.p, tp.data(), nt * sizeof(TabPoly), cudaMemcpyHostToDevice));
     // mixed-precision copies in double-float
     std::vector<TabUDmp> udm(nt);
     std::vector<TabSSmp> ssm(nt);
@@ -404,6 +497,9 @@ KernelArgs base_args(dmc_ctx* c)
     a.kv = c->kv.p;
     a.tud = c->tud.p;
     a.tss = c->tss.p;
+    a.tpoly = c->tpoly.p;
+    a.phi = c->phi.p;
+    a.phi_oct = c->phi_oct.p;
     a.kv_mp = c->kv_mp.p;
     a.tud_mp = c->tud_mp.p;
     a.tss_mp = c->tss_mp.p;
@@ -415,11 +511,13 @@ KernelArgs base_args(dmc_ctx* c)
     return a;
 }
 
+const SmemLayout& layout_of(const dmc_ctx* c) { return c->precision == DMC_PREC_MIXED ? c->L : c->L64; }
+
 int grid_for(dmc_ctx* c, int nw) { return std::max(1, std::min(nw, c->grid)); }
 
 int run_eval(dmc_ctx* c, int mode, int nw, const double* dx, double* psil, int* is, double* dpsi, double* d2psi,
              double* v, double* vext, double* psigl, double* dpsig, double* d2psig, double* sinv, cudaStream_t st,
-             double* dphi = nullptr)
+             double* dphi = nullptr, bool inv_only = false)
 {
     if (nw <= 0) return DMC_OK;
     KernelArgs a = base_args(c);
@@ -431,7 +529,7 @@ int run_eval(dmc_ctx* c, int mode, int nw, const double* dx, double* psil, int* 
     CK(c->wstat.alloc(nw));
     a.wstatus = c->wstat.p;
     c->wstat_n = nw;
-    CK(launch_walker(c->P, a, c->L, grid_for(c, nw), st, c->precision == DMC_PREC_MIXED));
+    CK(launch_walker(c->P, a, layout_of(c), grid_for(c, nw), st, c->precision == DMC_PREC_MIXED));
     return DMC_OK;
 }
 
@@ -568,12 +666,31 @@ static int plan_layout(dmc_ctx* c, int optin, int kind, SmemLayout* Lout, int* p
 static int apply_layout(dmc_ctx* c, const SmemLayout& L, int per_sm)
 {
     const int grid = c->nsm * per_sm;
-    if (L.gstride > 0 && c->gscratch.alloc((size_t)grid * L.gstride) != cudaSuccess)
+    // the FP64 kernel's layout: all it can keep on chip with as many CTAs per SM
+    int smem_sm = 0, optin = 0;
+    cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, c->device);
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
+    const int st_on = std::max(0, walker_static_smem_bytes(c->rd.idmc == 10));
+    const int st_big = std::max(0, walker_big_static_smem_bytes());
+    SmemLayout L64{};
+    bool found = false;
+    for (int level = 0; level < 3 && !found; ++level) {
+        const int st = level < 2 ? st_on : st_big;
+        const int limit = std::min(smem_sm / per_sm - st - 1024, std::min(optin, 227 * 1024) - 64 - st);
+        L64 = make_layout64(c->P, limit, level);
+        found = (long long)L64.total * 8 <= (long long)limit;
+    }
+    if (!found) return fail(c, DMC_ERR_UNSUPPORTED, "the pair matrix does not fit one CTA's shared memory");
+    const int stride = std::max(L.gstride, L64.gstride);
+    if (stride > 0 && c->gscratch.alloc((size_t)grid * stride) != cudaSuccess)
         return fail(c, DMC_ERR_NOMEM, "walker scratch");
-    cudaError_t e = prepare_walker(L);
-    if (e == cudaSuccess && c->rd.idmc == 10) e = prepare_walker(L, true);
+    cudaError_t e = prepare_walker(L, true, false);
+    if (e == cudaSuccess) e = prepare_walker(L64, false, false);
+    if (e == cudaSuccess && c->rd.idmc == 10) e = prepare_walker(L, true, true);
+    if (e == cudaSuccess && c->rd.idmc == 10) e = prepare_walker(L64, false, true);
     if (e != cudaSuccess) return fail(c, DMC_ERR_CUDA, std::string("walker layout: ") + cudaGetErrorString(e));
     c->L = L;
+    c->L64 = L64;
     c->grid = grid;
     ++c->layout_gen;
     return DMC_OK;
@@ -664,7 +781,7 @@ int dmc_destroy(dmc_ctx* c)
     if (!c) return DMC_OK;
     if (c->stream) cudaStreamSynchronize(c->stream);
     c->kv.release(); c->tud.release(); c->tss.release(); c->kv_mp.release(); c->tud_mp.release();
-    c->tss_mp.release(); c->jumpA.release(); c->jumpC.release(); c->jq.release();
+    c->tss_mp.release(); c->tpoly.release(); c->phi.release(); c->phi_oct.release(); c->jumpA.release(); c->jumpC.release(); c->jq.release();
     c->gscratch.release(); c->st[0].release(); c->st[1].release(); c->est.release(); c->counts.release();
     c->offs.release(); c->status.release(); c->wstat.release(); c->irn1.release(); c->wtisto.release(); c->vb.release();
     c->bx.release(); c->bpsil.release(); c->bdpsi.release();
@@ -1192,7 +1309,7 @@ int dmc_step(dmc_ctx* c, int opcomp)
     // records are computed one thread per walker after the walker kernel
     a.defer = (c->P.idmc == 1 || c->P.idmc == -2) ? 1 : 0;
     CK(cudaEventRecord(c->ev0, c->stream));
-    CK(launch_walker(c->P, a, c->L, grid_for(c, n), c->stream, c->precision == DMC_PREC_MIXED));
+    CK(launch_walker(c->P, a, layout_of(c), grid_for(c, n), c->stream, c->precision == DMC_PREC_MIXED));
     if (a.defer) CK(launch_step_decide(c->P, a, c->stream));
     CK(cudaEventRecord(c->ev1, c->stream));
     CK(launch_estimators(c->est.p, n, c->P.nest, c->vb.p, c->vb2, c->wb, c->vbc, c->estpart.p, c->estticket.p,
@@ -1282,7 +1399,7 @@ static int gen_async(dmc_ctx* c, int opcomp, int* nlaunch, const DevStack* in_ho
     CK(cudaStreamIsCapturing(c->stream, &cap));
     const unsigned evflags = cap == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault;
     CK(cudaEventRecordWithFlags(c->ev0, c->stream, evflags));
-    CK(launch_walker(c->P, a, c->L, c->grid, c->stream, c->precision == DMC_PREC_MIXED));
+    CK(launch_walker(c->P, a, layout_of(c), c->grid, c->stream, c->precision == DMC_PREC_MIXED));
     ++nl;
     if (a.defer) {
         CK(launch_step_decide(c->P, a, c->stream));
@@ -1407,9 +1524,9 @@ int dmc_tune_layout(dmc_ctx* c, int passes, int* kind_out, double* ms_out)
         a.xin = c->st[c->istin].x.p;
         a.status = nullptr;
         const bool mixed = c->precision == DMC_PREC_MIXED;
-        CK(launch_walker(c->P, a, c->L, c->grid, c->stream, mixed));
+        CK(launch_walker(c->P, a, layout_of(c), c->grid, c->stream, mixed));
         CK(cudaEventRecord(c->ev0, c->stream));
-        for (int i = 0; i < passes; ++i) CK(launch_walker(c->P, a, c->L, c->grid, c->stream, mixed));
+        for (int i = 0; i < passes; ++i) CK(launch_walker(c->P, a, layout_of(c), c->grid, c->stream, mixed));
         CK(cudaEventRecord(c->ev1, c->stream));
         CK(cudaEventSynchronize(c->ev1));
         float ms = 0.0f;
@@ -2648,7 +2765,7 @@ int batch_eval_pass(dmc_batch* b, const std::vector<int>& grids, bool concurrent
             a.nw = c->n;
             a.xin = c->st[c->istin].x.p;
             a.status = nullptr;
-            if (launch_walker(c->P, a, c->L, std::max(1, std::min(grids[s], c->n)), c->stream,
+            if (launch_walker(c->P, a, layout_of(c), std::max(1, std::min(grids[s], c->n)), c->stream,
                               c->precision == DMC_PREC_MIXED) != cudaSuccess)
                 rc = DMC_ERR_CUDA;
         }

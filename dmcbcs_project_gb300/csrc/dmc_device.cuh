@@ -41,6 +41,31 @@ struct __align__(16) TabUDmp {
 struct __align__(16) TabSSmp {
     float v, u, du, d2u;
 };
+// FP64 path: the cubic through a grid interval's four points (the 4-point
+// Lagrange interpolation) as polynomial coefficients in t = grid position -
+// index, one 224-byte record per index: {beta, beta', lap beta, v, u, u', u''}
+// x {1, t, t^2, t^3}
+struct __align__(16) TabPoly {
+    double c[7][4];
+};
+
+// The pair function without beta as a sum over the octant n >= 0 of the
+// shells' integer vectors, phi(d) = sum_n A(n) c_nx c_ny c_nz with
+// c_m = cos(2 pi m d_axis / L) and A(n) = vorb(shell of |n|^2) 2^{non-zero
+// components of n} (every shell is complete), in 64-bit fixed point.
+// f: coefficients of the symmetric form for |n|^2 <= 6 (walker::PhiPair):
+// [0..6] phi, [7..12] Laplacian, [13..17] and [18..20] the two brackets of
+// the gradient.  Otherwise (fast = 0) the octant tables: entry
+// (nx (M+1) + ny)(M+1) + nz of A / scale, and behind them |n|^2 A / scale.
+// sphi, sgrad, slap: one unit of phi, of its gradient, of its Laplacian.
+constexpr int kPhiFast = 21;
+struct PhiFix {
+    long long f[kPhiFast];
+    double sphi, sgrad, slap;
+    int fast, M, kM, pad;     // octant form: the gradient's terms carry A / 2^kM
+};
+static_assert(sizeof(PhiFix) == 26 * 8, "staged as 26 doubles");
+
 struct __align__(16) KVecMP {
     df k[3];
     df k2;
@@ -127,6 +152,10 @@ struct KernelArgs {
     const KVecDev* kv;           // [nk]
     const TabUD* tud;            // [ntab+1]
     const TabSS* tss;            // [ntab+1]
+    const TabPoly* tpoly;        // FP64 path: the up-down tables by grid interval, [ntab+1]
+    const PhiFix* phi;           // FP64 path: the pair function's coefficients
+    const long long* phi_oct;    // its octant tables, 2 (M+1)^3 (nullptr in the symmetric form)
+    int inv_only;                // MODE_BCS: the caller reads the inverse alone (no drift, no Laplacian)
     const KVecMP* kv_mp;         // mixed-precision copies of kv, tud, tss
     const TabUDmp* tud_mp;
     const TabSSmp* tss_mp;
@@ -155,6 +184,8 @@ struct SmemLayout {
                           // the CTA's global scratch slice, at offset 0 of it
     int gstride;          // doubles of global scratch per CTA: the union region
                           // (when not on chip), then the beta pair data (idem)
+    int trig;             // FP64 layout: cos, sin of the axis angles [6][npart]
+    int rows64;           // FP64 layout: rows of Jastrow pair vectors per chunk
 };
 
 __host__ __device__ inline int round_up(int a, int b) { return (a + b - 1) / b * b; }
@@ -217,6 +248,61 @@ __host__ __device__ inline SmemLayout make_layout(const DevParams& p, int smem_l
         L.pb_in_smem = 0;
     }
     L.gstride = (union_global ? round_up(rsize, 2) : 0) + (L.pb_in_smem ? 0 : round_up(L.pb_size, 2));
+    L.total = off;
+    return L;
+}
+
+// Layout of the FP64 walker kernel, which forms no orbital matrices: beside
+// the positions, S and the reductions it holds every up-down pair's entry
+// gradient and Laplacian (pb: [4][nup ndn], kept from the pair stage to the
+// drift) and a union region with the axis cos/sin, the work area (Jastrow
+// pair vectors, long-range densities or same-spin pair vectors) and the
+// second inverse buffer.  level 0: all on chip; 1: the pair gradients in the
+// CTA's global slice; 2: the union region as well (the BIG instances).
+__host__ __device__ inline SmemLayout make_layout64(const DevParams& p, int smem_limit_bytes, int level)
+{
+    SmemLayout L{};
+    L.nt = kThreads;
+    const int n3 = p.npart * 3, pairs = p.nup * p.ndn;
+    int off = 0;
+    auto take = [&](int nd) { int o = off; off += round_up(nd, 2); return o; };
+    L.x = take(n3);
+    L.xr = take(n3);              // positions as 64-bit fractions of the box
+    L.xo = take(n3);
+    L.dx = take(n3);
+    L.drift = take(n3);
+    L.dg = take(n3);
+    L.kq = take((int)(sizeof(PhiFix) / 8));   // the pair function's coefficients
+    L.ksoa = L.kq;
+    L.S = take(p.nd * p.ldS);
+    L.colk = take(2 * p.nd + 2);
+    L.acc = take(p.npart * 8);
+    L.red = take(kThreads * 8);
+    const int row = 3 * (p.ndn > 0 ? p.ndn : 1), most = 3 * (p.nup > p.ndn ? p.nup : p.ndn);
+    const int fixed = round_up(6 * p.npart, 2) + round_up(p.nd * p.ldS, 2);
+    int work = row > most ? row : most;
+    work = round_up(work > 2 * p.nql ? work : 2 * p.nql, 2);   // at least one row, the densities, one same-spin row
+    L.pb_size = round_up(4 * pairs, 2);
+    L.pb_in_smem = level == 0 ? 1 : 0;
+    L.un_in_smem = level < 2 ? 1 : 0;
+    // as many rows of pair vectors per chunk as the rest leaves room for
+    const int room = smem_limit_bytes / 8 - off - fixed - (L.pb_in_smem ? L.pb_size : 0);
+    const int want = round_up(row * (p.nup > 0 ? p.nup : 1), 2);
+    if (level == 2 || room >= want)
+        work = work > want ? work : want;
+    else if (room > work)
+        work = room & ~1;
+    L.R = off;
+    L.U = L.D = L.E = L.R;
+    L.trig = L.R + work;
+    L.S2 = L.trig + round_up(6 * p.npart, 2);
+    L.rsize = work + fixed;
+    if (L.un_in_smem) off += L.rsize;
+    L.rows64 = work / row;
+    L.rows_jas = L.rows_beta = L.rows64;
+    L.pb = -1;
+    if (L.pb_in_smem) L.pb = take(L.pb_size);
+    L.gstride = (L.un_in_smem ? 0 : L.rsize) + (L.pb_in_smem ? 0 : L.pb_size);
     L.total = off;
     return L;
 }

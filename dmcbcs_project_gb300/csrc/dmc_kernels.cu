@@ -354,7 +354,7 @@ static int set_smem_attr(int v)
     return (int)cudaFuncSetAttribute(walker_kernel<R, NT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
 }
 
-static cudaError_t walker_attrs(int smem, int nt, bool both, bool mixed)
+static cudaError_t walker_attrs(int smem, int nt, bool mixed)
 {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -375,22 +375,18 @@ static cudaError_t walker_attrs(int smem, int nt, bool both, bool mixed)
     // the mixed kernel runs with the layout's thread count, the FP64 kernel
     // always with 256 (it is FP64-pipe bound: 16 warps did not speed it up)
     const bool wide = nt != kThreads;
-    if (both || mixed) {
+    if (mixed)
         rc = g_attr.ensure(dev, kAttrSmemBase + (wide ? 2 : 0), smem,
                            wide ? set_smem_attr<df, 2 * kThreads> : set_smem_attr<df, kThreads>);
-        if (rc) return (cudaError_t)rc;
-    }
-    if (both || !mixed) {
+    else
         rc = g_attr.ensure(dev, kAttrSmemBase + 1, smem, set_smem_attr<double, kThreads>);
-        if (rc) return (cudaError_t)rc;
-    }
-    return cudaSuccess;
+    return (cudaError_t)rc;
 }
 
-cudaError_t prepare_walker(const SmemLayout& L, bool gf)
+cudaError_t prepare_walker(const SmemLayout& L, bool mixed, bool gf)
 {
-    if (!L.un_in_smem) return walker_big_attrs(L.total * 8);
-    return gf ? walker_gf_attrs(L.total * 8, L.nt, true, false) : walker_attrs(L.total * 8, L.nt, true, false);
+    if (!L.un_in_smem) return walker_big_attrs(L.total * 8, mixed, gf);
+    return gf ? walker_gf_attrs(L.total * 8, L.nt, mixed) : walker_attrs(L.total * 8, L.nt, mixed);
 }
 
 cudaError_t launch_walker(const DevParams& p, const KernelArgs& a, const SmemLayout& L, int grid, cudaStream_t st,
@@ -401,7 +397,7 @@ cudaError_t launch_walker(const DevParams& p, const KernelArgs& a, const SmemLay
     const size_t smem = (size_t)L.total * 8;
     // the shared-memory opt-in is recorded per device and size (prepare_walker
     // sets it before any graph capture; this finds it set)
-    const cudaError_t e = walker_attrs((int)smem, L.nt, false, mixed);
+    const cudaError_t e = walker_attrs((int)smem, L.nt, mixed);
     if (e != cudaSuccess) return e;
     if (!mixed)
         walker_kernel<double, kThreads, false><<<grid, kThreads, smem, st>>>(p, a, L);

@@ -26,6 +26,7 @@
 
 #include "dmc_device.cuh"
 #include "dmc_dfmath.cuh"
+#include "dmc_pairfix.cuh"
 
 namespace dmc {
 namespace walker {
@@ -310,7 +311,7 @@ __device__ __forceinline__ T* at(double* sm, int off) { return reinterpret_cast<
 // the same-spin pairs (FP64 on both paths).
 // ---------------------------------------------------------------------------
 template <class R, int NT, bool BIG>
-__device__ void pair_stage(const Ctx<R, NT, BIG>& c, typename Prec<R>::J (&jt)[3], double (&ss)[3])
+__device__ void pair_stage(const Ctx<R, NT, BIG>& c, typename Prec<R>::J (&jt)[3])
 {
     using J = typename Prec<R>::J;
     const DevParams& p = c.p;
@@ -324,7 +325,6 @@ __device__ void pair_stage(const Ctx<R, NT, BIG>& c, typename Prec<R>::J (&jt)[3
     const auto* tud = Prec<R>::tud(c.a);
     const double imu_ud = 1.0 / (p.mass[0] * p.mass[1] / (p.mass[0] + p.mass[1]));
     const R imu_df = from_dbl<R>(imu_ud);
-    (void)imu_df;
     for (int i = threadIdx.x; i < 3 * p.npart; i += NT) du[i] = 0.0;
     // per-thread partial sums in the Jastrow type
     J tu = rzero<J>(), tv = rzero<J>(), td = rzero<J>();
@@ -345,76 +345,45 @@ __device__ void pair_stage(const Ctx<R, NT, BIG>& c, typename Prec<R>::J (&jt)[3
             const R rinv = rcp(rb);
             J g0 = rzero<J>(), g1 = rzero<J>(), g2 = rzero<J>();
             R f = rzero<R>(), dfr = rzero<R>(), d2f = rzero<R>();
-            if constexpr (!is_df<R>::value) {
-                // FP64: the reference's arithmetic (tiny clamp, separate grids)
-                const double r = fmax(rb, 1.0e-14);
-                if (r < p.range) {
-                    const Lagrange<double> W = lagrange(r, p.scale, p.ntab);
-                    const TabUD* T = c.a.tud + (W.idx - 1);
-                    const TabUD A0 = T[0], A1 = T[1], A2 = T[2], A3 = T[3];
-                    const double vp = W.c1 * A0.v + W.c2 * A1.v + W.c3 * A2.v + W.c4 * A3.v;
-                    const double uj = W.c1 * A0.u + W.c2 * A1.u + W.c3 * A2.u + W.c4 * A3.u;
-                    const double duj = W.c1 * A0.du + W.c2 * A1.du + W.c3 * A2.du + W.c4 * A3.du;
-                    const double d2uj = W.c1 * A0.d2u + W.c2 * A1.d2u + W.c3 * A2.d2u + W.c4 * A3.d2u;
-                    const double ri = (r == rb) ? rinv : 1.0 / r;
-                    tv += vp;
-                    tu += uj;
-                    const double gf = duj * ri;
-                    g0 = d0 * gf;
-                    g1 = d1 * gf;
-                    g2 = d2 * gf;
-                    td += (d2uj + 2.0 * gf) * imu_ud;
+            // mixed: one double-float grid position for beta and Jastrow.
+            // Inside the healing distance the Jastrow kinetic term and the
+            // potential nearly cancel, so both stay in double-float there;
+            // beyond it the Jastrow is exactly zero and only the
+            // exponentially small potential tail is left (FP32).
+            // full double-float comparisons: a pair within an FP32 ulp of
+            // a range end must fall on the same side as in FP64
+            const bool in_j = lt(rb, p.range_df);
+            const bool in_b = !p.nobeta && !lt(p.rangeb_df, rb);
+            if (in_j || in_b) {
+                df t;
+                const int idx = grid_pos(rb, p.scaleb_df, p.ntab, t);
+                const auto* T = tud + (idx - 1);
+                const auto A0 = T[0], A1 = T[1], A2 = T[2], A3 = T[3];
+                const Lagrange<df> W = lagrange_df(t, idx);
+                if (in_j) {
+                    if (idx - 1 <= p.ntab0) {
+                        const df vp = lag4(W, A0.v, A1.v, A2.v, A3.v);
+                        const df uj = lag4(W, A0.u, A1.u, A2.u, A3.u);
+                        const df duj = lag4(W, A0.du, A1.du, A2.du, A3.du);
+                        const df d2uj = lag4(W, A0.d2u, A1.d2u, A2.d2u, A3.d2u);
+                        const df gf = duj * rinv;
+                        tv += vp;
+                        tu += uj;
+                        g0 = d0 * gf;
+                        g1 = d1 * gf;
+                        g2 = d2 * gf;
+                        td += (d2uj + gf * 2.0f) * imu_df;
+                    } else {
+                        const float vp = W.c1.hi * A0.v.hi + W.c2.hi * A1.v.hi + W.c3.hi * A2.v.hi +
+                                         W.c4.hi * A3.v.hi;
+                        tv += df{vp, 0.0f};
+                    }
                 }
-                if (!p.nobeta && !(rb > p.rangeb)) {
-                    const Lagrange<double> W = lagrange(rb, p.scaleb, p.ntab);
-                    const TabUD* T = c.a.tud + (W.idx - 1);
-                    const TabUD A0 = T[0], A1 = T[1], A2 = T[2], A3 = T[3];
-                    f = W.c1 * A0.b + W.c2 * A1.b + W.c3 * A2.b + W.c4 * A3.b;
-                    const double df_ = W.c1 * A0.db + W.c2 * A1.db + W.c3 * A2.db + W.c4 * A3.db;
-                    d2f = W.c1 * A0.d2b + W.c2 * A1.d2b + W.c3 * A2.d2b + W.c4 * A3.d2b;
+                if (in_b) {
+                    f = lag4(W, A0.b, A1.b, A2.b, A3.b);
+                    const df df_ = lag4(W, A0.db, A1.db, A2.db, A3.db);
+                    d2f = lag4(W, A0.d2b, A1.d2b, A2.d2b, A3.d2b);
                     dfr = df_ * rinv;
-                }
-            } else {
-                // mixed: one double-float grid position for beta and Jastrow.
-                // Inside the healing distance the Jastrow kinetic term and the
-                // potential nearly cancel, so both stay in double-float there;
-                // beyond it the Jastrow is exactly zero and only the
-                // exponentially small potential tail is left (FP32).
-                // full double-float comparisons: a pair within an FP32 ulp of
-                // a range end must fall on the same side as in FP64
-                const bool in_j = lt(rb, p.range_df);
-                const bool in_b = !p.nobeta && !lt(p.rangeb_df, rb);
-                if (in_j || in_b) {
-                    df t;
-                    const int idx = grid_pos(rb, p.scaleb_df, p.ntab, t);
-                    const auto* T = tud + (idx - 1);
-                    const auto A0 = T[0], A1 = T[1], A2 = T[2], A3 = T[3];
-                    const Lagrange<df> W = lagrange_df(t, idx);
-                    if (in_j) {
-                        if (idx - 1 <= p.ntab0) {
-                            const df vp = lag4(W, A0.v, A1.v, A2.v, A3.v);
-                            const df uj = lag4(W, A0.u, A1.u, A2.u, A3.u);
-                            const df duj = lag4(W, A0.du, A1.du, A2.du, A3.du);
-                            const df d2uj = lag4(W, A0.d2u, A1.d2u, A2.d2u, A3.d2u);
-                            const df gf = duj * rinv;
-                            tv += vp;
-                            tu += uj;
-                            g0 = d0 * gf;
-                            g1 = d1 * gf;
-                            g2 = d2 * gf;
-                            td += (d2uj + gf * 2.0f) * imu_df;
-                        } else {
-                            const float vp = W.c1.hi * A0.v.hi + W.c2.hi * A1.v.hi + W.c3.hi * A2.v.hi +
-                                             W.c4.hi * A3.v.hi;
-                            tv += df{vp, 0.0f};
-                        }
-                    }
-                    if (in_b) {
-                        f = lag4(W, A0.b, A1.b, A2.b, A3.b);
-                        const df df_ = lag4(W, A0.db, A1.db, A2.db, A3.db);
-                        d2f = lag4(W, A0.d2b, A1.d2b, A2.d2b, A3.d2b);
-                        dfr = df_ * rinv;
-                    }
                 }
             }
             S[i * ldS + j] = f;
@@ -448,12 +417,23 @@ __device__ void pair_stage(const Ctx<R, NT, BIG>& c, typename Prec<R>::J (&jt)[3
     jt[0] = tu;
     jt[1] = tv;
     jt[2] = td;
-    if (!p.ieq) return;
+}
+
+// ---------------------------------------------------------------------------
+// Same-spin pairs (coshpot.f90:167 with cjas(2) != 0): up-up then down-down,
+// in FP64 on both paths (off the benchmark configurations); ss[] gets the
+// per-thread sums of u, v and the pair Laplacian part.
+// ---------------------------------------------------------------------------
+template <class R, int NT, bool BIG>
+__device__ void same_spin_stage(const Ctx<R, NT, BIG>& c, double (&ss)[3])
+{
+    const DevParams& p = c.p;
+    double* sm = c.sm;
+    double* du = sm + c.L.acc + 4 * p.npart;
+    const int nup = p.nup, ndn = p.ndn;
     double& su = ss[0];
     double& sv = ss[1];
     double& sd2 = ss[2];
-    // same-spin pairs (coshpot.f90:167 with cjas(2) != 0): up-up then down-down,
-    // in FP64 on both paths (off the benchmark configurations)
     const double* xd = sm + c.L.x;
     for (int blk = 0; blk < 2; ++blk) {
         const int n = blk == 0 ? nup : ndn;
@@ -534,6 +514,231 @@ __device__ void pair_stage(const Ctx<R, NT, BIG>& c, typename Prec<R>::J (&jt)[3
     }
 }
 
+// ---------------------------------------------------------------------------
+// FP64 path, before the pairs: positions as 64-bit fractions of the box
+// (differences then wrap to the minimum image by themselves), the axis
+// angles' cos and sin, and a flag per particle with a coordinate that is not
+// finite (such a particle's pairs get NaN, as its distances would).
+// x / L is formed as h + l, l the division's remainder, so that a fraction is
+// exact to 2^-64 whatever the coordinate.
+// ---------------------------------------------------------------------------
+template <int NT, bool BIG>
+__device__ void fix_positions(const Ctx<double, NT, BIG>& c)
+{
+    const DevParams& p = c.p;
+    double* sm = c.sm;
+    const double* x = sm + c.L.x;
+    long long* xf = at<long long>(sm, c.L.xr);
+    long long* tr = c.template uat<long long>(c.L.trig);
+    int* nf = reinterpret_cast<int*>(sm + c.L.acc + 7 * p.npart);
+    const double two64 = 18446744073709551616.0;
+    for (int t = threadIdx.x; t < 3 * p.npart; t += NT) {
+        const int pt = t / 3, a = t - 3 * pt;
+        const double xv = x[t];
+        const double h = xv * p.eli, l = fma(-h, p.el, xv) * p.eli;
+        const double hf = h - rint(h);
+        xf[t] = fadd(__double2ll_rn(hf * two64), __double2ll_rn(l * two64));
+        double sn, cs;
+        sincospi(2.0 * hf, &sn, &cs);
+        tr[(2 * a) * p.npart + pt] = __double2ll_rn(cs * kFixScale);
+        tr[(2 * a + 1) * p.npart + pt] = __double2ll_rn(sn * kFixScale);
+        if (a == 0) nf[pt] = !(isfinite(x[t]) && isfinite(x[t + 1]) && isfinite(x[t + 2]));
+    }
+    __syncthreads();
+}
+
+// ---------------------------------------------------------------------------
+// FP64 path, stages 1 to 3 in one pass over the up-down pairs: Jastrow and
+// potential (coshpot.f90:154-205) and the pair function with beta
+// (psislaterbcs.f90:247-293, betafun.f90:173-194).  Every shell is complete,
+// so the plane-wave sum of an entry and of its derivatives is a short
+// polynomial in the cosines of the pair's three axis angles (dmc_pairfix.cuh):
+// no orbitals, no products over k.  Writes S[i][j], the entry's gradient with
+// respect to x_i and its Laplacian to pb ([4][nup ndn]; inv_only: S alone)
+// and the Jastrow gradients' sums to acc.  jt[] gets the per-thread sums of
+// u, v and the pair Laplacian part; returns whether a pair at distance zero
+// left the derivatives not finite (inv_only, which does not form them).
+// Bound: the FP64 pipe, about 60 of its instructions a pair; the 64 high
+// products run beside it on the integer pipe.
+// ---------------------------------------------------------------------------
+template <int NT, bool BIG>
+__device__ bool pair_stage64(const Ctx<double, NT, BIG>& c, int mode, double (&jt)[3])
+{
+    const DevParams& p = c.p;
+    double* sm = c.sm;
+    const double* x = sm + c.L.x;
+    const long long* xf = at<long long>(sm, c.L.xr);
+    const long long* tr = c.template uat<long long>(c.L.trig);
+    const int* nf = reinterpret_cast<const int*>(sm + c.L.acc + 7 * p.npart);
+    const PhiFix* F = reinterpret_cast<const PhiFix*>(sm + c.L.kq);
+    double* S = sm + c.L.S;
+    double* pv = c.template uat<double>(c.L.R);
+    double* du = sm + c.L.acc + 4 * p.npart;
+    const int nup = p.nup, ndn = p.ndn, ldS = p.ldS, P = p.npart, pairs = nup * ndn;
+    double* w0 = c.pb;
+    const bool jas = mode != MODE_BCS, det = mode != MODE_GETPHI, grad = det && !(mode == MODE_BCS && c.a.inv_only);
+    const double unit = p.el * 5.421010862427522e-20;    // L 2^-64: distances below are in this unit, L/2 = 2^63
+    const double tscale = (double)p.ntab * 1.0842021724855044e-19;   // grid points per unit: ntab / 2^63
+    const double r_min = 1.0e-14 / unit, two_iu = 2.0 / unit;
+    const long long half = 0x43E0000000000000ll;         // 2^63 as a double's bits
+    const double imu_ud = 1.0 / (p.mass[0] * p.mass[1] / (p.mass[0] + p.mass[1]));
+    double tu = 0.0, tv = 0.0, td = 0.0;
+    bool bad = false;
+    if (jas)
+        for (int i = threadIdx.x; i < 3 * P; i += NT) du[i] = 0.0;
+    __syncthreads();
+    const int rows = jas ? c.L.rows64 : nup;
+    for (int r0 = 0; r0 < nup; r0 += rows) {
+        const int r1 = min(nup, r0 + rows);
+        const int npc = (r1 - r0) * ndn;
+        const UDiv dv(ndn);
+        for (int q = threadIdx.x; q < npc; q += NT) {
+            const int qi = dv.quo(q);
+            const int i = r0 + qi, j = q - qi * ndn, pj = nup + j;
+            // the integer part first: its temporaries are dead before the distances
+            PhiPair o;
+            if (det) {
+                if (F->fast)
+                    phi_sym(F, tr, P, i, pj, grad, o);
+                else
+                    phi_octant(F, c.a.phi_oct, tr, P, i, pj, o);
+            }
+            const bool nan = (nf[i] | nf[pj]) != 0;
+            const long long e0 = fsub(xf[3 * i], xf[3 * pj]), e1 = fsub(xf[3 * i + 1], xf[3 * pj + 1]);
+            const long long e2 = fsub(xf[3 * i + 2], xf[3 * pj + 2]);
+            double d0 = (double)e0, d1 = (double)e1, d2 = (double)e2, r, ri;
+            if (nan) d0 = __longlong_as_double(0x7ff8000000000000ll);
+            if (((e0 | e1) | e2) != 0 || nan) {
+                inv_dist(fma(d0, d0, fma(d1, d1, d2 * d2)), r, ri);
+            } else {   // closer than a unit, or coincident: 1/r is large or infinite
+                d0 = min_image(x[3 * i] - x[3 * pj], p) / unit;
+                d1 = min_image(x[3 * i + 1] - x[3 * pj + 1], p) / unit;
+                d2 = min_image(x[3 * i + 2] - x[3 * pj + 2], p) / unit;
+                r = sqrt(norm2(d0, d1, d2));
+                ri = 1.0 / r;
+            }
+            const long long rb = __double_as_longlong(r);
+            double t;
+            const TabPoly* T = c.a.tpoly + grid_split(r * tscale, p.ntab, t);
+            if (jas) {
+                double g0 = 0.0, g1 = 0.0, g2 = 0.0;
+                if (rb < half) {   // r < L/2 (false for NaN)
+                    const TabPoly* TJ = T;
+                    double tj = t, rj = ri;
+                    if (r < r_min) {   // the reference's clamp, coshpot.f90:170
+                        TJ = c.a.tpoly + grid_split(r_min * tscale, p.ntab, tj);
+                        rj = 1.0 / r_min;
+                    }
+                    tv += poly3(TJ->c[3], tj);
+                    tu += poly3(TJ->c[4], tj);
+                    const double gf = poly3(TJ->c[5], tj) * rj;
+                    td += fma(gf, two_iu, poly3(TJ->c[6], tj));
+                    g0 = d0 * gf;
+                    g1 = d1 * gf;
+                    g2 = d2 * gf;
+                }
+                pv[3 * q + 0] = g0;
+                pv[3 * q + 1] = g1;
+                pv[3 * q + 2] = g2;
+            }
+            if (det) {
+                const bool in_b = !p.nobeta && (rb <= half || nan);
+                double f = in_b ? poly3(T->c[0], t) : 0.0;
+                if (nan) f = d0;
+                S[i * ldS + j] = fma((double)o.f, F->sphi, f);
+                if (grad) {
+                    double gr = 0.0, lp = 0.0;
+                    if (in_b) {
+                        gr = poly3(T->c[1], t) * ri;
+                        lp = poly3(T->c[2], t);
+                    }
+                    if (nan) gr = lp = d0;
+                    double* w = w0 + i * ndn + j;
+                    w[0] = fma((double)o.g[0], F->sgrad, gr * d0);
+                    w[pairs] = fma((double)o.g[1], F->sgrad, gr * d1);
+                    w[2 * pairs] = fma((double)o.g[2], F->sgrad, gr * d2);
+                    w[3 * pairs] = fma((double)o.l, F->slap, lp);
+                } else if (in_b && !isfinite(ri)) {
+                    bad = true;   // the drift would not be finite
+                }
+            }
+        }
+        __syncthreads();
+        if (!jas) continue;
+        // row sums -> up particles (+), column sums -> down particles (-);
+        // one thread per (particle, component)
+        const int nr = r1 - r0;
+        for (int tc = threadIdx.x; tc < 3 * (nr + ndn); tc += NT) {
+            const int t = tc / 3, cmp = tc % 3;
+            double s0 = 0.0, s1 = 0.0;
+            if (t < nr) {
+                const double* row = pv + 3 * (t * ndn) + cmp;
+                int j = 0;
+                for (; j + 1 < ndn; j += 2) {
+                    s0 += row[3 * j];
+                    s1 += row[3 * j + 3];
+                }
+                if (j < ndn) s0 += row[3 * j];
+                du[3 * (r0 + t) + cmp] += (s0 + s1) * p.isqm[0];
+            } else {
+                const int j = t - nr;
+                int r = 0;
+                for (; r + 1 < nr; r += 2) {
+                    s0 += pv[3 * (r * ndn + j) + cmp];
+                    s1 += pv[3 * ((r + 1) * ndn + j) + cmp];
+                }
+                if (r < nr) s0 += pv[3 * (r * ndn + j) + cmp];
+                du[3 * (nup + j) + cmp] -= (s0 + s1) * p.isqm[1];
+            }
+        }
+        __syncthreads();
+    }
+    jt[0] = tu;
+    jt[1] = tv;
+    jt[2] = td * imu_ud;
+    return bad;
+}
+
+// ---------------------------------------------------------------------------
+// FP64 path, stages 5 and 6: drift and Laplacian of log det from the inverse
+// and the entries' derivatives (psislaterbcs.f90:209-223),
+//   up i: sum_j Sinv[j][i] w[i][j],  down j: sum_i Sinv[j][i] w[i][j]
+// (the drift with a minus sign); two threads per (particle, component), every
+// second term each.
+// ---------------------------------------------------------------------------
+template <int NT, bool BIG>
+__device__ void pair_drift64(const Ctx<double, NT, BIG>& c)
+{
+    const DevParams& p = c.p;
+    double* sm = c.sm;
+    const double* Si = sm + c.L.S;
+    double* acc = sm + c.L.acc;
+    const int nup = p.nup, ndn = p.ndn, ld = p.ldS, P = p.npart, pairs = nup * ndn;
+    for (int t0 = 0; t0 < 8 * P; t0 += NT) {
+        const int t = t0 + (int)threadIdx.x, it = t >> 1, h = t & 1;
+        const int k = it / P, pt = it - k * P;
+        double s0 = 0.0, s1 = 0.0;
+        if (t < 8 * P) {
+            const double* w = c.pb + (size_t)k * pairs;
+            const bool up = pt < nup;
+            const int j = up ? 0 : pt - nup, n = up ? ndn : nup;
+            const double* a = up ? Si + pt + h * ld : Si + j * ld + h;
+            const double* b = up ? w + pt * ndn + h : w + j + h * ndn;
+            const int sa = up ? 2 * ld : 2, sb = up ? 2 : 2 * ndn, m = (n - h + 1) / 2;
+            int e = 0;
+            for (; e + 1 < m; e += 2) {
+                s0 = fma(a[e * sa], b[e * sb], s0);
+                s1 = fma(a[(e + 1) * sa], b[(e + 1) * sb], s1);
+            }
+            if (e < m) s0 = fma(a[e * sa], b[e * sb], s0);
+        }
+        s0 += s1;
+        s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
+        if (t < 8 * P && h == 0) acc[k < 3 ? 3 * pt + k : 3 * P + pt] = (k < 3 && pt >= nup) ? -s0 : s0;
+    }
+    __syncthreads();
+}
+
 // complex product in the arithmetic type
 __device__ __forceinline__ void cmul(double ar, double ai, double br, double bi, double& cr, double& ci)
 {
@@ -573,20 +778,51 @@ __device__ __forceinline__ void cmul(df ar, df ai, df br, df bi, df& cr, df& ci)
     ci = acc_value(i);
 }
 
+// Unpaired plane waves in S (psislaterbcs.f90:171-206): up columns ndn..,
+// down rows nup.., zero corner.
+template <class R, int NT, bool BIG>
+__device__ __forceinline__ void unpaired_entries(const Ctx<R, NT, BIG>& c)
+{
+    const DevParams& p = c.p;
+    double* sm = c.sm;
+    const double* x = sm + c.L.x;
+    R* S = at<R>(sm, c.L.S);
+    const int ldS = p.ldS;
+    for (int t = threadIdx.x; t < p.nup * p.nexup; t += NT) {
+        const int i = t / p.nexup, jj = t % p.nexup;
+        const double* xi = x + 3 * i;
+        const double arg = p.akup[jj][0] * xi[0] + p.akup[jj][1] * xi[1] + p.akup[jj][2] * xi[2];
+        double s, co;
+        sincos(arg, &s, &co);
+        S[i * ldS + p.ndn + jj] = from_dbl<R>(p.sinup[jj] ? s : co);
+    }
+    for (int t = threadIdx.x; t < p.ndn * p.nexdn; t += NT) {
+        const int j = t / p.nexdn, jj = t % p.nexdn;
+        const double* xj = x + 3 * (p.nup + j);
+        const double arg = p.akdn[jj][0] * xj[0] + p.akdn[jj][1] * xj[1] + p.akdn[jj][2] * xj[2];
+        double s, co;
+        sincos(arg, &s, &co);
+        S[(p.nup + jj) * ldS + j] = from_dbl<R>(p.sindn[jj] ? s : co);
+    }
+    for (int t = threadIdx.x; t < p.nexdn * p.nexup; t += NT) {
+        const int r = t / p.nexup, cc = t % p.nexup;
+        S[(p.nup + r) * ldS + p.ndn + cc] = rzero<R>();
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Stage 2: pair orbitals (psislaterbcs.f90:248-277).  exp(i k.x) is built
 // from exp(i 2 pi x_c / L) and its integer powers, so each particle needs
 // three sincos instead of one per k vector.
 // U[i][0] = vorb(1), U[i][2q-1] = v_q cos(k_q.x_i), U[i][2q] = v_q sin(k_q.x_i)
 // D[j][0] = 1,       D[j][2q-1] = cos(k_q.x_j),     D[j][2q] = sin(k_q.x_j)
-// Then the unpaired plane-wave rows and columns of S (:171-206).
+// Then the unpaired plane-wave rows and columns of S (:171-206).  (Mixed path.)
 // ---------------------------------------------------------------------------
 template <class R, int NT, bool BIG>
 __device__ void orbital_stage(const Ctx<R, NT, BIG>& c)
 {
     const DevParams& p = c.p;
     double* sm = c.sm;
-    const double* x = sm + c.L.x;
     R* U = c.template uat<R>(c.L.U);
     R* D = c.template uat<R>(c.L.D);
     R* E = c.template uat<R>(c.L.E);
@@ -595,12 +831,8 @@ __device__ void orbital_stage(const Ctx<R, NT, BIG>& c)
     // powers e^{i m theta_c}, m = 0..nmax, E[(p*3+c)*np1 + m] = (re, im)
     for (int t = threadIdx.x; t < 3 * p.npart; t += NT) {
         R s1, c1;
-        if constexpr (is_df<R>::value) {
-            // base angle 2 pi x / L in double-float, off the FP64 pipe
-            dfm::sincospi_df(at<R>(sm, c.L.xr)[t] * p.eli2_df, s1, c1);
-        } else {
-            sincospi(2.0 * x[t] * p.eli, &s1, &c1);
-        }
+        // base angle 2 pi x / L in double-float, off the FP64 pipe
+        dfm::sincospi_df(at<R>(sm, c.L.xr)[t] * p.eli2_df, s1, c1);
         R* e = E + 2 * t * np1;
         e[0] = rone<R>();
         e[1] = rzero<R>();
@@ -668,28 +900,7 @@ __device__ void orbital_stage(const Ctx<R, NT, BIG>& c)
             ++part;
         }
     }
-    // unpaired plane waves: up columns ndn.., down rows nup.., zero corner
-    const int ldS = p.ldS;
-    for (int t = threadIdx.x; t < p.nup * p.nexup; t += NT) {
-        const int i = t / p.nexup, jj = t % p.nexup;
-        const double* xi = x + 3 * i;
-        const double arg = p.akup[jj][0] * xi[0] + p.akup[jj][1] * xi[1] + p.akup[jj][2] * xi[2];
-        double s, co;
-        sincos(arg, &s, &co);
-        S[i * ldS + p.ndn + jj] = from_dbl<R>(p.sinup[jj] ? s : co);
-    }
-    for (int t = threadIdx.x; t < p.ndn * p.nexdn; t += NT) {
-        const int j = t / p.nexdn, jj = t % p.nexdn;
-        const double* xj = x + 3 * (p.nup + j);
-        const double arg = p.akdn[jj][0] * xj[0] + p.akdn[jj][1] * xj[1] + p.akdn[jj][2] * xj[2];
-        double s, co;
-        sincos(arg, &s, &co);
-        S[(p.nup + jj) * ldS + j] = from_dbl<R>(p.sindn[jj] ? s : co);
-    }
-    for (int t = threadIdx.x; t < p.nexdn * p.nexup; t += NT) {
-        const int r = t / p.nexup, cc = t % p.nexup;
-        S[(p.nup + r) * ldS + p.ndn + cc] = rzero<R>();
-    }
+    unpaired_entries(c);
     __syncthreads();
 }
 
@@ -703,7 +914,6 @@ constexpr int kGJ = 5;
 template <class R, int NT, bool BIG>
 __device__ void gemm_stage(const Ctx<R, NT, BIG>& c)
 {
-    using Acc = typename AccOf<R>::type;
     const DevParams& p = c.p;
     double* sm = c.sm;
     const R* U = c.template uat<R>(c.L.U);
@@ -711,17 +921,14 @@ __device__ void gemm_stage(const Ctx<R, NT, BIG>& c)
     R* S = at<R>(sm, c.L.S);
     const int ldU = p.ldU;
     const int ng = (p.ndn + kGJ - 1) / kGJ;
-    // double-float path: |U[i][q] D[j][q]| <= |v_q| bounds every term (cos and
+    // |U[i][q] D[j][q]| <= |v_q| bounds every term (cos and
     // sin columns, |D| <= 1; the k = 0 column holds v_0 and 1), so one bound
     // per walker serves the bounded accumulator (6 FP32 instructions per
     // multiply-add instead of 12; error of order K 2^-48 sigma)
-    float sig = 0.0f;
-    if constexpr (is_df<R>::value) {
-        const R* kv = at<R>(sm, c.L.ksoa) + 4 * p.nk;
-        float sv = fabsf(kv[0].hi);
-        for (int q = 1; q < p.nk; ++q) sv += 2.0f * fabsf(kv[q].hi);
-        sig = pow2_ceil(4.0f * 1.001f * sv);
-    }
+    const R* kv = at<R>(sm, c.L.ksoa) + 4 * p.nk;
+    float sv = fabsf(kv[0].hi);
+    for (int q = 1; q < p.nk; ++q) sv += 2.0f * fabsf(kv[q].hi);
+    const float sig = pow2_ceil(4.0f * 1.001f * sv);
     const UDiv dg(ng);
     for (int t = threadIdx.x; t < p.nup * ng; t += NT) {
         const int i = dg.quo(t), g = t - i * ng;
@@ -734,49 +941,26 @@ __device__ void gemm_stage(const Ctx<R, NT, BIG>& c)
             ok[m] = j < p.ndn;
             d[m] = D + (ok[m] ? j : g) * ldU;
         }
-        if constexpr (is_df<R>::value) {
-            bacc a[kGJ];
+        bacc a[kGJ];
 #pragma unroll
-            for (int m = 0; m < kGJ; ++m) bacc_init(a[m], sig);
-            for (int q = 0; q < ldU; q += 2) {
-                R ua, ub;
-                ld2(u + q, ua, ub);
+        for (int m = 0; m < kGJ; ++m) bacc_init(a[m], sig);
+        for (int q = 0; q < ldU; q += 2) {
+            R ua, ub;
+            ld2(u + q, ua, ub);
 #pragma unroll
-                for (int m = 0; m < kGJ; ++m) {
-                    R xa, xb;
-                    ld2(d[m] + q, xa, xb);
-                    bacc_madd(a[m], ua, xa);
-                    bacc_madd(a[m], ub, xb);
-                }
+            for (int m = 0; m < kGJ; ++m) {
+                R xa, xb;
+                ld2(d[m] + q, xa, xb);
+                bacc_madd(a[m], ua, xa);
+                bacc_madd(a[m], ub, xb);
             }
-#pragma unroll
-            for (int m = 0; m < kGJ; ++m)
-                if (ok[m]) {
-                    R* sij = S + i * p.ldS + g + ng * m;
-                    *sij = bacc_value(a[m], sig) + *sij;
-                }
-        } else {
-            Acc a[kGJ];
-#pragma unroll
-            for (int m = 0; m < kGJ; ++m) acc_init(a[m]);
-            for (int q = 0; q < ldU; q += 2) {
-                R ua, ub;
-                ld2(u + q, ua, ub);
-#pragma unroll
-                for (int m = 0; m < kGJ; ++m) {
-                    R xa, xb;
-                    ld2(d[m] + q, xa, xb);
-                    acc_madd(a[m], ua, xa);
-                    acc_madd(a[m], ub, xb);
-                }
-            }
-#pragma unroll
-            for (int m = 0; m < kGJ; ++m)
-                if (ok[m]) {
-                    R* sij = S + i * p.ldS + g + ng * m;
-                    *sij = acc_value(a[m]) + *sij;
-                }
         }
+#pragma unroll
+        for (int m = 0; m < kGJ; ++m)
+            if (ok[m]) {
+                R* sij = S + i * p.ldS + g + ng * m;
+                *sij = bacc_value(a[m], sig) + *sij;
+            }
     }
     __syncthreads();
 }
@@ -1789,6 +1973,59 @@ __device__ void drift_stage(const Ctx<R, NT, BIG>& c)
     __syncthreads();
 }
 
+// Unpaired plane waves in the drift and Laplacian (psislaterbcs.f90:171-206
+// with :211-223).
+template <class R, int NT, bool BIG>
+__device__ __forceinline__ void unpaired_drift(const Ctx<R, NT, BIG>& c)
+{
+    const DevParams& p = c.p;
+    double* sm = c.sm;
+    const double* x = sm + c.L.x;
+    const R* Si = at<R>(sm, c.L.S);
+    double* acc = sm + c.L.acc;
+    const int nup = p.nup, ndn = p.ndn, ld = p.ldS, P = p.npart;
+    if (p.nexup > 0 || p.nexdn > 0) {
+        for (int pt = threadIdx.x; pt < P; pt += NT) {
+            const double* xp = x + 3 * pt;
+            double g0 = 0, g1 = 0, g2 = 0, lp = 0;
+            if (pt < nup) {
+                for (int jj = 0; jj < p.nexup; ++jj) {
+                    const double* k = p.akup[jj];
+                    double s, co;
+                    sincos(k[0] * xp[0] + k[1] * xp[1] + k[2] * xp[2], &s, &co);
+                    const double w = to_double(Si[(ndn + jj) * ld + pt]);
+                    // sin: grad k cos, lap -k2 sin; cos: grad -k sin, lap -k2 cos
+                    const double gcoef = p.sinup[jj] ? co : -s;
+                    const double val = p.sinup[jj] ? s : co;
+                    g0 += w * k[0] * gcoef;
+                    g1 += w * k[1] * gcoef;
+                    g2 += w * k[2] * gcoef;
+                    lp += w * (-p.ak2up[jj] * val);
+                }
+            } else {
+                const int j = pt - nup;
+                for (int jj = 0; jj < p.nexdn; ++jj) {
+                    const double* k = p.akdn[jj];
+                    double s, co;
+                    sincos(k[0] * xp[0] + k[1] * xp[1] + k[2] * xp[2], &s, &co);
+                    const double w = to_double(Si[j * ld + nup + jj]);
+                    const double gcoef = p.sindn[jj] ? co : -s;
+                    const double val = p.sindn[jj] ? s : co;
+                    g0 += w * k[0] * gcoef;
+                    g1 += w * k[1] * gcoef;
+                    g2 += w * k[2] * gcoef;
+                    lp += w * (-p.ak2dn[jj] * val);
+                }
+            }
+            acc[3 * pt + 0] += g0;
+            acc[3 * pt + 1] += g1;
+            acc[3 * pt + 2] += g2;
+            acc[3 * P + pt] += lp;
+        }
+        __syncthreads();
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Stage 6: beta terms of the drift and Laplacian (psislaterbcs.f90:290-291
 // through :213-222): per up-down pair h = Sinv[j][i] f'/r dx, l = Sinv[j][i]
@@ -1847,47 +2084,7 @@ __device__ void beta_drift_stage(const Ctx<R, NT, BIG>& c)
             __syncthreads();
         }
     }
-    // unpaired plane waves (psislaterbcs.f90:171-206 with :211-223)
-    if (p.nexup > 0 || p.nexdn > 0) {
-        for (int pt = threadIdx.x; pt < P; pt += NT) {
-            const double* xp = x + 3 * pt;
-            double g0 = 0, g1 = 0, g2 = 0, lp = 0;
-            if (pt < nup) {
-                for (int jj = 0; jj < p.nexup; ++jj) {
-                    const double* k = p.akup[jj];
-                    double s, co;
-                    sincos(k[0] * xp[0] + k[1] * xp[1] + k[2] * xp[2], &s, &co);
-                    const double w = to_double(Si[(ndn + jj) * ld + pt]);
-                    // sin: grad k cos, lap -k2 sin; cos: grad -k sin, lap -k2 cos
-                    const double gcoef = p.sinup[jj] ? co : -s;
-                    const double val = p.sinup[jj] ? s : co;
-                    g0 += w * k[0] * gcoef;
-                    g1 += w * k[1] * gcoef;
-                    g2 += w * k[2] * gcoef;
-                    lp += w * (-p.ak2up[jj] * val);
-                }
-            } else {
-                const int j = pt - nup;
-                for (int jj = 0; jj < p.nexdn; ++jj) {
-                    const double* k = p.akdn[jj];
-                    double s, co;
-                    sincos(k[0] * xp[0] + k[1] * xp[1] + k[2] * xp[2], &s, &co);
-                    const double w = to_double(Si[j * ld + nup + jj]);
-                    const double gcoef = p.sindn[jj] ? co : -s;
-                    const double val = p.sindn[jj] ? s : co;
-                    g0 += w * k[0] * gcoef;
-                    g1 += w * k[1] * gcoef;
-                    g2 += w * k[2] * gcoef;
-                    lp += w * (-p.ak2dn[jj] * val);
-                }
-            }
-            acc[3 * pt + 0] += g0;
-            acc[3 * pt + 1] += g1;
-            acc[3 * pt + 2] += g2;
-            acc[3 * P + pt] += lp;
-        }
-        __syncthreads();
-    }
+    unpaired_drift(c);
 }
 
 // ---------------------------------------------------------------------------
@@ -1952,6 +2149,7 @@ struct HRes {
     double psil, d2psi, v, vext, psigl, d2psig, u, d2u, logdet, d2phi;
     int is;
     bool singular;
+    bool bad;   // this thread met a pair whose drift terms (not formed: inv_only) are not finite
 };
 
 // ---------------------------------------------------------------------------
@@ -1968,16 +2166,23 @@ __device__ HRes hpsi_eval(const Ctx<R, NT, BIG>& c, int mode)
     double* acc = sm + c.L.acc;
     double* du = acc + 4 * P;
     const double* x = sm + c.L.x;
-    {
-        R* xr = at<R>(sm, c.L.xr);
-        for (int i = threadIdx.x; i < n3; i += NT) xr[i] = from_dbl<R>(x[i]);
-        __syncthreads();
-    }
     HRes h;
     using J = typename Prec<R>::J;
     J jt[3] = {rzero<J>(), rzero<J>(), rzero<J>()};
     double ss[3] = {0.0, 0.0, 0.0};
-    pair_stage<R>(c, jt, ss);   // also fills the beta part of S (needed by MODE_BCS too)
+    bool bad = false;
+    // the pair stage also forms S (FP64) or its beta part (mixed), which
+    // MODE_BCS needs too
+    if constexpr (is_df<R>::value) {
+        R* xr = at<R>(sm, c.L.xr);
+        for (int i = threadIdx.x; i < n3; i += NT) xr[i] = from_dbl<R>(x[i]);
+        __syncthreads();
+        pair_stage<R>(c, jt);
+    } else {
+        fix_positions(c);
+        bad = pair_stage64(c, mode, jt);
+    }
+    if (p.ieq && mode != MODE_BCS) same_spin_stage(c, ss);
     double su = 0.0, sv = 0.0, sd2 = 0.0;
     if (mode == MODE_BCS) {
         for (int i = threadIdx.x; i < n3; i += NT) du[i] = 0.0;
@@ -2007,12 +2212,22 @@ __device__ HRes hpsi_eval(const Ctx<R, NT, BIG>& c, int mode)
     int sgn = 1;
     bool ok = true;
     if (mode != MODE_GETPHI) {
-        orbital_stage<R>(c);
-        gemm_stage<R>(c);
+        if constexpr (is_df<R>::value) {
+            orbital_stage<R>(c);
+            gemm_stage<R>(c);
+        } else {
+            unpaired_entries(c);
+            __syncthreads();
+        }
         ok = inverse_stage<R>(c, logdet, sgn);
-        if (ok) {
-            drift_stage<R>(c);
-            beta_drift_stage<R>(c);
+        if (ok && !(mode == MODE_BCS && c.a.inv_only)) {
+            if constexpr (is_df<R>::value) {
+                drift_stage<R>(c);
+                beta_drift_stage<R>(c);
+            } else {
+                pair_drift64(c);
+                unpaired_drift(c);
+            }
         } else {
             for (int i = threadIdx.x; i < 4 * P; i += NT) acc[i] = 0.0;
             __syncthreads();
@@ -2110,6 +2325,7 @@ __device__ HRes hpsi_eval(const Ctx<R, NT, BIG>& c, int mode)
     }
     __syncthreads();
     h = s_h;
+    h.bad = bad;
     if (p.a2 == 0.0 || (mode != MODE_HPSI && mode != MODE_STEP)) {
         h.psigl = h.psil;
         h.d2psig = h.d2psi;

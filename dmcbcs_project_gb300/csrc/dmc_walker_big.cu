@@ -36,7 +36,7 @@ static int set_smem_attr_big(int v)
                                      v);
 }
 
-cudaError_t walker_big_attrs(int smem)
+cudaError_t walker_big_attrs(int smem, bool mixed, bool gf)
 {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -56,10 +56,13 @@ cudaError_t walker_big_attrs(int smem)
                                      cudaFuncAttributePreferredSharedMemoryCarveout, c);
         return (int)r;
     });
-    if (!rc) rc = g_attr_big.ensure(dev, 1, smem, set_smem_attr_big<double, false>);
-    if (!rc) rc = g_attr_big.ensure(dev, 2, smem, set_smem_attr_big<df, false>);
-    if (!rc) rc = g_attr_big.ensure(dev, 3, smem, set_smem_attr_big<double, true>);
-    if (!rc) rc = g_attr_big.ensure(dev, 4, smem, set_smem_attr_big<df, true>);
+    if (rc) return (cudaError_t)rc;
+    if (mixed)
+        rc = gf ? g_attr_big.ensure(dev, 4, smem, set_smem_attr_big<df, true>)
+                : g_attr_big.ensure(dev, 2, smem, set_smem_attr_big<df, false>);
+    else
+        rc = gf ? g_attr_big.ensure(dev, 3, smem, set_smem_attr_big<double, true>)
+                : g_attr_big.ensure(dev, 1, smem, set_smem_attr_big<double, false>);
     return (cudaError_t)rc;
 }
 
@@ -67,7 +70,7 @@ cudaError_t launch_walker_big(const DevParams& p, const KernelArgs& a, const Sme
                               bool mixed, bool gf)
 {
     const size_t smem = (size_t)L.total * 8;
-    const cudaError_t e = walker_big_attrs((int)smem);
+    const cudaError_t e = walker_big_attrs((int)smem, mixed, gf);
     if (e != cudaSuccess) return e;
     if (!a.gscratch) return cudaErrorInvalidValue;   // the union region needs the scratch slices
     if (gf) {

@@ -32,7 +32,7 @@ static int set_smem_attr_gf(int v)
     return (int)cudaFuncSetAttribute(walker_kernel<R, NT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
 }
 
-cudaError_t walker_gf_attrs(int smem, int nt, bool both, bool mixed)
+cudaError_t walker_gf_attrs(int smem, int nt, bool mixed)
 {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -51,23 +51,19 @@ cudaError_t walker_gf_attrs(int smem, int nt, bool both, bool mixed)
     });
     if (rc) return (cudaError_t)rc;
     const bool wide = nt != kThreads;
-    if (both || mixed) {
+    if (mixed)
         rc = g_attr_gf.ensure(dev, wide ? 3 : 2, smem,
                               wide ? set_smem_attr_gf<df, 2 * kThreads> : set_smem_attr_gf<df, kThreads>);
-        if (rc) return (cudaError_t)rc;
-    }
-    if (both || !mixed) {
+    else
         rc = g_attr_gf.ensure(dev, 1, smem, set_smem_attr_gf<double, kThreads>);
-        if (rc) return (cudaError_t)rc;
-    }
-    return cudaSuccess;
+    return (cudaError_t)rc;
 }
 
 cudaError_t launch_walker_gf(const DevParams& p, const KernelArgs& a, const SmemLayout& L, int grid, cudaStream_t st,
                              bool mixed)
 {
     const size_t smem = (size_t)L.total * 8;
-    const cudaError_t e = walker_gf_attrs((int)smem, L.nt, false, mixed);
+    const cudaError_t e = walker_gf_attrs((int)smem, L.nt, mixed);
     if (e != cudaSuccess) return e;
     if (!mixed)
         walker_kernel<double, kThreads, true><<<grid, kThreads, smem, st>>>(p, a, L);

@@ -207,9 +207,13 @@ walker_kernel(const __grid_constant__ DevParams p, const __grid_constant__ Kerne
 {
     extern __shared__ __align__(16) double sm[];
     const int P = p.npart, n3 = 3 * P;
-    const double* kvsrc = reinterpret_cast<const double*>(walker::Prec<R>::kv(a));
-    for (int i = threadIdx.x; i < p.nk * 8; i += NT) sm[L.kq + i] = kvsrc[i];
-    {
+    if constexpr (!walker::is_df<R>::value) {
+        // FP64 path: the pair function's fixed-point coefficients
+        const double* src = reinterpret_cast<const double*>(a.phi);
+        for (int i = threadIdx.x; i < (int)(sizeof(PhiFix) / 8); i += NT) sm[L.kq + i] = src[i];
+    } else {
+        const double* kvsrc = reinterpret_cast<const double*>(walker::Prec<R>::kv(a));
+        for (int i = threadIdx.x; i < p.nk * 8; i += NT) sm[L.kq + i] = kvsrc[i];
         using KV = typename walker::Prec<R>::KV;
         const KV* kg = walker::Prec<R>::kv(a);
         R* ks = walker::at<R>(sm, L.ksoa);
@@ -332,7 +336,14 @@ walker_kernel(const __grid_constant__ DevParams p, const __grid_constant__ Kerne
         // not finite (NaN or infinite positions, overflowing terms).  Ends
         // with a barrier, after which the evaluation's shared data may change.
         auto flag_walker = [&](const HRes& hh) {
-            int bad = 0;
+            int bad = hh.bad;
+            if (a.mode == MODE_BCS && a.inv_only && !hh.singular) {
+                // no drift to look at: it is finite when the inverse is
+                const R* Si = walker::at<R>(sm, L.S);
+                const int nd = p.nd;
+                for (int e = threadIdx.x; e < nd * nd; e += NT)
+                    if (!isfinite(to_double(Si[(e / nd) * p.ldS + e % nd]))) bad = 1;
+            }
             for (int e = threadIdx.x; e < n3; e += NT) {
                 const double val = a.mode == MODE_GETPHI ? sm[L.acc + 4 * P + e] : dpsi[e];
                 if (!isfinite(val)) bad = 1;
