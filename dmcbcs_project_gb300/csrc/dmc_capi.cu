@@ -138,6 +138,7 @@ struct dmc_ctx {
     DevBuf<TabPoly> tpoly;          // FP64 walker path: tables by grid interval
     DevBuf<PhiFix> phi;             // and the pair function's fixed-point coefficients
     DevBuf<long long> phi_oct;
+    bool phi_sym = false;           // in the symmetric form
     int precision = DMC_PREC_FP64;
     DevBuf<unsigned long long> jumpA, jumpC;
     DevBuf<double> gscratch;
@@ -381,6 +382,7 @@ int upload_phi(dmc_ctx* c)
     F.sphi = bad * sc / one;
     F.sgrad = bad * -kap * sc / one * (F.fast ? 4.0 : (double)(1 << F.kM));
     F.slap = bad * -kap * kap * sl / one;
+    c->phi_sym = F.fast != 0;
     CK(c->phi.alloc(1));
     CK(cudaMemcpy(c->phi.p, &F, sizeof F, cudaMemcpyHostToDevice));
     CK(c->phi_oct.alloc(oct.size()));
@@ -2116,12 +2118,12 @@ int dmc_add_operators(dmc_ctx* c)
             const int prec = c->precision;
             c->precision = DMC_PREC_FP64;
             int rc = run_eval(c, MODE_BCS, n, s.x.p, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                              nullptr, nullptr, c->ssinv.p, c->stream);
+                              nullptr, nullptr, c->ssinv.p, c->stream, nullptr, true);
             c->precision = prec;
             if (rc) return rc;
             ++c->launches;
-            CK(launch_ops_enk(c->P, o, c->kv.p, c->tud.p, c->tss.p, s.x.p, s.irn.p, c->ssinv.p, n, O.tk.p, c->grid,
-                              c->stream));
+            CK(launch_ops_enk(c->P, o, c->kv.p, c->tud.p, c->tss.p, c->phi.p, c->tpoly.p, c->phi_sym, s.x.p, s.irn.p,
+                              c->ssinv.p, n, O.tk.p, c->nsm, c->stream));
             ++c->launches;
         }
         CK(O.wts.alloc((size_t)n));

@@ -131,8 +131,9 @@ size_t ops_walker_smem(const DevParams& p, const OpsDev& o);
 cudaError_t launch_ops_walker(const DevParams& p, const OpsDev& o, const double* x, int n, int* hg, int* hd,
                               double* sv, int grid, cudaStream_t st);
 cudaError_t launch_ops_enk(const DevParams& p, const OpsDev& o, const KVecDev* kv, const TabUD* tud,
-                           const TabSS* tss, const double* x, const unsigned long long* irn, const double* sinv,
-                           int n, double* tk, int grid, cudaStream_t st);
+                           const TabSS* tss, const PhiFix* phi, const TabPoly* tpoly, bool sym, const double* x,
+                           const unsigned long long* irn, const double* sinv, int n, double* tk, int nsm,
+                           cudaStream_t st);
 // wts: scratch of n doubles for the walker weights
 cudaError_t launch_ops_reduce(const OpsDev& o, int n, const DevStack& s, const int* hg, const int* hd,
                               const double* sv, const double* tk, double* sums, double* wts, cudaStream_t st);

@@ -4,7 +4,7 @@
 // (DFMA, DADD and every conversion to or from double alike), a 64 x 64 -> 128
 // high product (__mul64hi) takes 28 cycles there and a 64-bit add 2.  So
 // whatever is bounded is computed in 64-bit fixed point on the integer pipe
-// (at least 58 fractional bits where a double has 52), and FP64 keeps what
+// (good to 2^-57 or better, where a double's values near 1 are spaced 2^-53), and FP64 keeps what
 // needs a floating exponent: distances, tables, the pair sums.
 #pragma once
 
@@ -35,18 +35,59 @@ __device__ __forceinline__ long long fshl(long long a, int n) { return (long lon
 __device__ __forceinline__ long long fmh(long long a, long long b) { return __mul64hi(a, b); }
 __device__ __forceinline__ long long fmul(long long a, long long b) { return fshl(__mul64hi(a, b), 2); }
 
-// cos and sin of the pair's axis angles 2 pi (x_i - x_j) / L from the
-// particles' tables tr[6][P] (cos, sin per axis)
-__device__ __forceinline__ void pair_axes(const long long* tr, int P, int i, int j, long long (&c)[3], long long (&s)[3],
-                                          bool want_sin)
+// cos and sin of the turn fraction t (2^64 is one turn): the nearest quarter
+// turn off, then the Taylor series in y^2, y = theta / (pi/4), with
+// coefficients (pi/4)^n / n! (the first one left out is below 2^-63).
+// Nineteen high products, where sincospi takes some thirty FP64 instructions.
+__device__ __forceinline__ void fix_sincos(long long t, long long& c, long long& s)
+{
+    // (-1)^k (pi/4)^(2k) / (2k)! and (-1)^k (pi/4)^(2k+1) / (2k+1)!
+    constexpr long long kc[10] = {
+        4611686018427387904ll, -1422359894497287770ll, 73115257680538683ll, -1503372227063806ll, 16559920924893ll,
+        -113499908640ll, 530397347ll, -1797669ll, 4620ll, -9ll};
+    constexpr long long ks[9] = {
+        3622009729038561421ll, -372372949609452720ll, 11484917819725252ll, -168677969434092ll, 1445125720046ll,
+        -8103874527ll, 32044085ll, -94126ll, 213ll};
+    const unsigned q = (unsigned)((unsigned long long)fadd(t, 1ll << 61) >> 62);
+    const long long y = fshl(fsub(t, (long long)((unsigned long long)q << 62)), 1);
+    const long long w = fmul(y, y);
+    long long a = kc[9], b = ks[8];
+#pragma unroll
+    for (int k = 8; k >= 0; --k) a = fadd(kc[k], fmul(a, w));
+#pragma unroll
+    for (int k = 7; k >= 0; --k) b = fadd(ks[k], fmul(b, w));
+    b = fmul(b, y);
+    const long long cc = (q & 1u) ? b : a, ss = (q & 1u) ? a : b;
+    c = (q == 1u || q == 2u) ? -cc : cc;
+    s = q >= 2u ? -ss : ss;
+}
+
+// x / L as a turn fraction: h + l, l the division's remainder, so that the
+// fraction is exact to 2^-64 whatever the coordinate
+__device__ __forceinline__ long long box_fraction(double x, double el, double eli)
+{
+    const double two64 = 18446744073709551616.0;
+    const double h = x * eli, l = fma(-h, el, x) * eli;
+    return fadd(__double2ll_rn((h - rint(h)) * two64), __double2ll_rn(l * two64));
+}
+
+// cos and sin of the axis angles between a point (ci, si) and particle j of
+// the table tr[6][P] (cos, sin per axis)
+__device__ __forceinline__ void rel_axes(const long long (&ci)[3], const long long (&si)[3], const long long* tr, int P,
+                                         int j, long long (&c)[3], long long (&s)[3], bool want_sin)
 {
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const long long ci = tr[(2 * a) * P + i], si = tr[(2 * a + 1) * P + i];
         const long long cj = tr[(2 * a) * P + j], sj = tr[(2 * a + 1) * P + j];
-        c[a] = fshl(fadd(fmh(ci, cj), fmh(si, sj)), 2);
-        if (want_sin) s[a] = fshl(fsub(fmh(si, cj), fmh(ci, sj)), 2);
+        c[a] = fshl(fadd(fmh(ci[a], cj), fmh(si[a], sj)), 2);
+        if (want_sin) s[a] = fshl(fsub(fmh(si[a], cj), fmh(ci[a], sj)), 2);
     }
+}
+__device__ __forceinline__ void pair_axes(const long long* tr, int P, int i, int j, long long (&c)[3], long long (&s)[3],
+                                          bool want_sin)
+{
+    const long long ci[3] = {tr[i], tr[2 * P + i], tr[4 * P + i]}, si[3] = {tr[P + i], tr[3 * P + i], tr[5 * P + i]};
+    rel_axes(ci, si, tr, P, j, c, s, want_sin);
 }
 
 // The pair function's value, gradient with respect to x_i (without its
@@ -63,39 +104,53 @@ struct PhiPair {
 //   d phi / d c_x = 2 a1 + 8 a2 t_x + 8 a3 u_x + 8 a5 w_x + 16 a6 y_x
 //                   + 4 c_x (2 a4 + 8 a5 t_x + 8 a6 u_x),
 // 64 high products for value, gradient and Laplacian, where the plane-wave
-// sums take 3 x 80 multiply-adds at seven shells.
+// sums take 3 x 80 multiply-adds at seven shells.  SymTerms holds d, u, y and
+// the sums e1..e6 (sum c, sum u, sum d, sum y and sum d u in quarters, c_x u_x
+// whole).
+struct SymTerms {
+    long long d[3], u[3], y[3], e[6];
+};
+__device__ __forceinline__ void sym_terms(const long long (&c)[3], SymTerms& t)
+{
+#pragma unroll
+    for (int a = 0; a < 3; ++a) t.d[a] = fsub(fshl(fmh(c[a], c[a]), 3), kFixOne);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const int b = (a + 1) % 3, e = (a + 2) % 3;
+        t.u[a] = fmul(c[b], c[e]);
+        t.y[a] = fshl(fadd(fmh(t.d[b], c[e]), fmh(c[b], t.d[e])), 1);
+    }
+    t.e[0] = (c[0] >> 2) + (c[1] >> 2) + (c[2] >> 2);
+    t.e[1] = (t.u[0] >> 2) + (t.u[1] >> 2) + (t.u[2] >> 2);
+    t.e[2] = fmul(c[0], t.u[0]);
+    t.e[3] = (t.d[0] >> 2) + (t.d[1] >> 2) + (t.d[2] >> 2);
+    t.e[4] = (t.y[0] >> 2) + (t.y[1] >> 2) + (t.y[2] >> 2);
+    t.e[5] = fmh(t.d[0], t.u[0]) + fmh(t.d[1], t.u[1]) + fmh(t.d[2], t.u[2]);
+}
+// sum of six coefficients times e1..e6
+__device__ __forceinline__ long long sym_dot(const long long* f, const long long (&e)[6])
+{
+    return fshl(fadd(fadd(fadd(fmh(f[0], e[0]), fmh(f[1], e[1])), fadd(fmh(f[2], e[2]), fmh(f[3], e[3]))),
+                     fadd(fmh(f[4], e[4]), fmh(f[5], e[5]))), 2);
+}
 __device__ __forceinline__ void phi_sym(const PhiFix* F, const long long* tr, int P, int i, int j, bool all, PhiPair& o)
 {
-    long long c[3], s[3], d[3], u[3], y[3];
+    long long c[3], s[3];
+    SymTerms q;
     pair_axes(tr, P, i, j, c, s, all);
-#pragma unroll
-    for (int a = 0; a < 3; ++a) d[a] = fsub(fshl(fmh(c[a], c[a]), 3), kFixOne);
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const int b = (a + 1) % 3, e = (a + 2) % 3;
-        u[a] = fmul(c[b], c[e]);
-        y[a] = fshl(fadd(fmh(d[b], c[e]), fmh(c[b], d[e])), 1);
-    }
-    // sums in quarters (each at most 3)
-    const long long e1 = (c[0] >> 2) + (c[1] >> 2) + (c[2] >> 2);
-    const long long e2 = (u[0] >> 2) + (u[1] >> 2) + (u[2] >> 2);
-    const long long e3 = fmul(c[0], u[0]);
-    const long long e4 = (d[0] >> 2) + (d[1] >> 2) + (d[2] >> 2);
-    const long long e5 = (y[0] >> 2) + (y[1] >> 2) + (y[2] >> 2);
-    const long long e6 = fmh(d[0], u[0]) + fmh(d[1], u[1]) + fmh(d[2], u[2]);
+    sym_terms(c, q);
     const long long* f = F->f;
-    o.f = fadd(f[0], fshl(fadd(fadd(fadd(fmh(f[1], e1), fmh(f[2], e2)), fadd(fmh(f[3], e3), fmh(f[4], e4))),
-                               fadd(fmh(f[5], e5), fmh(f[6], e6))), 2));
+    o.f = fadd(f[0], sym_dot(f + 1, q.e));
     if (!all) return;
-    o.l = fshl(fadd(fadd(fadd(fmh(f[7], e1), fmh(f[8], e2)), fadd(fmh(f[9], e3), fmh(f[10], e4))),
-                    fadd(fmh(f[11], e5), fmh(f[12], e6))), 2);
+    o.l = sym_dot(f + 7, q.e);
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const int b = (a + 1) % 3, e = (a + 2) % 3;
-        const long long t = (c[b] >> 1) + (c[e] >> 1), w = (d[b] >> 1) + (d[e] >> 1);
+        const long long t = (c[b] >> 1) + (c[e] >> 1), w = (q.d[b] >> 1) + (q.d[e] >> 1);
         // the brackets are at most 1; their sum in quarters
-        const long long p1 = fadd(f[13] >> 2, fadd(fadd(fmh(f[14], t), fmh(f[15], u[a])), fadd(fmh(f[16], w), fmh(f[17], y[a]))));
-        const long long p2 = fadd(f[18], fshl(fadd(fmh(f[19], t), fmh(f[20], u[a])), 2));
+        const long long p1 = fadd(f[13] >> 2, fadd(fadd(fmh(f[14], t), fmh(f[15], q.u[a])),
+                                                   fadd(fmh(f[16], w), fmh(f[17], q.y[a]))));
+        const long long p2 = fadd(f[18], fshl(fadd(fmh(f[19], t), fmh(f[20], q.u[a])), 2));
         o.g[a] = fmul(s[a], fadd(p1, fmul(c[a], p2)));
     }
 }

@@ -41,6 +41,27 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
+// Warp sums of eight values with nine additions instead of forty: each step
+// halves the values a lane carries, then the lanes.  Lane l returns the sum of
+// v[l >> 2].
+__device__ __forceinline__ double warp_sum8(double (&v)[8])
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int n = 4, o = 16; n > 0; n >>= 1, o >>= 1) {
+        const bool hi = (lane & o) != 0;
+#pragma unroll
+        for (int k = 0; k < n; ++k) {
+            const double keep = hi ? v[k + n] : v[k], send = hi ? v[k] : v[k + n];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    double t = v[0];
+    t += __shfl_xor_sync(0xffffffffu, t, 2);
+    t += __shfl_xor_sync(0xffffffffu, t, 1);
+    return t;
+}
+
 // Deterministic block sum of NV values (fixed tree); the result is returned
 // in v on every thread.
 template <int NV, int NT = kThreads>
@@ -519,8 +540,6 @@ __device__ void same_spin_stage(const Ctx<R, NT, BIG>& c, double (&ss)[3])
 // (differences then wrap to the minimum image by themselves), the axis
 // angles' cos and sin, and a flag per particle with a coordinate that is not
 // finite (such a particle's pairs get NaN, as its distances would).
-// x / L is formed as h + l, l the division's remainder, so that a fraction is
-// exact to 2^-64 whatever the coordinate.
 // ---------------------------------------------------------------------------
 template <int NT, bool BIG>
 __device__ void fix_positions(const Ctx<double, NT, BIG>& c)
@@ -531,17 +550,11 @@ __device__ void fix_positions(const Ctx<double, NT, BIG>& c)
     long long* xf = at<long long>(sm, c.L.xr);
     long long* tr = c.template uat<long long>(c.L.trig);
     int* nf = reinterpret_cast<int*>(sm + c.L.acc + 7 * p.npart);
-    const double two64 = 18446744073709551616.0;
     for (int t = threadIdx.x; t < 3 * p.npart; t += NT) {
         const int pt = t / 3, a = t - 3 * pt;
-        const double xv = x[t];
-        const double h = xv * p.eli, l = fma(-h, p.el, xv) * p.eli;
-        const double hf = h - rint(h);
-        xf[t] = fadd(__double2ll_rn(hf * two64), __double2ll_rn(l * two64));
-        double sn, cs;
-        sincospi(2.0 * hf, &sn, &cs);
-        tr[(2 * a) * p.npart + pt] = __double2ll_rn(cs * kFixScale);
-        tr[(2 * a + 1) * p.npart + pt] = __double2ll_rn(sn * kFixScale);
+        const long long f = box_fraction(x[t], p.el, p.eli);
+        xf[t] = f;
+        fix_sincos(f, tr[(2 * a) * p.npart + pt], tr[(2 * a + 1) * p.npart + pt]);
         if (a == 0) nf[pt] = !(isfinite(x[t]) && isfinite(x[t + 1]) && isfinite(x[t + 2]));
     }
     __syncthreads();
