@@ -1682,7 +1682,7 @@ int dmc_bcsone_batch(dmc_ctx* c, int nw, const double* x, const double* smati, c
     if ((rc = stage_moves(c, nw, x, ipart, dr))) return rc;
     CK(c->ssinv.alloc(nw * nd2));
     CK(cudaMemcpyAsync(c->ssinv.p, smati, nw * nd2 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    CK(launch_bcsone(c->P, c->kv.p, c->tud.p, c->sx.p, c->ssinv.p, c->sip.p, c->sdr.p, c->sratio.p, nw, c->stream));
+    CK(launch_bcsone(c->P, c->kv.p, c->tud.p, c->phi.p, c->tpoly.p, c->phi_sym, c->sx.p, c->ssinv.p, c->sip.p, c->sdr.p, c->sratio.p, nw, c->stream));
     ++c->launches;
     CK(cudaMemcpyAsync(ratio, c->sratio.p, nw * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -1695,7 +1695,7 @@ int dmc_getphione_batch(dmc_ctx* c, int nw, const double* x, const int* ipart, c
     int rc = check_moves(c, nw, x, ipart, drr, ratio);
     if (rc || nw == 0) return rc;
     if ((rc = stage_moves(c, nw, x, ipart, drr))) return rc;
-    CK(launch_getphione(c->P, c->tud.p, c->tss.p, c->sx.p, c->sip.p, c->sdr.p, c->sratio.p, nw, c->stream));
+    CK(launch_getphione(c->P, c->tpoly.p, c->tud.p, c->tss.p, c->sx.p, c->sip.p, c->sdr.p, c->sratio.p, nw, c->stream));
     ++c->launches;
     CK(cudaMemcpyAsync(ratio, c->sratio.p, nw * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -1710,11 +1710,11 @@ static int derbcs_device(dmc_ctx* c, int nw, const double* dx, double* dder, int
     const int prec = c->precision;
     c->precision = DMC_PREC_FP64;
     int rc = run_eval(c, MODE_BCS, nw, dx, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                      nullptr, c->ssinv.p, c->stream);
+                      nullptr, c->ssinv.p, c->stream, nullptr, true);
     c->precision = prec;
     if (rc) return rc;
     ++c->launches;
-    CK(launch_derbcs(c->P, c->kv.p, dx, c->ssinv.p, dder, nw, c->grid, c->stream, stride, off));
+    CK(launch_derbcs(c->P, c->kv.p, dx, c->ssinv.p, dder, nw, c->grid, c->stream, stride, off, c->phi_sym));
     ++c->launches;
     return DMC_OK;
 }
@@ -1862,7 +1862,7 @@ int dmc_sm_sweeps(dmc_ctx* c, int nsweeps, int recompute_every, int64_t* accepte
     if (accepted) *accepted = 0;
     if (moves) *moves = 0;
     if (nsweeps == 0) return DMC_OK;   // nothing moves; the walkers keep their values
-    const size_t nd2 = (size_t)c->S.nd * c->S.nd, n3 = (size_t)c->n3;
+    const size_t nd2 = (size_t)c->S.nd * c->S.nd;
     const int nq = std::max(1, c->S.nk - 1);
     c->sm_n = 0;                       // no carried inverse until these sweeps end
     CK(c->sm_inv.alloc((size_t)n * nd2));
@@ -1895,11 +1895,10 @@ int dmc_sm_sweeps(dmc_ctx* c, int nsweeps, int recompute_every, int64_t* accepte
         const bool fresh = done == 0 || recompute_every > 0;
         if (fresh) {
             CK(c->ssinv.alloc((size_t)n * nd2));
-            CK(c->pg_dphi.alloc((size_t)n * n3));
             const int prec = c->precision;
             c->precision = DMC_PREC_FP64;
-            rc = run_eval(c, MODE_BCS, n, s.x.p, nullptr, nullptr, c->pg_dphi.p, nullptr, nullptr, nullptr, nullptr,
-                          nullptr, nullptr, c->ssinv.p, c->stream);
+            rc = run_eval(c, MODE_BCS, n, s.x.p, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
+                          nullptr, nullptr, c->ssinv.p, c->stream, nullptr, true);
             c->precision = prec;
             if (rc) return rc;
             ++c->launches;

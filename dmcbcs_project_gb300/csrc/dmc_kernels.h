@@ -63,11 +63,13 @@ cudaError_t launch_popctl(const int* pn, double nwalk, double popup, double popd
                           int* flags, cudaStream_t st);
 
 // Single-particle ratios and parameter derivatives (dmc_single.cu)
-cudaError_t launch_bcsone(const DevParams& p, const KVecDev* kv, const TabUD* tud, const double* x,
-                          const double* smati, const int* ipart, const double* dr, double* ratio, int nw,
-                          cudaStream_t st);
-cudaError_t launch_getphione(const DevParams& p, const TabUD* tud, const TabSS* tss, const double* x,
-                             const int* ipart, const double* drr, double* ratio, int nw, cudaStream_t st);
+// (sym: the shells are in the symmetric fixed-point form, phi->fast)
+cudaError_t launch_bcsone(const DevParams& p, const KVecDev* kv, const TabUD* tud, const PhiFix* phi,
+                          const TabPoly* tpoly, bool sym, const double* x, const double* smati, const int* ipart,
+                          const double* dr, double* ratio, int nw, cudaStream_t st);
+cudaError_t launch_getphione(const DevParams& p, const TabPoly* tpoly, const TabUD* tud, const TabSS* tss,
+                             const double* x, const int* ipart, const double* drr, double* ratio, int nw,
+                             cudaStream_t st);
 // walker arrays in host memory the device addresses directly (pinned and
 // mapped, or managed), laid out as dmc_walkers
 struct HostWalkers {
@@ -114,7 +116,7 @@ cudaError_t launch_sweeps(const DevParams& p, const DevStack& st, int n, int nsw
                           double* prop, cudaStream_t stream);
 // dpsi[w*stride + off + shell]; stride < 0 means norb
 cudaError_t launch_derbcs(const DevParams& p, const KVecDev* kv, const double* x, const double* smati, double* dpsi,
-                          int nw, int grid, cudaStream_t st, int stride = -1, int off = 0);
+                          int nw, int grid, cudaStream_t st, int stride = -1, int off = 0, bool sym = false);
 // getjasder: dpsi[w*stride + 0..1] = d U_long / d beta, d U_long / d gamma
 cudaError_t launch_jasder(const DevParams& p, const double* jq, const double* x, double* dpsi, int nw, int grid,
                           cudaStream_t st, int stride);

@@ -28,6 +28,62 @@ namespace dmc {
 
 namespace {
 
+// Single-particle ratios: kMoveThreads threads per walker (33 partners at
+// N = 66 in one round; a call is often a few dozen walkers, so latency counts).
+constexpr int kMoveThreads = 64;
+
+__device__ __forceinline__ double move_sum(double v)
+{
+    __shared__ double red[kMoveThreads / 32];
+    v = walker::warp_sum(v);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double t = red[0];
+#pragma unroll
+    for (int k = 1; k < kMoveThreads / 32; ++k) t += red[k];
+    return t;
+}
+
+// bcsone (psislaterbcs.f90:296-376) with the shells in the symmetric form: an
+// entry is one polynomial of the displacement's axis cosines in fixed point
+// instead of a cosine per k vector (64 walkers at N = 66: 144 -> 10 us)
+__global__ void __launch_bounds__(kMoveThreads) bcsone_sym_kernel(const __grid_constant__ DevParams p,
+                                                                 const PhiFix* __restrict__ F,
+                                                                 const TabPoly* __restrict__ tpoly,
+                                                                 const double* __restrict__ x,
+                                                                 const double* __restrict__ smati,
+                                                                 const int* __restrict__ ipart,
+                                                                 const double* __restrict__ dr,
+                                                                 double* __restrict__ ratio)
+{
+    const int w = blockIdx.x, P = p.npart, nd = p.nd;
+    const double* xw = x + (size_t)w * 3 * P;
+    const double* S = smati + (size_t)w * nd * nd;
+    const int i = ipart[w] - 1;   // checked on the host
+    const bool up = i < p.nup;
+    const double xi[3] = {xw[3 * i] - dr[3 * w], xw[3 * i + 1] - dr[3 * w + 1], xw[3 * i + 2] - dr[3 * w + 2]};
+    const int nloop = up ? p.ndn : p.nup, j0 = up ? p.nup : 0;
+    double acc = 0.0;
+    for (int q = threadIdx.x; q < nd; q += kMoveThreads) {
+        double ph;
+        if (q < nloop) {
+            double d[3];
+            for (int c = 0; c < 3; ++c) d[c] = xi[c] - xw[3 * (j0 + q) + c];
+            ph = single::phi_beta_sym(p, F, tpoly, d);
+        } else {
+            // unpaired plane wave of the moved particle (psislaterbcs.f90:352-365)
+            const int u = q - nloop;
+            const double* k = up ? p.akup[u] : p.akdn[u];
+            const double arg = k[0] * xi[0] + k[1] * xi[1] + k[2] * xi[2];
+            ph = (up ? p.sinup[u] : p.sindn[u]) ? sin(arg) : cos(arg);
+        }
+        // up: row i of S replaced, ratio = sum_q Sinv(q,i) phi_q; down: column
+        acc = fma(up ? S[q + (size_t)i * nd] : S[(i - p.nup) + (size_t)q * nd], ph, acc);
+    }
+    const double r = move_sum(acc);
+    if (threadIdx.x == 0) ratio[w] = r;
+}
+
 __global__ void bcsone_kernel(const __grid_constant__ DevParams p, const KVecDev* __restrict__ kv,
                               const TabUD* __restrict__ tud, const double* __restrict__ x,
                               const double* __restrict__ smati, const int* __restrict__ ipart,
@@ -44,20 +100,97 @@ __global__ void bcsone_kernel(const __grid_constant__ DevParams p, const KVecDev
     if (lane == 0) ratio[w] = r;
 }
 
-__global__ void getphione_kernel(const __grid_constant__ DevParams p, const TabUD* __restrict__ tud,
-                                 const TabSS* __restrict__ tss, const double* __restrict__ x,
-                                 const int* __restrict__ ipart, const double* __restrict__ drr,
-                                 double* __restrict__ ratio, int nw)
+__global__ void __launch_bounds__(kMoveThreads) getphione_kernel(const __grid_constant__ DevParams p,
+                                                                const TabPoly* __restrict__ tpoly,
+                                                                const TabUD* __restrict__ tud,
+                                                                const TabSS* __restrict__ tss,
+                                                                const double* __restrict__ x,
+                                                                const int* __restrict__ ipart,
+                                                                const double* __restrict__ drr,
+                                                                double* __restrict__ ratio)
 {
-    const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (w >= nw) return;
-    const double* xw = x + (size_t)w * 3 * p.npart;
-    const double d[3] = {drr[3 * w], drr[3 * w + 1], drr[3 * w + 2]};
-    const double r = single::warp_getphione(p, tud, tss, xw, ipart[w] - 1, d);
-    if (lane == 0) ratio[w] = r;
+    const int w = blockIdx.x, P = p.npart;
+    const double* xw = x + (size_t)w * 3 * P;
+    const int i = ipart[w] - 1;
+    const bool up = i < p.nup;
+    // opposite-spin partners first, then (equal-spin Jastrow on) the others
+    const int no = up ? p.ndn : p.nup, o0 = up ? p.nup : 0, s0 = up ? 0 : p.nup;
+    const int cnt = p.ieq ? P : no;
+    double u = 0.0;
+    for (int q = threadIdx.x; q < cnt; q += kMoveThreads) {
+        const bool opp = q < no;
+        const int j = opp ? o0 + q : s0 + q - no;
+        if (j == i) continue;
+        double a[3], b[3];
+        for (int c = 0; c < 3; ++c) {
+            const double d = xw[3 * i + c] - xw[3 * j + c], e = d - drr[3 * w + c];
+            a[c] = d - p.el * single::fnint(d * p.eli);
+            b[c] = e - p.el * single::fnint(e * p.eli);
+        }
+        const double ro = single::length(a), rn = single::length(b);
+        u += opp ? single::jastrow_ud(p, tpoly, rn) - single::jastrow_ud(p, tpoly, ro)
+                 : single::jastrow_u(p, tud, tss, false, fmax(rn, 1.0e-14)) -
+                       single::jastrow_u(p, tud, tss, false, fmax(ro, 1.0e-14));
+    }
+    const double t = move_sum(u);
+    if (threadIdx.x == 0) ratio[w] = exp(t);
 }
 
+// d log|det| / d vorb(shell) with the shells in the symmetric form (at most
+// seven, |n|^2 = shell - 1): tr(S^-1 dS/dvorb) is the inverse's up-down block
+// against each pair's shell sums e1..e6, which come from one set of axis
+// cosines.  One walker per CTA; 13 FP64 instructions a pair.
+__global__ void __launch_bounds__(kThreads) derbcs_sym_kernel(const __grid_constant__ DevParams p,
+                                                             const double* __restrict__ x,
+                                                             const double* __restrict__ smati,
+                                                             double* __restrict__ dpsi, int nw, int stride, int off)
+{
+    using namespace walker;
+    __shared__ long long tr[6 * DMC_MAX_PART];
+    __shared__ int nf[DMC_MAX_PART];
+    __shared__ double red[kWarps][8];
+    const int nd = p.nd, nup = p.nup, ndn = p.ndn, P = p.npart;
+    // e1..e6 in their units: 2 sum c, 4 sum u, 8 c_x u_x, 2 sum d, 8 sum y, 8 sum d u
+    const double unit[6] = {8.0, 16.0, 8.0, 8.0, 32.0, 32.0};
+    for (int w = blockIdx.x; w < nw; w += gridDim.x) {
+        const double* xw = x + (size_t)w * 3 * P;
+        const double* Si = smati + (size_t)w * nd * nd;
+        for (int t = threadIdx.x; t < 3 * P; t += kThreads) {
+            const int pt = t / 3, a = t - 3 * pt;
+            fix_sincos(box_fraction(xw[t], p.el, p.eli), tr[(2 * a) * P + pt], tr[(2 * a + 1) * P + pt]);
+            if (a == 0) nf[pt] = !(isfinite(xw[t]) && isfinite(xw[t + 1]) && isfinite(xw[t + 2]));
+        }
+        __syncthreads();
+        double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        const UDiv dv(ndn > 0 ? ndn : 1);
+        for (int t = threadIdx.x; t < nup * ndn; t += kThreads) {
+            const int i = dv.quo(t), j = t - i * ndn;
+            double a = Si[j + (size_t)i * nd];
+            long long c[3], s[3];
+            SymTerms q;
+            pair_axes(tr, P, i, nup + j, c, s, false);
+            sym_terms(c, q);
+            acc[0] += a;
+            if (nf[i] | nf[nup + j]) a = __longlong_as_double(0x7ff8000000000000ll);
+#pragma unroll
+            for (int k = 0; k < 6; ++k)
+                if (k + 1 < p.norb) acc[k + 1] = fma(a, (double)q.e[k], acc[k + 1]);
+        }
+        const double v = warp_sum8(acc);
+        const int lane = threadIdx.x & 31;
+        if ((lane & 3) == 0) red[threadIdx.x >> 5][lane >> 2] = v;
+        __syncthreads();
+        if ((int)threadIdx.x < p.norb) {
+            double t = 0.0;
+            for (int k = 0; k < kWarps; ++k) t += red[k][threadIdx.x];
+            if (threadIdx.x > 0) t *= unit[threadIdx.x - 1] * (1.0 / kFixScale);
+            dpsi[(size_t)w * stride + off + threadIdx.x] = t;
+        }
+        __syncthreads();
+    }
+}
+
+// The same for any shells:
 // d log|det| / d vorb(shell) for one walker per CTA.  smati is the inverse in
 // the reference's column-major layout: smati[j + i*nd] = inv(S)[j][i].
 //  shell 1: sum over the up-down block of inv(S)[j][i];
@@ -584,51 +717,79 @@ __global__ void sr_energy_kernel(const double* __restrict__ d2psi, const double*
         ene[w] = __ddiv_rn(__ddiv_rn(__dadd_rn(__dmul_rn(-hbar, d2psi[w]), v[w]), eunit), npart);
 }
 
-__global__ void sr_sums_kernel(const double* __restrict__ der, const double* __restrict__ ene, int n, int np,
-                               double* __restrict__ sums)
+// Bound: the serial chain of one addition per walker (65 cycles each).  One
+// warp per CTA adds 32 outputs' chains; the other three make the next tile's
+// products meanwhile, so nothing but the addition is on the chain (loads and
+// products on it too, in one CTA: 0.95 ms for 2048 walkers and 65 sums).
+constexpr int kSrTile = 64, kSrOut = 32;
+
+__global__ void __launch_bounds__(128) sr_sums_kernel(const double* __restrict__ der, const double* __restrict__ ene,
+                                                      int n, int np, double* __restrict__ sums)
 {
-    const int nout = np * np + 2 * np + 2;
-    for (int t = threadIdx.x; t < nout; t += blockDim.x) {
-        double s = sums[t];
-        for (int w = n - 1; w >= 0; --w) {
+    __shared__ double term[2][kSrTile][kSrOut + 1];
+    const int nout = np * np + 2 * np + 2, o0 = blockIdx.x * kSrOut;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = o0 + lane;
+    const int ntile = (n + kSrTile - 1) / kSrTile;
+    // the terms of tile k (walkers n-1 - k kSrTile downwards), every third row by each of three warps
+    auto fill = [&](int k) {
+        if (t >= nout) return;
+        for (int r = warp - 1; r < kSrTile; r += 3) {
+            const int w = n - 1 - k * kSrTile - r;
+            if (w < 0) break;
             const double e = ene[w];
             const double* d = der + (size_t)w * np;
-            double term;
+            double v;
             if (t < np)
-                term = d[t];
+                v = d[t];
             else if (t < 2 * np)
-                term = __dmul_rn(d[t - np], e);
+                v = __dmul_rn(d[t - np], e);
             else if (t < 2 * np + np * np) {
                 const int q = t - 2 * np, i = q % np, j = q / np;   // column-major pmat(i,j)
-                term = __dmul_rn(d[i], d[j]);
-            } else if (t == nout - 2)
-                term = e;
-            else
-                term = __dmul_rn(e, e);
-            s = __dadd_rn(s, term);
+                v = __dmul_rn(d[i], d[j]);
+            } else
+                v = t == nout - 2 ? e : __dmul_rn(e, e);
+            term[k & 1][r][lane] = v;
         }
-        sums[t] = s;
+    };
+    double s = warp == 0 && t < nout ? sums[t] : 0.0;
+    if (warp > 0) fill(0);
+    __syncthreads();
+    for (int k = 0; k < ntile; ++k) {
+        if (warp == 0) {
+            if (t < nout) {
+                const int m = min(kSrTile, n - k * kSrTile);
+                for (int r = 0; r < m; ++r) s = __dadd_rn(s, term[k & 1][r][lane]);
+            }
+        } else if (k + 1 < ntile) {
+            fill(k + 1);
+        }
+        __syncthreads();
     }
+    if (warp == 0 && t < nout) sums[t] = s;
 }
 
 }  // namespace
 
-cudaError_t launch_bcsone(const DevParams& p, const KVecDev* kv, const TabUD* tud, const double* x,
-                          const double* smati, const int* ipart, const double* dr, double* ratio, int nw,
-                          cudaStream_t st)
+cudaError_t launch_bcsone(const DevParams& p, const KVecDev* kv, const TabUD* tud, const PhiFix* phi,
+                          const TabPoly* tpoly, bool sym, const double* x, const double* smati, const int* ipart,
+                          const double* dr, double* ratio, int nw, cudaStream_t st)
 {
     if (nw <= 0) return cudaSuccess;
+    if (sym) {
+        bcsone_sym_kernel<<<nw, kMoveThreads, 0, st>>>(p, phi, tpoly, x, smati, ipart, dr, ratio);
+        return cudaGetLastError();
+    }
     const int warps = 8;
     bcsone_kernel<<<(nw + warps - 1) / warps, 32 * warps, 0, st>>>(p, kv, tud, x, smati, ipart, dr, ratio, nw);
     return cudaGetLastError();
 }
 
-cudaError_t launch_getphione(const DevParams& p, const TabUD* tud, const TabSS* tss, const double* x,
-                             const int* ipart, const double* drr, double* ratio, int nw, cudaStream_t st)
+cudaError_t launch_getphione(const DevParams& p, const TabPoly* tpoly, const TabUD* tud, const TabSS* tss,
+                             const double* x, const int* ipart, const double* drr, double* ratio, int nw,
+                             cudaStream_t st)
 {
     if (nw <= 0) return cudaSuccess;
-    const int warps = 8;
-    getphione_kernel<<<(nw + warps - 1) / warps, 32 * warps, 0, st>>>(p, tud, tss, x, ipart, drr, ratio, nw);
+    getphione_kernel<<<nw, kMoveThreads, 0, st>>>(p, tpoly, tud, tss, x, ipart, drr, ratio);
     return cudaGetLastError();
 }
 
@@ -639,9 +800,14 @@ size_t derbcs_smem_bytes(const DevParams& p)
 }
 
 cudaError_t launch_derbcs(const DevParams& p, const KVecDev* kv, const double* x, const double* smati, double* dpsi,
-                          int nw, int grid, cudaStream_t st, int stride, int off)
+                          int nw, int grid, cudaStream_t st, int stride, int off, bool sym)
 {
     if (nw <= 0) return cudaSuccess;
+    if (sym) {
+        // 1.19 -> 0.07 ms for 2048 walkers at N = 66
+        derbcs_sym_kernel<<<nw, kThreads, 0, st>>>(p, x, smati, dpsi, nw, stride < 0 ? p.norb : stride, off);
+        return cudaGetLastError();
+    }
     const size_t smem = derbcs_smem_bytes(p);
     cudaError_t e = cudaFuncSetAttribute(derbcs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -722,7 +888,8 @@ cudaError_t launch_sr_sums(const double* der, const double* d2psi, const double*
 {
     if (n <= 0) return cudaSuccess;
     sr_energy_kernel<<<(n + 255) / 256, 256, 0, st>>>(d2psi, v, n, hbar, eunit, (double)npart, ene);
-    sr_sums_kernel<<<1, 1024, 0, st>>>(der, ene, n, np, sums);
+    const int nout = np * np + 2 * np + 2;
+    sr_sums_kernel<<<(nout + kSrOut - 1) / kSrOut, 128, 0, st>>>(der, ene, n, np, sums);
     return cudaGetLastError();
 }
 

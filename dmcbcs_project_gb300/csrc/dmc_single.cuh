@@ -119,6 +119,50 @@ __device__ __forceinline__ double warp_bcsone_tab(const DevParams& p, const KVec
     return walker::warp_sum(acc);
 }
 
+// |d| of a displacement (FP64; the root's iteration needs a normal
+// single-precision seed)
+__device__ __forceinline__ double length(const double (&d)[3])
+{
+    const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+    if (!(r2 > 1.0e-30 && r2 < 1.0e30)) return sqrt(r2);
+    double r, ri;
+    walker::inv_dist(r2, r, ri);
+    return r;
+}
+
+// The pair function phi(d) with beta for a displacement d of any image, the
+// shells in the symmetric fixed-point form (F->fast): the axis cosines come
+// straight from the displacement's turn fractions, so no table of the
+// particles is needed.
+__device__ __forceinline__ double phi_beta_sym(const DevParams& p, const PhiFix* __restrict__ F,
+                                               const TabPoly* __restrict__ tpoly, double (&d)[3])
+{
+    long long c[3], s[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        walker::fix_sincos(walker::box_fraction(d[a], p.el, p.eli), c[a], s[a]);
+        d[a] -= p.el * fnint(d[a] * p.eli);
+    }
+    walker::SymTerms T;
+    walker::sym_terms(c, T);
+    const double r = length(d);
+    double t;
+    const TabPoly* tp = tpoly + walker::grid_split(r * p.scaleb, p.ntab, t);
+    const double b = (p.nobeta || r > p.rangeb) ? 0.0 : walker::poly3(tp->c[0], t);
+    const double phi = fma((double)walker::fadd(F->f[0], walker::sym_dot(F->f + 1, T.e)), F->sphi, b);
+    return r == r ? phi : r;   // a coordinate that is not a number
+}
+
+// Jastrow u(r) of an opposite-spin pair from the interval polynomials
+__device__ __forceinline__ double jastrow_ud(const DevParams& p, const TabPoly* __restrict__ tpoly, double r)
+{
+    r = fmax(r, 1.0e-14);
+    if (!(r < p.range)) return 0.0;
+    double t;
+    const TabPoly* T = tpoly + walker::grid_split(r * p.scale, p.ntab, t);
+    return walker::poly3(T->c[4], t);
+}
+
 // getphione (coshpot.f90:207-264): exp(U' - U) for particle i (0-based)
 // displaced by -drr.  Called by a whole warp; every lane returns the ratio.
 __device__ __forceinline__ double warp_getphione(const DevParams& p, const TabUD* __restrict__ tud,
