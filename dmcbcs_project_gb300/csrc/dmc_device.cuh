@@ -184,8 +184,7 @@ struct SmemLayout {
                           // the CTA's global scratch slice, at offset 0 of it
     int gstride;          // doubles of global scratch per CTA: the union region
                           // (when not on chip), then the beta pair data (idem)
-    int trig;             // cos, sin of the axis angles in fixed point [6][npart], in the union region
-    int rows_drift;       // mixed layout: rows of pair drift terms per chunk
+    int trig;             // FP64 layout: cos, sin of the axis angles [6][npart]
     int rows64;           // FP64 layout: rows of Jastrow pair vectors per chunk
 };
 
@@ -208,10 +207,8 @@ __host__ __device__ inline SmemLayout make_layout(const DevParams& p, int smem_l
     L.dx = take(n3);              // drift + gaussian displacement (step)
     L.drift = take(n3);           // old drift (step)
     L.dg = take(n3);              // guide-function gradient when a2 != 0
-    // the pair function's coefficients (the room of the k-vector records, which
-    // bounds the systems a context accepts)
-    L.kq = take(p.nk * 8 > (int)(sizeof(PhiFix) / 8) ? p.nk * 8 : (int)(sizeof(PhiFix) / 8));
-    L.ksoa = take(p.nk * 7);      // k-vector fields as arrays (conflict-free reads across k)
+    L.kq = take(p.nk * 8);        // k vector records
+    L.ksoa = take(p.nk * 7);      // the same fields as arrays (conflict-free reads across k)
     L.S = take(p.nd * p.ldS);     // pair matrix -> inverse
     L.colk = take(2 * p.nd + 2);  // pivot column of the unblocked Gauss-Jordan
     L.acc = take(p.npart * 8);    // per particle: drift(3), lap, du(3), spare
@@ -231,13 +228,10 @@ __host__ __device__ inline SmemLayout make_layout(const DevParams& p, int smem_l
     const int row_pairs = p.ndn > 0 ? p.ndn : 1;
     const int minrows = 1;
     // at least one row of pair data must fit
-    if (rsize < row_pairs * 4 + 6 * p.npart) rsize = row_pairs * 4 + 6 * p.npart;
-    rsize = round_up(rsize, 2);
+    if (rsize < row_pairs * 4) rsize = row_pairs * 4;
     L.un_in_smem = union_global ? 0 : 1;
     if (!union_global) off += round_up(rsize, 2);
     L.rsize = rsize;
-    L.trig = L.R + rsize - 6 * p.npart;
-    L.rows_drift = (rsize - 6 * p.npart) / (row_pairs * 4);
     L.rows_jas = rsize / (row_pairs * 3);
     L.rows_beta = rsize / (row_pairs * 4);
     if (L.rows_jas < minrows) L.rows_jas = minrows;

@@ -31,25 +31,9 @@ __device__ __forceinline__ long long fsub(long long a, long long b)
     return (long long)((unsigned long long)a - (unsigned long long)b);
 }
 __device__ __forceinline__ long long fshl(long long a, int n) { return (long long)((unsigned long long)a << n); }
-// a b / 4 of two fixed-point values (shift left by 2 for the product).
-// MulFull: the exact high half.  MulShort: without the product of the low
-// halves and with the cross terms truncated, at most five units off (2^-57),
-// in about half the instructions; the mixed path's (its values carry 48 bits).
-struct MulFull {
-    static __device__ __forceinline__ long long hi(long long a, long long b) { return __mul64hi(a, b); }
-};
-struct MulShort {
-    static __device__ __forceinline__ long long hi(long long a, long long b)
-    {
-        const int ah = (int)(a >> 32), bh = (int)(b >> 32);
-        const int t = __mulhi(ah, (int)((unsigned)b >> 1)) + __mulhi(bh, (int)((unsigned)a >> 1));
-        return (long long)ah * bh + 2 * (long long)t;
-    }
-};
-template <class M = MulFull>
-__device__ __forceinline__ long long fmh(long long a, long long b) { return M::hi(a, b); }
-template <class M = MulFull>
-__device__ __forceinline__ long long fmul(long long a, long long b) { return fshl(M::hi(a, b), 2); }
+// a b / 4 of two fixed-point values (shift left by 2 for the product)
+__device__ __forceinline__ long long fmh(long long a, long long b) { return __mul64hi(a, b); }
+__device__ __forceinline__ long long fmul(long long a, long long b) { return fshl(__mul64hi(a, b), 2); }
 
 // cos and sin of the turn fraction t (2^64 is one turn): the nearest quarter
 // turn off, then the Taylor series in y^2, y = theta / (pi/4), with
@@ -89,23 +73,21 @@ __device__ __forceinline__ long long box_fraction(double x, double el, double el
 
 // cos and sin of the axis angles between a point (ci, si) and particle j of
 // the table tr[6][P] (cos, sin per axis)
-template <class M = MulFull>
 __device__ __forceinline__ void rel_axes(const long long (&ci)[3], const long long (&si)[3], const long long* tr, int P,
                                          int j, long long (&c)[3], long long (&s)[3], bool want_sin)
 {
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const long long cj = tr[(2 * a) * P + j], sj = tr[(2 * a + 1) * P + j];
-        c[a] = fshl(fadd(fmh<M>(ci[a], cj), fmh<M>(si[a], sj)), 2);
-        if (want_sin) s[a] = fshl(fsub(fmh<M>(si[a], cj), fmh<M>(ci[a], sj)), 2);
+        c[a] = fshl(fadd(fmh(ci[a], cj), fmh(si[a], sj)), 2);
+        if (want_sin) s[a] = fshl(fsub(fmh(si[a], cj), fmh(ci[a], sj)), 2);
     }
 }
-template <class M = MulFull>
 __device__ __forceinline__ void pair_axes(const long long* tr, int P, int i, int j, long long (&c)[3], long long (&s)[3],
                                           bool want_sin)
 {
     const long long ci[3] = {tr[i], tr[2 * P + i], tr[4 * P + i]}, si[3] = {tr[P + i], tr[3 * P + i], tr[5 * P + i]};
-    rel_axes<M>(ci, si, tr, P, j, c, s, want_sin);
+    rel_axes(ci, si, tr, P, j, c, s, want_sin);
 }
 
 // The pair function's value, gradient with respect to x_i (without its
@@ -128,51 +110,48 @@ struct PhiPair {
 struct SymTerms {
     long long d[3], u[3], y[3], e[6];
 };
-template <class M = MulFull>
 __device__ __forceinline__ void sym_terms(const long long (&c)[3], SymTerms& t)
 {
 #pragma unroll
-    for (int a = 0; a < 3; ++a) t.d[a] = fsub(fshl(fmh<M>(c[a], c[a]), 3), kFixOne);
+    for (int a = 0; a < 3; ++a) t.d[a] = fsub(fshl(fmh(c[a], c[a]), 3), kFixOne);
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const int b = (a + 1) % 3, e = (a + 2) % 3;
-        t.u[a] = fmul<M>(c[b], c[e]);
-        t.y[a] = fshl(fadd(fmh<M>(t.d[b], c[e]), fmh<M>(c[b], t.d[e])), 1);
+        t.u[a] = fmul(c[b], c[e]);
+        t.y[a] = fshl(fadd(fmh(t.d[b], c[e]), fmh(c[b], t.d[e])), 1);
     }
     t.e[0] = (c[0] >> 2) + (c[1] >> 2) + (c[2] >> 2);
     t.e[1] = (t.u[0] >> 2) + (t.u[1] >> 2) + (t.u[2] >> 2);
-    t.e[2] = fmul<M>(c[0], t.u[0]);
+    t.e[2] = fmul(c[0], t.u[0]);
     t.e[3] = (t.d[0] >> 2) + (t.d[1] >> 2) + (t.d[2] >> 2);
     t.e[4] = (t.y[0] >> 2) + (t.y[1] >> 2) + (t.y[2] >> 2);
-    t.e[5] = fmh<M>(t.d[0], t.u[0]) + fmh<M>(t.d[1], t.u[1]) + fmh<M>(t.d[2], t.u[2]);
+    t.e[5] = fmh(t.d[0], t.u[0]) + fmh(t.d[1], t.u[1]) + fmh(t.d[2], t.u[2]);
 }
 // sum of six coefficients times e1..e6
-template <class M = MulFull>
 __device__ __forceinline__ long long sym_dot(const long long* f, const long long (&e)[6])
 {
-    return fshl(fadd(fadd(fadd(fmh<M>(f[0], e[0]), fmh<M>(f[1], e[1])), fadd(fmh<M>(f[2], e[2]), fmh<M>(f[3], e[3]))),
-                     fadd(fmh<M>(f[4], e[4]), fmh<M>(f[5], e[5]))), 2);
+    return fshl(fadd(fadd(fadd(fmh(f[0], e[0]), fmh(f[1], e[1])), fadd(fmh(f[2], e[2]), fmh(f[3], e[3]))),
+                     fadd(fmh(f[4], e[4]), fmh(f[5], e[5]))), 2);
 }
-template <class M = MulFull>
 __device__ __forceinline__ void phi_sym(const PhiFix* F, const long long* tr, int P, int i, int j, bool all, PhiPair& o)
 {
     long long c[3], s[3];
     SymTerms q;
-    pair_axes<M>(tr, P, i, j, c, s, all);
-    sym_terms<M>(c, q);
+    pair_axes(tr, P, i, j, c, s, all);
+    sym_terms(c, q);
     const long long* f = F->f;
-    o.f = fadd(f[0], sym_dot<M>(f + 1, q.e));
+    o.f = fadd(f[0], sym_dot(f + 1, q.e));
     if (!all) return;
-    o.l = sym_dot<M>(f + 7, q.e);
+    o.l = sym_dot(f + 7, q.e);
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const int b = (a + 1) % 3, e = (a + 2) % 3;
         const long long t = (c[b] >> 1) + (c[e] >> 1), w = (q.d[b] >> 1) + (q.d[e] >> 1);
         // the brackets are at most 1; their sum in quarters
-        const long long p1 = fadd(f[13] >> 2, fadd(fadd(fmh<M>(f[14], t), fmh<M>(f[15], q.u[a])),
-                                                   fadd(fmh<M>(f[16], w), fmh<M>(f[17], q.y[a]))));
-        const long long p2 = fadd(f[18], fshl(fadd(fmh<M>(f[19], t), fmh<M>(f[20], q.u[a])), 2));
-        o.g[a] = fmul<M>(s[a], fadd(p1, fmul<M>(c[a], p2)));
+        const long long p1 = fadd(f[13] >> 2, fadd(fadd(fmh(f[14], t), fmh(f[15], q.u[a])),
+                                                   fadd(fmh(f[16], w), fmh(f[17], q.y[a]))));
+        const long long p2 = fadd(f[18], fshl(fadd(fmh(f[19], t), fmh(f[20], q.u[a])), 2));
+        o.g[a] = fmul(s[a], fadd(p1, fmul(c[a], p2)));
     }
 }
 

@@ -2100,91 +2100,6 @@ __device__ void beta_drift_stage(const Ctx<R, NT, BIG>& c)
     unpaired_drift(c);
 }
 
-// Mixed path, stages 5 and 6 in one for shells in the symmetric form: the
-// entries' gradients and Laplacians, the pair function's from its polynomial
-// (dmc_pairfix.cuh, on the integer pipe) and beta's from the pair terms, times
-// the inverse; row sums go to the up particle, column sums (negated drift) to
-// the down particle.  Replaces two contractions of the inverse with the
-// orbitals (2 x 88k bounded multiply-adds of six instructions each at N = 66,
-// and the sums over k of their products): 62k -> 30k cycles a walker.
-template <class R, int NT, bool BIG>
-__device__ void pair_drift_mp(const Ctx<R, NT, BIG>& c)
-{
-    const DevParams& p = c.p;
-    double* sm = c.sm;
-    const double* x = sm + c.L.x;
-    const R* xr = at<R>(sm, c.L.xr);
-    const R* Si = at<R>(sm, c.L.S);
-    R* pv = c.template uat<R>(c.L.R);
-    const R* pb = reinterpret_cast<const R*>(c.pb);
-    const PhiFix* F = reinterpret_cast<const PhiFix*>(sm + c.L.kq);
-    long long* tr = c.template uat<long long>(c.L.trig);
-    double* acc = sm + c.L.acc;
-    const int nup = p.nup, ndn = p.ndn, ld = p.ldS, P = p.npart;
-    // axis cosines and sines of the particles (the orbitals are dead)
-    for (int t = threadIdx.x; t < 3 * P; t += NT) {
-        const int pt = t / 3, a = t - 3 * pt;
-        fix_sincos(box_fraction(x[t], p.el, p.eli), tr[(2 * a) * P + pt], tr[(2 * a + 1) * P + pt]);
-    }
-    for (int t = threadIdx.x; t < 4 * P; t += NT) acc[t] = 0.0;
-    const df sg = from_double(F->sgrad * 65536.0), sl = from_double(F->slap * 65536.0);
-    __syncthreads();
-    // a fixed-point value in units of 2^16: 24 and 23 bits of it, each exact
-    auto fix_df = [](long long v) {
-        return fast_two_sum((float)(int)(v >> 39) * 8388608.0f, (float)(int)((v >> 16) & 0x7fffff));
-    };
-    for (int r0 = 0; r0 < nup; r0 += c.L.rows_drift) {
-        const int r1 = min(nup, r0 + c.L.rows_drift);
-        const int npc = (r1 - r0) * ndn;
-        const UDiv dv(ndn);
-        for (int q = threadIdx.x; q < npc; q += NT) {
-            const int qi = dv.quo(q);
-            const int i = r0 + qi, j = q - qi * ndn;
-            PhiPair o;
-            phi_sym<MulShort>(F, tr, P, i, nup + j, true, o);
-            const R* xi = xr + 3 * i;
-            const R* xj = xr + 3 * (nup + j);
-            const R* pbq = pb + 2 * (i * ndn + j);
-            const R sij = Si[j * ld + i], fr = pbq[0];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                dfacc a;
-                acc_init(a);
-                acc_madd(a, fix_df(o.g[k]), sg);
-                acc_madd(a, fr, min_image(xi[k] - xj[k], p));
-                pv[4 * q + k] = sij * acc_value(a);
-            }
-            dfacc a;
-            acc_init(a);
-            acc_madd(a, fix_df(o.l), sl);
-            acc_add(a, pbq[1]);
-            pv[4 * q + 3] = sij * acc_value(a);
-        }
-        __syncthreads();
-        const int nr = r1 - r0;
-        for (int tc = threadIdx.x; tc < 4 * (nr + ndn); tc += NT) {
-            const int t = tc / 4, cmp = tc % 4;
-            dfacc sacc;
-            acc_init(sacc);
-            if (t < nr) {
-                const R* row = pv + 4 * (t * ndn) + cmp;
-                for (int j = 0; j < ndn; ++j) acc_add(sacc, row[4 * j]);
-                const int i = r0 + t;
-                acc[cmp < 3 ? 3 * i + cmp : 3 * P + i] += to_double(acc_value(sacc));
-            } else {
-                const int j = t - nr;
-                for (int r = 0; r < nr; ++r) acc_add(sacc, pv[4 * (r * ndn + j) + cmp]);
-                if (cmp < 3)
-                    acc[3 * (nup + j) + cmp] -= to_double(acc_value(sacc));
-                else
-                    acc[3 * P + nup + j] += to_double(acc_value(sacc));
-            }
-        }
-        __syncthreads();
-    }
-    unpaired_drift(c);
-}
-
 // ---------------------------------------------------------------------------
 // Long-range Jastrow (getjaslong, jastrowlongrange.f90:22-46), FP64 on both
 // paths.  The reference's pair sum is evaluated through the densities
@@ -2320,12 +2235,8 @@ __device__ HRes hpsi_eval(const Ctx<R, NT, BIG>& c, int mode)
         ok = inverse_stage<R>(c, logdet, sgn);
         if (ok && !(mode == MODE_BCS && c.a.inv_only)) {
             if constexpr (is_df<R>::value) {
-                if (reinterpret_cast<const PhiFix*>(sm + c.L.kq)->fast) {
-                    pair_drift_mp<R>(c);
-                } else {   // more shells: the contractions cost less than the octant form
-                    drift_stage<R>(c);
-                    beta_drift_stage<R>(c);
-                }
+                drift_stage<R>(c);
+                beta_drift_stage<R>(c);
             } else {
                 pair_drift64(c);
                 unpaired_drift(c);

@@ -207,10 +207,13 @@ walker_kernel(const __grid_constant__ DevParams p, const __grid_constant__ Kerne
 {
     extern __shared__ __align__(16) double sm[];
     const int P = p.npart, n3 = 3 * P;
-    // the pair function's fixed-point coefficients
-    for (int i = threadIdx.x; i < (int)(sizeof(PhiFix) / 8); i += NT)
-        sm[L.kq + i] = reinterpret_cast<const double*>(a.phi)[i];
-    if constexpr (walker::is_df<R>::value) {
+    if constexpr (!walker::is_df<R>::value) {
+        // FP64 path: the pair function's fixed-point coefficients
+        const double* src = reinterpret_cast<const double*>(a.phi);
+        for (int i = threadIdx.x; i < (int)(sizeof(PhiFix) / 8); i += NT) sm[L.kq + i] = src[i];
+    } else {
+        const double* kvsrc = reinterpret_cast<const double*>(walker::Prec<R>::kv(a));
+        for (int i = threadIdx.x; i < p.nk * 8; i += NT) sm[L.kq + i] = kvsrc[i];
         using KV = typename walker::Prec<R>::KV;
         const KV* kg = walker::Prec<R>::kv(a);
         R* ks = walker::at<R>(sm, L.ksoa);
