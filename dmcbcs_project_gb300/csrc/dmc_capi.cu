@@ -185,8 +185,8 @@ struct dmc_ctx {
     // single-particle moves and parameter derivatives
     DevBuf<double> sx, sdr, sratio, sder, ssinv, srsum, srene;
     DevBuf<double> pg_dpsi, pg_dphi, pg_dlog, pg_del, pg_scr;   // adjoint parameter gradients
-    DevBuf<PgTab> pg_btab;                                      // d beta / d b, d beta / d d tables
-    DevBuf<PgTab> pg_ktab;                                      // Jastrow knot basis on the table grid
+    DevBuf<PgPoly> pg_btab;                                     // d beta / d b, d beta / d d by grid interval
+    DevBuf<PgPoly> pg_ktab;                                     // Jastrow knot basis by grid interval
     DevBuf<double> pg_slice;                                    // per-CTA slices of the adjoint kernel
     // particle-by-particle sweeps: FP32 inverses carried between calls, the
     // cos/sin tables, accepted moves per walker
@@ -423,6 +423,18 @@ int upload_kv(dmc_ctx* c)
     return upload_phi(c);
 }
 
+// the cubic through four grid points T[0..3] in t = position - 1, from
+// differences (an interval's own points give no cancellation)
+void interval_cubic(const double* T, double* c)
+{
+    const double d1 = T[2] - T[1];
+    const double a3 = ((T[3] - T[0]) - 3.0 * d1) / 6.0, a2 = ((T[0] - T[1]) + d1) / 2.0;
+    c[0] = T[1];
+    c[1] = (d1 - a2) - a3;
+    c[2] = a2;
+    c[3] = a3;
+}
+
 int upload_tables(dmc_ctx* c)
 {
     const Setup& S = c->S;
@@ -437,21 +449,11 @@ int upload_tables(dmc_ctx* c)
     CK(c->tss.alloc(nt));
     CK(cudaMemcpy(c->tud.p, ud.data(), nt * sizeof(TabUD), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c->tss.p, ss.data(), nt * sizeof(TabSS), cudaMemcpyHostToDevice));
-    // FP64 walker path: the cubic through points i-1 .. i+2 in t = position - i,
-    // from differences (an interval's own points give no cancellation)
-    std::vector<TabPoly> tp(nt);
+    std::vector<TabPoly> tp(nt);   // FP64 walker path
     std::memset(tp.data(), 0, nt * sizeof(TabPoly));
     const std::vector<double>* src[7] = {&S.btab, &S.dbtab, &S.d2btab, &S.vtab[0], &S.utab[0], &S.dutab[0], &S.d2utab[0]};
     for (int i = 1; i + 2 < nt; ++i)
-        for (int k = 0; k < 7; ++k) {
-            const double* T = src[k]->data() + i - 1;
-            const double d1 = T[2] - T[1];
-            const double a3 = ((T[3] - T[0]) - 3.0 * d1) / 6.0, a2 = ((T[0] - T[1]) + d1) / 2.0;
-            tp[i].c[k][0] = T[1];
-            tp[i].c[k][1] = (d1 - a2) - a3;
-            tp[i].c[k][2] = a2;
-            tp[i].c[k][3] = a3;
-        }
+        for (int k = 0; k < 7; ++k) interval_cubic(src[k]->data() + i - 1, tp[i].c[k]);
     CK(c->tpoly.alloc(nt));
     CK(cudaMemcpy(c->tpoly.p, tp.data(), nt * sizeof(TabPoly), cudaMemcpyHostToDevice));
     // mixed-precision copies in double-float
@@ -1748,11 +1750,13 @@ static int pgrad_btab(dmc_ctx* c)
     std::vector<double> t[2][3];
     c->S.beta_param_tables(t);
     const size_t nt = (size_t)c->S.ntabb + 1;
-    std::vector<PgTab> h(2 * nt);
-    for (int w = 0; w < 2; ++w)
-        for (size_t i = 0; i < nt; ++i) h[w * nt + i] = PgTab{t[w][0][i], t[w][1][i], t[w][2][i], 0.0};
+    std::vector<PgPoly> h(2 * nt);
+    std::memset(h.data(), 0, h.size() * sizeof(PgPoly));
+    for (size_t i = 1; i + 2 < nt; ++i)
+        for (int w = 0; w < 2; ++w)
+            for (int m = 0; m < 3; ++m) interval_cubic(t[w][m].data() + i - 1, h[2 * i + w].c[m]);
     CK(c->pg_btab.alloc(2 * nt));
-    CK(cudaMemcpy(c->pg_btab.p, h.data(), 2 * nt * sizeof(PgTab), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(c->pg_btab.p, h.data(), 2 * nt * sizeof(PgPoly), cudaMemcpyHostToDevice));
     return DMC_OK;
 }
 
@@ -1763,10 +1767,14 @@ static int pgrad_ktab(dmc_ctx* c)
     if (c->S.jknots.empty() || c->pg_ktab.p) return DMC_OK;
     std::vector<double> t[3];
     c->S.knot_basis_tables(t);
-    std::vector<PgTab> h(t[0].size());
-    for (size_t i = 0; i < h.size(); ++i) h[i] = PgTab{t[0][i], t[1][i], t[2][i], 0.0};
+    const size_t nk = c->S.jknots.size(), nt = t[0].size() / nk;
+    std::vector<PgPoly> h(t[0].size());
+    std::memset(h.data(), 0, h.size() * sizeof(PgPoly));
+    for (size_t i = 1; i + 2 < nt; ++i)
+        for (size_t k = 0; k < nk; ++k)
+            for (int m = 0; m < 3; ++m) interval_cubic(t[m].data() + k * nt + i - 1, h[i * nk + k].c[m]);
     CK(c->pg_ktab.alloc(h.size()));
-    CK(cudaMemcpy(c->pg_ktab.p, h.data(), h.size() * sizeof(PgTab), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(c->pg_ktab.p, h.data(), h.size() * sizeof(PgPoly), cudaMemcpyHostToDevice));
     return DMC_OK;
 }
 
@@ -1801,17 +1809,17 @@ static int pgrad_device(dmc_ctx* c, int nw, const double* dx, double* dlog, doub
     int optin = 0;
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
     const size_t need = pgrad_doubles(c->P);
-    const int grid = pgrad_grid(c->P, nw, c->nsm, optin);
+    const int grid = pgrad_grid(c->P, nw, c->nsm, optin, c->phi_sym);
     if (grid < 1) return fail(c, DMC_ERR_CUDA, "adjoint kernel occupancy");
     double* scr = nullptr;
     if (need * 8 > (size_t)optin) {
         CK(c->pg_scr.alloc((size_t)grid * need));
         scr = c->pg_scr.p;
     }
-    CK(c->pg_slice.alloc((size_t)grid * pgrad_slice_doubles(c->P)));
-    CK(launch_pgrad(c->P, c->kv.p, c->tud.p, dx, c->ssinv.p, c->pg_dpsi.p, c->pg_dphi.p, dlog, del, nw, np,
-                    c->S.bfact, c->pg_btab.p, c->pg_ktab.p, pgrad_nbeta(c), pgrad_nknot(c), grid, scr,
-                    c->pg_slice.p, optin, c->stream));
+    CK(c->pg_slice.alloc((size_t)grid * pgrad_slice_doubles(c->P, c->phi_sym)));
+    CK(launch_pgrad(c->P, c->kv.p, c->tpoly.p, dx, c->ssinv.p, c->pg_dpsi.p, c->pg_dphi.p, dlog, del, nw, np,
+                    c->S.bfact, c->pg_btab.p, c->pg_ktab.p, pgrad_nbeta(c), pgrad_nknot(c), c->phi_sym,
+                    grid, scr, c->pg_slice.p, optin, c->stream));
     ++c->launches;
     return DMC_OK;
 }

@@ -86,22 +86,25 @@ size_t derbcs_smem_bytes(const DevParams& p);
 // most parameters of the adjoint gradients: vorb (DMC_MAX_SHELLS), bfact,
 // b, d and the 16 Jastrow knots
 constexpr int kPgradMax = DMC_MAX_SHELLS + 3 + 16;
-// {f, f', lap f} records of the b and d derivative tables of beta
-struct PgTab {
-    double f, df, d2f, pad;
+// {f, f', lap f} of a parameter's radial function on a grid interval, as cubics
+// in the position in it
+struct __align__(16) PgPoly {
+    double c[3][4];
 };
 // adjoint parameter gradients (dmc_single.cu): doubles of one CTA's core
 // (on chip when it fits in smem_limit bytes, else in gscr: grid x that) and
 // of its global slice (slices: grid x that, always); the grid that keeps
-// every SM's resident CTAs busy (0 on a CUDA error); ktd the Jastrow knot
-// basis on the table grid ([16][ntab+1], needed with nknot > 0)
+// every SM's resident CTAs busy (0 on a CUDA error).  By grid interval: btd
+// the b and d derivatives of beta ([ntab+1][2], with nbeta > 1), ktd the
+// Jastrow knot basis ([ntab+1][16], with nknot > 0).  sym: the shells are in
+// the symmetric form of PhiFix.
 size_t pgrad_doubles(const DevParams& p);
-size_t pgrad_slice_doubles(const DevParams& p);
-int pgrad_grid(const DevParams& p, int nw, int nsm, int smem_limit);
-cudaError_t launch_pgrad(const DevParams& p, const KVecDev* kv, const TabUD* tud, const double* x, const double* sinv,
-                         const double* dpsi, const double* dphi, double* dlog, double* deloc, int nw, int np,
-                         double bfact, const PgTab* btd, const PgTab* ktd, int nbeta, int nknot, int grid,
-                         double* gscr, double* slices, int smem_limit, cudaStream_t st);
+size_t pgrad_slice_doubles(const DevParams& p, bool sym);
+int pgrad_grid(const DevParams& p, int nw, int nsm, int smem_limit, bool sym);
+cudaError_t launch_pgrad(const DevParams& p, const KVecDev* kv, const TabPoly* tpoly, const double* x,
+                         const double* sinv, const double* dpsi, const double* dphi, double* dlog, double* deloc, int nw,
+                         int np, double bfact, const PgPoly* btd, const PgPoly* ktd, int nbeta, int nknot, bool sym,
+                         int grid, double* gscr, double* slices, int smem_limit, cudaStream_t st);
 // particle-by-particle sweeps with Sherman-Morrison updates (dmc_sweep.cu):
 // nsweep sweeps of the n walkers of stack st (positions and random states
 // updated in place); the inverse comes from inv64 (FP64, fresh) or, when

@@ -277,41 +277,30 @@ __global__ void __launch_bounds__(kThreads) derbcs_kernel(const __grid_constant_
     }
 }
 
-// beta(r) with its radial derivative and Laplacian (radialfun,
-// betafun.f90:173-194); zero beyond the range
-__device__ __forceinline__ void beta_all(const DevParams& p, const TabUD* tud, double r, double& f, double& df,
-                                         double& d2f)
-{
-    f = df = d2f = 0.0;
-    if (p.nobeta || r > p.rangeb) return;
-    const walker::Lagrange<double> W = walker::lagrange(r, p.scaleb, p.ntab);
-    const TabUD* T = tud + (W.idx - 1);
-    f = W.c1 * T[0].b + W.c2 * T[1].b + W.c3 * T[2].b + W.c4 * T[3].b;
-    df = W.c1 * T[0].db + W.c2 * T[1].db + W.c3 * T[2].db + W.c4 * T[3].db;
-    d2f = W.c1 * T[0].d2b + W.c2 * T[1].d2b + W.c3 * T[2].d2b + W.c4 * T[3].d2b;
-}
-
-// N sums over the CTA in a fixed order (warp trees, then the warps in
-// order); red holds at least kWarps * N doubles; sum k goes to outa[k] for
-// k < N/2 and to outb[k - N/2] otherwise
+// N sums over the CTA (N a multiple of 8) in a fixed order: transposed warp
+// sums, then the warps in order.  red holds at least kWarps * N doubles; the
+// first n of the sums k < N/2 go to outa[k], those of the rest to
+// outb[k - N/2].
 template <int N>
-__device__ void block_sum_n(double (&v)[N], double* red, double* outa, double* outb)
+__device__ void block_sum_n(double (&v)[N], double* red, double* outa, double* outb, int n)
 {
+    static_assert(N % 8 == 0 && N * kWarps <= kThreads, "sums of eight, in the reduction buffer");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int k = 0; k < N; ++k) {
-        double a = v[k];
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-        if (lane == 0) red[warp * N + k] = a;
+    for (int g = 0; g < N / 8; ++g) {
+        double u[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) u[k] = v[8 * g + k];
+        const double a = walker::warp_sum8(u);
+        if ((lane & 3) == 0) red[warp * N + 8 * g + (lane >> 2)] = a;
     }
     __syncthreads();
     if (threadIdx.x < N) {
+        const bool second = threadIdx.x >= N / 2;
+        const int k = second ? (int)threadIdx.x - N / 2 : (int)threadIdx.x;
         double t = 0.0;
         for (int q = 0; q < kWarps; ++q) t += red[q * N + threadIdx.x];
-        if (threadIdx.x < N / 2)
-            outa[threadIdx.x] = t;
-        else
-            outb[threadIdx.x - N / 2] = t;
+        if (k < n) (second ? outb : outa)[k] = t;
     }
     __syncthreads();
 }
@@ -354,9 +343,17 @@ __device__ double block_sum1(double v, double* red)
 //   S_ij  = ... + v_s C_s                      S'_s,ij = 2 C_s
 //   M_ij  = ... - v_s (k_s^2 C_s (1/m_i + 1/m_j) + 2 H_s . (w_i - w_j))
 //   M'_s,ij = -2 k_s^2 C_s (1/m_i + 1/m_j) - 4 H_s . (w_i - w_j)
-// The pass that forms M keeps (S'_s, M'_s) of every pair and shell, so the
-// shell parameters' sums after T cost three multiply-adds per pair and shell
-// instead of a second pass over the k vectors.
+// and M is the sum of vorb(s) M'_s and of beta's share.  SYM (shells in the
+// symmetric form, |n|^2 = s - 1 <= 6): with kappa = 2 pi / L, S'_s is a
+// polynomial U_s of the pair's axis cosines c_a, and
+//   M'_s,ij = -kappa^2 (s - 1) (1/m_i + 1/m_j) S'_s
+//             - 2 kappa sum_a sin_a dU_s/dc_a (w_i - w_j)_a,
+// 34 integer high products and 65 FP64 instructions a pair for six shells,
+// where the 40 k vectors took about 400.  The pass that forms M keeps
+// (S', M') of every pair and pair-function parameter, so that the sums after
+// T cost three multiply-adds a pair and parameter, and it takes the distance
+// and the grid interval once for beta, its derivatives and the knots, each a
+// cubic per interval.
 //
 // The 16 knots t_k of the opt-in up-down Jastrow spline are Jastrow
 // parameters: J = ... + sum_pairs sum_k t_k phi_k(r), so
@@ -364,29 +361,38 @@ __device__ double block_sum1(double v, double* red)
 //   d E_L / d t_k     = -hbar sum_pairs [ (1/m_i + 1/m_j)(phi_k'' + 2 phi_k'/r)
 //                        + 2 phi_k'/r d.(g_i - g_j) ],  g_p = grad_p log Psi / m_p,
 // with phi_k, phi_k', phi_k'' interpolated from their values on the Jastrow
-// table's grid (ktd[k][g]: the values the table itself was built from) with
-// the pair's Lagrange weights, exactly as the pair loop interpolates the
-// Jastrow table they are added to.
+// table's grid (the values the table itself was built from) with the pair's
+// 4-point interpolation, as the pair loop interpolates the Jastrow table they
+// are added to.
 // Inputs per walker: x, the inverse (column-major as smati), the total and
 // determinant drifts (grad / sqrt m) whose difference is grad J.  Outputs
 // dlog[w*np + t], deloc[w*np + t] for t = vorb(1..norb), then bfact, b, d
 // (nbeta = 3 with the beta function on), then the knots (nknot = 16 with the
 // spline on).
 // Memory: the CTA's core (inverse, M, product buffer, per-particle vectors,
-// reductions) in shared memory (in core_g when it does not fit); the axis
-// powers e^{i 2 pi m x_a / L}, the plane waves of every k at every particle
-// and the per-pair shell derivatives in the CTA's slice of slice_g (L2).
-__global__ void __launch_bounds__(kThreads) pgrad_kernel(const __grid_constant__ DevParams p,
-                                                         const KVecDev* __restrict__ kv,
-                                                         const TabUD* __restrict__ tud, const double* __restrict__ x,
-                                                         const double* __restrict__ sinv,
-                                                         const double* __restrict__ dpsi,
-                                                         const double* __restrict__ dphi, double* __restrict__ dlog,
-                                                         double* __restrict__ deloc, int nw, int np, double bfact,
-                                                         const PgTab* __restrict__ btd, const PgTab* __restrict__ ktd,
-                                                         int nbeta, int nknot, double* core_g, size_t core_per,
-                                                         double* slice_g, size_t slice_per)
+// reductions) in shared memory (in core_g when it does not fit); the per-pair
+// parameter derivatives and, without SYM, the axis powers e^{i 2 pi m x_a / L}
+// and the plane waves of every k at every particle in the CTA's slice of
+// slice_g (L2).
+// Bound: the FP64 pipe (89 % busy); 66 of its instructions a pair are the two
+// products, about 190 the pass that forms M.  2048 walkers at N = 66 with 26
+// parameters: 1.37 ms, the whole call 5.12 -> 2.33 ms (sums over k vectors,
+// Lagrange weights and a distance per parameter group before).
+template <bool SYM>
+__global__ void __launch_bounds__(kThreads, 2) pgrad_kernel(const __grid_constant__ DevParams p,
+                                                            const KVecDev* __restrict__ kv,
+                                                            const TabPoly* __restrict__ tpoly,
+                                                            const double* __restrict__ x,
+                                                            const double* __restrict__ sinv,
+                                                            const double* __restrict__ dpsi,
+                                                            const double* __restrict__ dphi, double* __restrict__ dlog,
+                                                            double* __restrict__ deloc, int nw, int np, double bfact,
+                                                            const PgPoly* __restrict__ btd,
+                                                            const PgPoly* __restrict__ ktd, int nbeta, int nknot,
+                                                            double* core_g, size_t core_per, double* slice_g,
+                                                            size_t slice_per)
 {
+    using namespace walker;
     extern __shared__ __align__(16) double smp[];
     double* base = core_g ? core_g + (size_t)blockIdx.x * core_per : smp;
     const int nd = p.nd, nup = p.nup, ndn = p.ndn, P = p.npart, nq = p.nk - 1, norb = p.norb;
@@ -399,18 +405,31 @@ __global__ void __launch_bounds__(kThreads) pgrad_kernel(const __grid_constant__
     double* gt = w + 3 * P;            // [P][3]: grad log Psi / m
     double* red = gt + 3 * P;
     double* res = red + kThreads;      // [2][kPgradMax]: d log Psi, then d Q
-    int* sh0 = reinterpret_cast<int*>(res + 2 * kPgradMax);   // first k of each shell s >= 2, then the end
+    double* va = res + 2 * kPgradMax;  // vorb of the shells s >= 2
+    int* sh0 = reinterpret_cast<int*>(va + norb);             // first k of each shell s >= 2, then the end
+    int* nf = sh0 + norb + 1;                                 // [P]: a coordinate that is not finite
+    long long* xf = reinterpret_cast<long long*>(va + norb + (norb + 2 + P) / 2);   // [P][3]: fractions of the box
+    long long* tr = xf + 3 * P;                               // [6][P]: cos, sin of the axis angles
     const int np1 = p.nmax + 1, nsh = norb - 1, npairs = nup * ndn;
-    double2* E = reinterpret_cast<double2*>(slice_g + (size_t)blockIdx.x * slice_per);   // [P][3][np1]
-    double2* cs = E + (size_t)3 * P * np1;                                             // [nq][P]
-    double2* dsm = cs + (size_t)P * (nq > 0 ? nq : 1);                                 // [nsh][npairs]
+    const int nsp = nsh + nbeta;       // parameters with an entry in dsm
+    double2* dsm = reinterpret_cast<double2*>(slice_g + (size_t)blockIdx.x * slice_per);   // [nsp][npairs]
+    double2* E = dsm + (size_t)nsp * npairs;                                               // [P][3][np1]
+    double2* cs = E + (size_t)3 * P * np1;                                                 // [nq][P]
     const int npb = norb + nbeta;      // parameters of the pair function
     const double imu = p.imass[0], imd = p.imass[1], ims = imu + imd;
+    // distances in units of L 2^-64 (L/2 = 2^63), as in the walker kernel
+    const double unit = p.el * 5.421010862427522e-20, iu = 1.0 / unit;
+    const double tscale = (double)p.ntab * 1.0842021724855044e-19, r_min = 1.0e-14 * iu;
+    const long long half = 0x43E0000000000000ll;
+    const double two62 = 4.611686018427387904e18, i62 = 1.0 / two62;
+    const double kap = 6.283185307179586 * p.eli;
+    const UDiv dv(ndn > 0 ? ndn : 1);
     if (threadIdx.x == 0) {
         // k vectors are sorted by shell; shell 1 is k = 0
         int q = 1;
         for (int sh = 2; sh <= norb; ++sh) {
             sh0[sh - 2] = q;
+            va[sh - 2] = q < p.nk && kv[q].shell == sh ? 0.5 * kv[q].v : 0.0;
             while (q < p.nk && kv[q].shell == sh) ++q;
         }
         sh0[norb - 1] = q;
@@ -419,57 +438,99 @@ __global__ void __launch_bounds__(kThreads) pgrad_kernel(const __grid_constant__
         for (size_t t = threadIdx.x; t < nd2; t += kThreads) Si[t] = sinv[(size_t)wk * nd2 + t];
         for (int t = threadIdx.x; t < 3 * P; t += kThreads) {
             const size_t g = (size_t)wk * 3 * P + t;
+            const int pt = t / 3, a = t - 3 * pt;
             const double xv = x[g];
             xs[t] = xv;
-            const int sp = (t / 3) < nup ? 0 : 1;
+            const int sp = pt < nup ? 0 : 1;
             w[t] = (dpsi[g] - dphi[g]) * p.isqm[sp];
             gt[t] = dpsi[g] * p.isqm[sp];
-            // powers of e^{i 2 pi x_a / L}, m = 0..nmax
-            double s1, c1;
-            sincospi(2.0 * xv * p.eli, &s1, &c1);
-            double2* e = E + (size_t)t * np1;
-            e[0] = make_double2(1.0, 0.0);
-            double cr = c1, ci = s1;
-            if (np1 > 1) e[1] = make_double2(c1, s1);
-            for (int m = 2; m < np1; ++m) {
-                const double nr = cr * c1 - ci * s1, ni = cr * s1 + ci * c1;
-                cr = nr;
-                ci = ni;
-                e[m] = make_double2(cr, ci);
+            xf[t] = box_fraction(xv, p.el, p.eli);
+            if (a == 0) nf[pt] = !(isfinite(xv) && isfinite(x[g + 1]) && isfinite(x[g + 2]));
+            if constexpr (SYM) {
+                fix_sincos(xf[t], tr[(2 * a) * P + pt], tr[(2 * a + 1) * P + pt]);
+            } else {
+                // powers of e^{i 2 pi x_a / L}, m = 0..nmax
+                double s1, c1;
+                sincospi(2.0 * xv * p.eli, &s1, &c1);
+                double2* e = E + (size_t)t * np1;
+                e[0] = make_double2(1.0, 0.0);
+                double cr = c1, ci = s1;
+                if (np1 > 1) e[1] = make_double2(c1, s1);
+                for (int m = 2; m < np1; ++m) {
+                    const double nr = cr * c1 - ci * s1, ni = cr * s1 + ci * c1;
+                    cr = nr;
+                    ci = ni;
+                    e[m] = make_double2(cr, ci);
+                }
             }
         }
         __syncthreads();
-        // e^{i k_q . x_p} as the product of the three axis powers
-        for (int t = threadIdx.x; t < nq * P; t += kThreads) {
-            const int q = t / P + 1, pp = t - (q - 1) * P;
-            const KVecDev& K = kv[q];
-            const double2* eb = E + (size_t)pp * 3 * np1;
-            const int n0 = K.n[0];
-            const double2 e0 = eb[n0 < 0 ? -n0 : n0];
-            double zr = e0.x, zi = n0 < 0 ? -e0.y : e0.y;
+        if constexpr (!SYM) {
+            // e^{i k_q . x_p} as the product of the three axis powers
+            for (int t = threadIdx.x; t < nq * P; t += kThreads) {
+                const int q = t / P + 1, pp = t - (q - 1) * P;
+                const KVecDev& K = kv[q];
+                const double2* eb = E + (size_t)pp * 3 * np1;
+                const int n0 = K.n[0];
+                const double2 e0 = eb[n0 < 0 ? -n0 : n0];
+                double zr = e0.x, zi = n0 < 0 ? -e0.y : e0.y;
 #pragma unroll
-            for (int a = 1; a < 3; ++a) {
-                const int n = K.n[a];
-                const double2 e = eb[a * np1 + (n < 0 ? -n : n)];
-                const double er = e.x, ei = n < 0 ? -e.y : e.y;
-                const double nr = zr * er - zi * ei, ni = zr * ei + zi * er;
-                zr = nr;
-                zi = ni;
+                for (int a = 1; a < 3; ++a) {
+                    const int n = K.n[a];
+                    const double2 e = eb[a * np1 + (n < 0 ? -n : n)];
+                    const double er = e.x, ei = n < 0 ? -e.y : e.y;
+                    const double nr = zr * er - zi * ei, ni = zr * ei + zi * er;
+                    zr = nr;
+                    zi = ni;
+                }
+                cs[t] = make_double2(zr, zi);
             }
-            cs[t] = make_double2(zr, zi);
+            __syncthreads();
         }
-        __syncthreads();
-        // M (psislaterbcs.f90:171-206, 249-293 for the entries and their
-        // derivatives), with every pair's shell derivatives on the side
-        for (size_t t = threadIdx.x; t < nd2; t += kThreads) {
-            const int i = (int)(t % nd), j = (int)(t / nd);
+        // the up-down block of M (psislaterbcs.f90:249-293 for the entries and
+        // their derivatives), every pair's parameter derivatives on the side,
+        // and the knots' sums, which need no more than the pair
+        double kacc[2 * kJastrowKnots];
+#pragma unroll
+        for (int k = 0; k < 2 * kJastrowKnots; ++k) kacc[k] = 0.0;
+        for (int t = threadIdx.x; t < npairs; t += kThreads) {
+            const int i = dv.quo(t), j = t - i * ndn, pj = nup + j;
+            const double wd[3] = {w[3 * i] - w[3 * pj], w[3 * i + 1] - w[3 * pj + 1], w[3 * i + 2] - w[3 * pj + 2]};
+            const bool nan = (nf[i] | nf[pj]) != 0;
+            const double not_num = __longlong_as_double(0x7ff8000000000000ll);
+            double2* dp = dsm + t;
             double m = 0.0;
-            if (i < nup && j < ndn) {
-                const int pj = nup + j;
-                const double wd0 = w[3 * i] - w[3 * pj], wd1 = w[3 * i + 1] - w[3 * pj + 1];
-                const double wd2 = w[3 * i + 2] - w[3 * pj + 2];
+            if constexpr (SYM) {
+                // S' in units of 2^-62 {8, 16, 8, 8, 32, 32}, M' likewise
+                long long c[3], s[3];
+                SymTerms q;
+                pair_axes(tr, P, i, pj, c, s, true);
+                sym_terms(c, q);
+                double g[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    const int b = (a + 1) % 3, e = (a + 2) % 3;
+                    const long long tm = (c[b] >> 1) + (c[e] >> 1), hw = (q.d[b] >> 3) + (q.d[e] >> 3);
+                    const double f = wd[a] * (double)s[a];
+                    g[0] += f;
+                    g[1] = fma(f, (double)tm, g[1]);
+                    g[2] = fma(f, (double)q.u[a], g[2]);
+                    g[3] = fma(f, (double)c[a], g[3]);
+                    g[4] = fma(f, (double)fadd(hw, fmul(c[a], tm)), g[4]);
+                    g[5] = fma(f, (double)fadd(q.y[a] >> 1, fmul(c[a], q.u[a])), g[5]);
+                }
+                constexpr double ratio[6] = {0.25, 0.5, 1.0, 1.0, 1.0, 1.0}, un[6] = {8.0, 16.0, 8.0, 8.0, 32.0, 32.0};
+#pragma unroll
+                for (int k = 0; k < 6; ++k)
+                    if (k < nsh) {
+                        const double ds = nan ? not_num : (double)q.e[k];
+                        const double dm = fma(g[k], -2.0 * ratio[k] * kap * (k == 0 ? 1.0 : i62),
+                                              ds * (-kap * kap * (k + 1) * ims));
+                        m = fma(va[k] * (un[k] * i62), dm, m);
+                        dp[(size_t)k * npairs] = make_double2(ds, dm);
+                    }
+            } else {
                 double l = 0.0, g0 = 0.0, g1 = 0.0, g2 = 0.0;
-                double2* dp = dsm + (size_t)i * ndn + j;
                 for (int s = 0; s < nsh; ++s) {
                     const int q0 = sh0[s], q1 = sh0[s + 1];
                     double cc = 0.0, h0 = 0.0, h1 = 0.0, h2 = 0.0;
@@ -487,7 +548,7 @@ __global__ void __launch_bounds__(kThreads) pgrad_kernel(const __grid_constant__
                     double ds = 0.0, dm = 0.0;
                     if (q1 > q0) {
                         const double v = kv[q0].v, k2c = kv[q0].k2 * cc;
-                        const double hw = h0 * wd0 + h1 * wd1 + h2 * wd2;
+                        const double hw = h0 * wd[0] + h1 * wd[1] + h2 * wd[2];
                         l -= v * k2c;
                         g0 -= v * h0;
                         g1 -= v * h1;
@@ -497,23 +558,87 @@ __global__ void __launch_bounds__(kThreads) pgrad_kernel(const __grid_constant__
                     }
                     dp[(size_t)s * npairs] = make_double2(ds, dm);
                 }
-                if (!p.nobeta) {
-                    double d[3];
-                    for (int cc = 0; cc < 3; ++cc) d[cc] = walker::min_image(xs[3 * i + cc] - xs[3 * pj + cc], p);
-                    const double r = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
-                    double f, df, d2f;
-                    beta_all(p, tud, r, f, df, d2f);
-                    if (r > 0.0) {
-                        const double dr = df / r;
-                        g0 += dr * d[0];
-                        g1 += dr * d[1];
-                        g2 += dr * d[2];
-                    }
-                    l += d2f;
+                m = l * ims + 2.0 * (g0 * wd[0] + g1 * wd[1] + g2 * wd[2]);
+            }
+            if (nbeta > 0 || nknot > 0) {
+                const long long e0 = fsub(xf[3 * i], xf[3 * pj]), e1 = fsub(xf[3 * i + 1], xf[3 * pj + 1]);
+                const long long e2 = fsub(xf[3 * i + 2], xf[3 * pj + 2]);
+                double d0 = (double)e0, d1 = (double)e1, d2 = (double)e2, r, ri;
+                if (nan) d0 = not_num;
+                if (((e0 | e1) | e2) != 0 || nan) {
+                    inv_dist(fma(d0, d0, fma(d1, d1, d2 * d2)), r, ri);
+                } else {   // closer than a unit, or coincident
+                    d0 = min_image(xs[3 * i] - xs[3 * pj], p) * iu;
+                    d1 = min_image(xs[3 * i + 1] - xs[3 * pj + 1], p) * iu;
+                    d2 = min_image(xs[3 * i + 2] - xs[3 * pj + 2], p) * iu;
+                    r = sqrt(norm2(d0, d1, d2));
+                    ri = r > 0.0 ? 1.0 / r : 0.0;
                 }
-                m = l * ims + 2.0 * (g0 * wd0 + g1 * wd1 + g2 * wd2);
-            } else if (i < nup) {
-                // unpaired up plane wave in column j (depends on up particle i)
+                double tt;
+                int o = grid_split(r * tscale, p.ntab, tt);
+                if (nbeta > 0) {
+                    // bfact (beta itself, over bfact at the end), b and d
+                    double f[3] = {0.0, 0.0, 0.0}, dm[3] = {0.0, 0.0, 0.0};
+                    if (__double_as_longlong(r) <= half || nan) {
+                        const double gw = 2.0 * (ri * fma(d0, wd[0], fma(d1, wd[1], d2 * wd[2])));
+                        const TabPoly* T = tpoly + o;
+                        f[0] = poly3(T->c[0], tt);
+                        dm[0] = fma(poly3(T->c[2], tt), ims, poly3(T->c[1], tt) * gw);
+#pragma unroll
+                        for (int q = 1; q < 3; ++q) {
+                            const PgPoly* G = btd + 2 * o + (q - 1);
+                            f[q] = poly3(G->c[0], tt);
+                            dm[q] = fma(poly3(G->c[2], tt), ims, poly3(G->c[1], tt) * gw);
+                        }
+                    }
+                    m += dm[0];
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) dp[(size_t)(nsh + q) * npairs] = make_double2(f[q], dm[q]);
+                }
+                if (nknot > 0) {
+                    if (!(r >= r_min)) {   // the reference's clamp, coshpot.f90:170
+                        r = r_min;
+                        ri = 1.0 / r_min;
+                        o = grid_split(r * tscale, p.ntab, tt);
+                    }
+                    if (__double_as_longlong(r) < half) {
+                        const double gd = fma(d0, gt[3 * i] - gt[3 * pj],
+                                              fma(d1, gt[3 * i + 1] - gt[3 * pj + 1], d2 * (gt[3 * i + 2] - gt[3 * pj + 2])));
+                        const double cp = 2.0 * ri * fma(ims, iu, gd);   // weight of phi' (phi'' has ims)
+                        // grid rows o - 1 .. o + 2 in units of the knot spacing
+                        // (t = r / h): the knots whose support (k - 2, k + 2)
+                        // (and the mirror image of k = 1 below one spacing)
+                        // reaches them, with a margin over FP32's rounding
+                        const float ts = 0.5f * (float)kJastrowCells / (float)p.ntab;
+                        const int klo = max(0, (int)((o - 1) * ts - 1.0e-4f) - 1);
+                        const int khi = min(kJastrowKnots - 1, (int)((o + 2) * ts + 1.0e-4f) + 2);
+                        const PgPoly* T = ktd + (size_t)o * kJastrowKnots;
+#pragma unroll 1
+                        for (int k = klo; k <= khi; ++k) {
+                            const double fp = poly3(T[k].c[1], tt), fpp = poly3(T[k].c[2], tt);
+                            kacc[k] += poly3(T[k].c[0], tt);
+                            kacc[kJastrowKnots + k] = fma(ims, fpp, fma(cp, fp, kacc[kJastrowKnots + k]));
+                        }
+                    }
+                }
+            }
+            M[i + (size_t)j * nd] = m;
+        }
+        // unpaired plane waves (psislaterbcs.f90:171-206): up ones in columns
+        // j >= ndn (each depends on up particle i), down ones in rows i >= nup
+        // (on down particle j), and the zero corner
+        const int nun = (nd - ndn) * nd, nrow = (nd - nup) * ndn;
+        for (int t = threadIdx.x; t < nun + nrow; t += kThreads) {
+            int i, j;
+            if (t < nun) {
+                i = t % nd;
+                j = ndn + t / nd;
+            } else {
+                i = nup + (t - nun) / ndn;
+                j = (t - nun) % ndn;
+            }
+            double m = 0.0;
+            if (i < nup) {
                 const int u = j - ndn;
                 const double* k = p.akup[u];
                 double sn, c;
@@ -522,7 +647,6 @@ __global__ void __launch_bounds__(kThreads) pgrad_kernel(const __grid_constant__
                 const double e = p.sinup[u] ? sn : c;
                 m = -p.ak2up[u] * e * imu + 2.0 * a * (k[0] * w[3 * i] + k[1] * w[3 * i + 1] + k[2] * w[3 * i + 2]);
             } else if (j < ndn) {
-                // unpaired down plane wave in row i (depends on down particle j)
                 const int u = i - nup, pj = nup + j;
                 const double* k = p.akdn[u];
                 double sn, c;
@@ -531,9 +655,10 @@ __global__ void __launch_bounds__(kThreads) pgrad_kernel(const __grid_constant__
                 const double e = p.sindn[u] ? sn : c;
                 m = -p.ak2dn[u] * e * imd + 2.0 * a * (k[0] * w[3 * pj] + k[1] * w[3 * pj + 1] + k[2] * w[3 * pj + 2]);
             }
-            M[t] = m;
+            M[i + (size_t)j * nd] = m;
         }
         __syncthreads();
+        if (nknot > 0) block_sum_n<2 * kJastrowKnots>(kacc, red, res + npb, res + kPgradMax + npb, nknot);
         // B = M S^-1, then T = S^-1 B (into M)
         for (size_t t = threadIdx.x; t < nd2; t += kThreads) {
             const int i = (int)(t % nd), j = (int)(t / nd);
@@ -549,113 +674,38 @@ __global__ void __launch_bounds__(kThreads) pgrad_kernel(const __grid_constant__
             M[t] = s;
         }
         __syncthreads();
-        // per pair-function shell parameter (eight at a time): sums over the
-        // up-down pairs of S^-1_ji S'_ij and S^-1_ji M'_ij - T_ji S'_ij
-        for (int th0 = 0; th0 < norb; th0 += 8) {
-            double acc[16];
+        // per pair-function parameter (twelve at a time): sums over the up-down
+        // pairs of S^-1_ji S'_ij and S^-1_ji M'_ij - T_ji S'_ij
+        for (int th0 = 0; th0 < npb; th0 += 12) {
+            double acc[24];
 #pragma unroll
-            for (int k = 0; k < 16; ++k) acc[k] = 0.0;
+            for (int k = 0; k < 24; ++k) acc[k] = 0.0;
             for (int t = threadIdx.x; t < npairs; t += kThreads) {
-                const int i = t / ndn, j = t - i * ndn;
+                const int i = dv.quo(t), j = t - i * ndn;
                 const double a = Si[j + (size_t)i * nd], tt = M[j + (size_t)i * nd];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
+                for (int u = 0; u < 12; ++u) {
                     const int th = th0 + u;
-                    if (th < norb) {
+                    if (th < npb) {
                         if (th == 0) {   // vorb(1): S' = 1, M' = 0
                             acc[u] += a;
-                            acc[8 + u] -= tt;
+                            acc[12 + u] -= tt;
                         } else {
                             const double2 v = dsm[(size_t)(th - 1) * npairs + t];
                             acc[u] = fma(a, v.x, acc[u]);
-                            acc[8 + u] += a * v.y - tt * v.x;
+                            acc[12 + u] = fma(-tt, v.x, fma(a, v.y, acc[12 + u]));
                         }
                     }
                 }
             }
-            block_sum_n<16>(acc, red, res + th0, res + kPgradMax + th0);
+            block_sum_n<24>(acc, red, res + th0, res + kPgradMax + th0, npb - th0);
         }
-        if (nbeta > 0) {
-            // bfact (beta / bfact), b and d (their derivative tables) in one
-            // pass: one distance and one set of Lagrange weights per pair
-            double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-            const double ib = 1.0 / bfact;
-            const PgTab* Tb = btd;
-            const PgTab* Td = btd + (size_t)(p.ntab + 1);
-            for (int t = threadIdx.x; t < npairs; t += kThreads) {
-                const int i = t / ndn, j = t % ndn, pj = nup + j;
-                double d[3];
-                for (int cc = 0; cc < 3; ++cc) d[cc] = walker::min_image(xs[3 * i + cc] - xs[3 * pj + cc], p);
-                const double r = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
-                if (p.nobeta || r > p.rangeb) continue;
-                const double a = Si[j + (size_t)i * nd], tt = M[j + (size_t)i * nd];
-                const walker::Lagrange<double> W = walker::lagrange(r, p.scaleb, p.ntab);
-                const double ri = r > 0.0 ? 1.0 / r : 0.0;
-                const double gw = d[0] * (w[3 * i] - w[3 * pj]) + d[1] * (w[3 * i + 1] - w[3 * pj + 1]) +
-                                  d[2] * (w[3 * i + 2] - w[3 * pj + 2]);
-                const int o = W.idx - 1;
-                double f[3], df[3], d2f[3];
-                {
-                    const TabUD* T = tud + o;
-                    f[0] = (W.c1 * T[0].b + W.c2 * T[1].b + W.c3 * T[2].b + W.c4 * T[3].b) * ib;
-                    df[0] = (W.c1 * T[0].db + W.c2 * T[1].db + W.c3 * T[2].db + W.c4 * T[3].db) * ib;
-                    d2f[0] = (W.c1 * T[0].d2b + W.c2 * T[1].d2b + W.c3 * T[2].d2b + W.c4 * T[3].d2b) * ib;
-                }
-                for (int q = 1; q < 3; ++q) {
-                    const PgTab* T = (q == 1 ? Tb : Td) + o;
-                    f[q] = W.c1 * T[0].f + W.c2 * T[1].f + W.c3 * T[2].f + W.c4 * T[3].f;
-                    df[q] = W.c1 * T[0].df + W.c2 * T[1].df + W.c3 * T[2].df + W.c4 * T[3].df;
-                    d2f[q] = W.c1 * T[0].d2f + W.c2 * T[1].d2f + W.c3 * T[2].d2f + W.c4 * T[3].d2f;
-                }
-                for (int q = 0; q < 3; ++q) {
-                    const double dm = d2f[q] * ims + 2.0 * df[q] * ri * gw;
-                    acc[q] += a * f[q];
-                    acc[3 + q] += a * dm - tt * f[q];
-                }
-            }
-            block_sum_n<6>(acc, red, res + norb, res + kPgradMax + norb);
-        }
-        if (nknot > 0) {
-            // the Jastrow knots, all in one pass over the up-down pairs
-            double acc[2 * kJastrowKnots];
-#pragma unroll
-            for (int k = 0; k < 2 * kJastrowKnots; ++k) acc[k] = 0.0;
-            // grid rows in units of the knot spacing (t = r / h): the knots
-            // whose support [k - 2, k + 2] (and the mirror image of k = 1
-            // below one spacing) reaches the pair's four grid rows
-            const double tstep = kJastrowCells / (p.el * p.scale);
-            const size_t kstride = (size_t)p.ntab + 1;
-            for (int t = threadIdx.x; t < npairs; t += kThreads) {
-                const int i = t / ndn, j = t % ndn, pj = nup + j;
-                double d[3];
-                for (int cc = 0; cc < 3; ++cc) d[cc] = walker::min_image(xs[3 * i + cc] - xs[3 * pj + cc], p);
-                const double r = fmax(sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]), 1.0e-14);
-                if (!(r < p.range)) continue;
-                const walker::Lagrange<double> W = walker::lagrange(r, p.scale, p.ntab);
-                const double ri = 1.0 / r;
-                const double gd = d[0] * (gt[3 * i] - gt[3 * pj]) + d[1] * (gt[3 * i + 1] - gt[3 * pj + 1]) +
-                                  d[2] * (gt[3 * i + 2] - gt[3 * pj + 2]);
-                const double cp = 2.0 * ri * (ims + gd);   // weight of phi' (phi'' has ims)
-                const int o = W.idx - 1;
-                const double t0 = o * tstep;
-                const int klo = max(0, (int)t0 - 2);
-                const int khi = min(kJastrowKnots - 1, (int)(t0 + 3.0 * tstep) + 2);
-#pragma unroll 1
-                for (int k = klo; k <= khi; ++k) {
-                    const PgTab* T = ktd + k * kstride + o;
-                    const double f = W.c1 * T[0].f + W.c2 * T[1].f + W.c3 * T[2].f + W.c4 * T[3].f;
-                    const double fp = W.c1 * T[0].df + W.c2 * T[1].df + W.c3 * T[2].df + W.c4 * T[3].df;
-                    const double fpp = W.c1 * T[0].d2f + W.c2 * T[1].d2f + W.c3 * T[2].d2f + W.c4 * T[3].d2f;
-                    acc[k] += f;
-                    acc[kJastrowKnots + k] += ims * fpp + cp * fp;
-                }
-            }
-            block_sum_n<2 * kJastrowKnots>(acc, red, res + npb, res + kPgradMax + npb);
-        }
-        __syncthreads();
         for (int th = threadIdx.x; th < np; th += kThreads) {
-            dlog[(size_t)wk * np + th] = res[th];
-            deloc[(size_t)wk * np + th] = -p.hbar * res[kPgradMax + th];
+            double f = 1.0;   // of the shells' units, and of beta / bfact
+            if (SYM && th > 0 && th < norb) f = (th == 2 ? 16.0 : th >= 5 ? 32.0 : 8.0) * i62;
+            if (nbeta > 0 && th == norb) f = 1.0 / bfact;
+            dlog[(size_t)wk * np + th] = res[th] * f;
+            deloc[(size_t)wk * np + th] = -p.hbar * (res[kPgradMax + th] * f);
         }
         __syncthreads();
     }
@@ -818,59 +868,62 @@ cudaError_t launch_derbcs(const DevParams& p, const KVecDev* kv, const double* x
 
 // Layout of one pgrad CTA's core, in doubles: inverse, M, product buffer
 // (nd^2 each), positions, grad J / m and grad log Psi / m (3 npart each),
-// reduction buffer, results, first k of each shell.
+// reduction buffer, results, amplitudes and first k of each shell, flags,
+// box fractions and axis cos/sin.
 size_t pgrad_doubles(const DevParams& p)
 {
     const size_t nd2 = (size_t)p.nd * p.nd;
-    return 3 * nd2 + 9 * (size_t)p.npart + kThreads + 2 * (size_t)kPgradMax + (size_t)(p.norb + 2);
+    return 3 * nd2 + 18 * (size_t)p.npart + kThreads + 2 * (size_t)kPgradMax + (size_t)p.norb +
+           (size_t)(p.norb + 2 + p.npart) / 2;
 }
 
-// The CTA's global slice, in doubles (even): axis powers (3 npart (nmax+1)
-// complex), plane waves (npart (nk-1) complex), shell derivatives
-// ((norb-1) nup ndn pairs of doubles).
-size_t pgrad_slice_doubles(const DevParams& p)
+// The CTA's global slice, in doubles (even): (S', M') of every up-down pair
+// for the shells and beta's three parameters; without the symmetric form also
+// axis powers (3 npart (nmax+1) complex) and plane waves (npart (nk-1) complex).
+size_t pgrad_slice_doubles(const DevParams& p, bool sym)
 {
-    const size_t nq = p.nk > 1 ? (size_t)p.nk - 1 : 1, nsh = p.norb > 1 ? (size_t)p.norb - 1 : 1;
-    return 2 * (3 * (size_t)p.npart * (p.nmax + 1) + (size_t)p.npart * nq + nsh * p.nup * p.ndn);
+    const size_t nq = p.nk > 1 ? (size_t)p.nk - 1 : 1, nsp = (size_t)p.norb - 1 + (p.nobeta ? 0 : 3);
+    const size_t waves = sym ? 0 : 3 * (size_t)p.npart * (p.nmax + 1) + (size_t)p.npart * nq;
+    return 2 * (nsp * p.nup * p.ndn + waves + 1);
 }
 
 // CTAs of one pgrad launch: as many as are resident on the device's SMs
 // together, at most one per walker.
-int pgrad_grid(const DevParams& p, int nw, int nsm, int smem_limit)
+int pgrad_grid(const DevParams& p, int nw, int nsm, int smem_limit, bool sym)
 {
+    const auto kern = sym ? pgrad_kernel<true> : pgrad_kernel<false>;
     const size_t need = pgrad_doubles(p) * 8;
     const int smem = need <= (size_t)smem_limit ? (int)need : 0;
     int per_sm = 1;
-    if (smem > 0 && cudaFuncSetAttribute(pgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    if (smem > 0 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
         return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pgrad_kernel, kThreads, smem) != cudaSuccess)
-        return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem) != cudaSuccess) return 0;
     const long long g = (long long)(per_sm > 0 ? per_sm : 1) * nsm;
     return (int)(g < nw ? g : (nw > 0 ? nw : 1));
 }
 
-cudaError_t launch_pgrad(const DevParams& p, const KVecDev* kv, const TabUD* tud, const double* x, const double* sinv,
-                         const double* dpsi, const double* dphi, double* dlog, double* deloc, int nw, int np,
-                         double bfact, const PgTab* btd, const PgTab* ktd, int nbeta, int nknot, int grid,
-                         double* gscr, double* slices, int smem_limit, cudaStream_t st)
+cudaError_t launch_pgrad(const DevParams& p, const KVecDev* kv, const TabPoly* tpoly, const double* x,
+                         const double* sinv, const double* dpsi, const double* dphi, double* dlog, double* deloc, int nw,
+                         int np, double bfact, const PgPoly* btd, const PgPoly* ktd, int nbeta, int nknot, bool sym,
+                         int grid, double* gscr, double* slices, int smem_limit, cudaStream_t st)
 {
     if (np > kPgradMax || nknot > kJastrowKnots || np != p.norb + nbeta + nknot || (nbeta > 1 && !btd) ||
         (nknot > 0 && !ktd) || !slices || grid < 1)
         return cudaErrorInvalidValue;
     if (nw <= 0) return cudaSuccess;
+    const auto kern = sym ? pgrad_kernel<true> : pgrad_kernel<false>;
     const size_t need = pgrad_doubles(p);
     const bool on_chip = need * 8 <= (size_t)smem_limit;
     const size_t smem = on_chip ? need * 8 : 0;
     if (on_chip) {
-        cudaError_t e = cudaFuncSetAttribute(pgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     } else if (!gscr) {
         return cudaErrorInvalidValue;
     }
-    pgrad_kernel<<<grid < nw ? grid : nw, kThreads, smem, st>>>(p, kv, tud, x, sinv, dpsi, dphi, dlog, deloc, nw, np,
-                                                                bfact, btd, ktd, nbeta, nknot,
-                                                                on_chip ? nullptr : gscr, need, slices,
-                                                                pgrad_slice_doubles(p));
+    kern<<<grid < nw ? grid : nw, kThreads, smem, st>>>(p, kv, tpoly, x, sinv, dpsi, dphi, dlog, deloc, nw, np, bfact,
+                                                        btd, ktd, nbeta, nknot, on_chip ? nullptr : gscr, need, slices,
+                                                        pgrad_slice_doubles(p, sym));
     return cudaGetLastError();
 }
 
