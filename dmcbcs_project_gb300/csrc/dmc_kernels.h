@@ -111,7 +111,6 @@ cudaError_t launch_pgrad(const DevParams& p, const KVecDev* kv, const TabPoly* t
 // inv64 is null, from inv32, and leaves in inv32; tab is cos/sin scratch
 // [n][nk-1][npart]; accepted[w] counts the walker's accepted moves; prop
 // is scratch for each sweep's proposals, [n][npart][4] doubles
-size_t sweep_smem_bytes(const DevParams& p, int walkers_per_cta);
 // jA/jC: ran1 jump-ahead tables for 0 .. 5 npart steps
 cudaError_t launch_sweeps(const DevParams& p, const DevStack& st, int n, int nsweep, const double* inv64,
                           float* inv32, float2* tab, const KVecMP* kv, const TabUDmp* tud, const TabSSmp* tss,

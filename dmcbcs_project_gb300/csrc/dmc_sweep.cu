@@ -6,13 +6,13 @@
 // bcsone / getphione / move1 (psislaterbcs.f90:296-376, coshpot.f90:207-264,
 // wavefunction.f90:393-404), which the reference uses only for n(k).
 //
-// One warp per walker.  Per move of particle i (in order 0..npart-1, every
-// sweep):
+// One CTA of four warps per walker.  Per move of particle i (in order
+// 0..npart-1, every sweep):
 //   - five draws of the walker's ran1 stream (ran.f90:8-27): three Gaussian
 //     deviates (gaussian(3), ran.f90:74-104) and one uniform, and the
 //     proposal x_i' = x_i + sigma_i g (sigma of setstep, step.f90:29-30)
 //     wrapped into the box, all in FP64 for the whole sweep ahead of its
-//     moves, one move per lane (particle i has not moved before its own move
+//     moves, one move per thread (particle i has not moved before its own move
 //     of the sweep);
 //   - distances in FP32;
 //   - the new row (up particle) or column (down particle) s' of the pair
@@ -37,19 +37,30 @@
 namespace dmc {
 namespace {
 
-constexpr int kSweepWarps = 4;   // most walkers per CTA, one warp each
+// Threads per walker.  Bound: the latency of a move's chain of stages, one move
+// after another.  A warp per walker took 24k cycles a move at N = 66: every
+// loop over 33 entries or 40 k vectors had a second, nearly empty round and the
+// table's loads were exposed.  Here an entry has two threads (the chains over
+// the even and over the odd k vectors, two of its four partial sums), the last
+// warp takes the Jastrow beside them and the rank-one update all of them; every
+// sum keeps its order and rounding.  One sweep of 1024 walkers at N = 66:
+// 822 -> 274 us.
 
-// floats of one warp's shared memory: FP32 positions for the distances (3
+// floats of a walker's shared memory: FP32 positions for the distances (3
 // npart), X (nd x ldx), the new entries s' and the v / w vector (nd each),
-// the moved particle's orbitals (v-scaled and plain, 2 (nk-1) float2).  The
-// FP64 positions stay in the walker stack and the sweep's proposals in a
-// global slice per walker, so that a warp's share is small enough for all
-// walkers of a 4096-walker population at N = 66 to be resident at once.
-__host__ __device__ inline int sweep_warp_floats(const DevParams& p)
+// the moved particle's orbitals (v-scaled and plain, 2 (nk-1) float2), the
+// Jastrow difference (two slots).  The FP64 positions stay in the walker stack
+// and the sweep's proposals in a global slice per walker.
+__host__ __device__ inline int sweep_floats(const DevParams& p)
 {
     const int ldx = p.nd | 1;
     const int nq = p.nk > 1 ? p.nk - 1 : 1;
     return 3 * p.npart + 2 + p.nd * ldx + 2 * p.nd + 8 * nq + 8;
+}
+// the same in whole float2, with the cos/sin table where it is on chip
+__host__ __device__ inline int walker_floats(const DevParams& p, bool onchip)
+{
+    return (sweep_floats(p) + 1) / 2 * 2 + (onchip ? 2 * (p.nk > 1 ? p.nk - 1 : 1) * p.npart : 0);
 }
 
 // FP32 4-point Lagrange grid position (index clamp of coshpot.f90:174)
@@ -99,52 +110,61 @@ __device__ __forceinline__ double ran1_step(unsigned long long& s)
 // FP32 minimum image
 __device__ __forceinline__ float min_image_f(float d, float el, float eli) { return d - el * rintf(d * eli); }
 
-__global__ void __launch_bounds__(32 * kSweepWarps) sweep_kernel(const __grid_constant__ DevParams p, DevStack st,
-                                                                 int n, int nsweep, const double* __restrict__ inv64,
-                                                                 float* __restrict__ inv32, float2* __restrict__ tab,
-                                                                 const KVecMP* __restrict__ kv,
-                                                                 const TabUDmp* __restrict__ tud,
-                                                                 const TabSSmp* __restrict__ tss,
-                                                                 const unsigned long long* __restrict__ jA,
-                                                                 const unsigned long long* __restrict__ jC,
-                                                                 unsigned long long* __restrict__ accepted, int wpc,
-                                                                 double* __restrict__ prop)
+// barrier of the threads that form the new entries
+template <int W>
+__device__ __forceinline__ void row_sync()
 {
-    extern __shared__ __align__(16) double smw[];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    if constexpr (W == 2)
+        __syncwarp();
+    else
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * (W - 1)) : "memory");
+}
+
+// A CTA of W warps per walker.  ONCHIP: the cos/sin table in shared memory,
+// otherwise in tab.  (Registers for 128 threads: with those for 64, two warps
+// took 5 % longer.)
+template <int W, bool ONCHIP>
+__global__ void __launch_bounds__(128) sweep_kernel(const __grid_constant__ DevParams p, DevStack st,
+                                                              int nsweep, const double* __restrict__ inv64,
+                                                              float* __restrict__ inv32, float2* __restrict__ tab,
+                                                              const KVecMP* __restrict__ kv,
+                                                              const TabUDmp* __restrict__ tud,
+                                                              const TabSSmp* __restrict__ tss,
+                                                              const unsigned long long* __restrict__ jA,
+                                                              const unsigned long long* __restrict__ jC,
+                                                              unsigned long long* __restrict__ accepted,
+                                                              double* __restrict__ prop)
+{
+    extern __shared__ __align__(16) float smw[];
+    constexpr int NT = 32 * W, NR = NT - 32;   // all threads; those for the new entries
+    const int tid = threadIdx.x, lane = tid & 31;
     const int P = p.npart, nd = p.nd, ldx = nd | 1, nq = p.nk - 1, nup = p.nup;
-    float* xsf = reinterpret_cast<float*>(smw + (size_t)wib * (sweep_warp_floats(p) / 2 + 1));
+    float* xsf = smw;
     float* X = xsf + 3 * P + (P & 1);                  // X(r, c) = X[r + c ldx]: column-major as smati
     float* snew = X + nd * ldx;
     float* vw = snew + nd;
     float2* onew = reinterpret_cast<float2*>(vw + nd + (((nd * ldx + 2 * nd) & 1) ? 1 : 0));   // v-scaled
     float2* oraw = onew + (nq > 0 ? nq : 1);                                                 // plain
+    float* s_du = reinterpret_cast<float*>(oraw + (nq > 0 ? nq : 1));                        // by the move's parity
     const float v0 = kv[0].v.hi;
     const float elf = (float)p.el, elif = (float)p.eli;
-    const int w = blockIdx.x * wpc + wib;
-    if (w >= n) return;   // whole warps only: the warp is the unit below
+    const int w = blockIdx.x;
     double* xs = st.x + (size_t)w * 3 * P;     // FP64 positions, wrapped in place
     double* drw = prop + (size_t)w * 4 * P;    // [P][4]: the proposal x_i + sigma g and u of move i
     // ---- load the walker: positions (wrapped), inverse, cos/sin table ----
-    for (int e = lane; e < 3 * P; e += 32) {
+    for (int e = tid; e < 3 * P; e += NT) {
         const double xv = walker::min_image(xs[e], p);
         xs[e] = xv;
         xsf[e] = (float)xv;
     }
-    if (inv64) {
-        for (int e = lane; e < nd * nd; e += 32) {
-            const int r = e % nd, c = e / nd;
-            X[r + c * ldx] = (float)inv64[(size_t)w * nd * nd + e];
-        }
-    } else {
-        for (int e = lane; e < nd * nd; e += 32) {
-            const int r = e % nd, c = e / nd;
-            X[r + c * ldx] = inv32[(size_t)w * nd * nd + e];
-        }
+    for (int e = tid; e < nd * nd; e += NT) {
+        const int r = e % nd, c = e / nd;
+        X[r + c * ldx] = inv64 ? (float)inv64[(size_t)w * nd * nd + e] : inv32[(size_t)w * nd * nd + e];
     }
-    float2* T = tab + (size_t)w * nq * P;   // T[q P + j] = (cos, sin)(k_{q+1} . x_j)
-    __syncwarp();
-    for (int e = lane; e < nq * P; e += 32) {
+    // T[q P + j] = (cos, sin)(k_{q+1} . x_j)
+    float2* T = ONCHIP ? reinterpret_cast<float2*>(xsf + walker_floats(p, false)) : tab + (size_t)w * nq * P;
+    __syncthreads();
+    for (int e = tid; e < nq * P; e += NT) {
         const int q = e / P, j = e % P;
         const KVecMP& K = kv[q + 1];
         float sn, cs;
@@ -154,16 +174,15 @@ __global__ void __launch_bounds__(32 * kSweepWarps) sweep_kernel(const __grid_co
     }
     unsigned long long s = st.irn[w] & walker::kMask48;
     unsigned long long nacc = 0;
-    __syncwarp();
+    const walker::UDiv dv(nd);
     for (int sw = 0; sw < nsweep; ++sw) {
-        // the sweep's draws, one move per lane: move i takes ran1 draws
+        // the sweep's draws, one move per thread: move i takes ran1 draws
         // 5i+1 .. 5i+5 of the stream -- gaussian(3) from four uniforms, then
-        // the acceptance uniform -- reached by jump-ahead (one FP64
-        // Box-Muller per lane instead of one per move on a single lane).
-        // Particle i moves only at its own move, so its proposal
-        // x_i + sigma g is fixed by the sweep's start and is made here too:
-        // the moves themselves do no FP64 arithmetic
-        for (int i = lane; i < P; i += 32) {
+        // the acceptance uniform -- reached by jump-ahead.  Particle i moves
+        // only at its own move, so its proposal x_i + sigma g is fixed by the
+        // sweep's start and is made here too: the moves themselves do no FP64
+        // arithmetic
+        for (int i = tid; i < P; i += NT) {
             unsigned long long t = (jA[5 * i] * s + jC[5 * i]) & walker::kMask48;
             const double u1 = ran1_step(t), u2 = ran1_step(t), u3 = ran1_step(t), u4 = ran1_step(t);
             const double rn = ran1_step(t);
@@ -176,8 +195,8 @@ __global__ void __launch_bounds__(32 * kSweepWarps) sweep_kernel(const __grid_co
             drw[4 * i + 3] = rn;
         }
         s = (jA[5 * P] * s + jC[5 * P]) & walker::kMask48;
-        __syncwarp();
-        // lanes 0-3 hold move i's proposal and uniform, read one move ahead
+        __syncthreads();
+        // lanes 0-3 of each warp hold move i's proposal and uniform, read one move ahead
         double pv = lane < 4 ? drw[lane] : 0.0;
         for (int i = 0; i < P; ++i) {
             const bool up = i < nup;
@@ -187,147 +206,144 @@ __global__ void __launch_bounds__(32 * kSweepWarps) sweep_kernel(const __grid_co
             const double pcur = pv;
             if (lane < 4 && i + 1 < P) pv = drw[4 * (i + 1) + lane];
             const float xf[3] = {(float)xn[0], (float)xn[1], (float)xn[2]};
-            // the moved particle's plane waves
-            for (int q = lane; q < nq; q += 32) {
-                const KVecMP& K = kv[q + 1];
-                float sn, cs;
-                sincosf(K.k[0].hi * xf[0] + K.k[1].hi * xf[1] + K.k[2].hi * xf[2], &sn, &cs);
-                oraw[q] = make_float2(cs, sn);
-                const float vq = K.v.hi;
-                onew[q] = make_float2(vq * cs, vq * sn);
-            }
-            __syncwarp();
-            // the new row (up) or column (down) of the pair matrix
-            const int nloop = up ? p.npair + p.nexdn : p.npair + p.nexup;
-            for (int e = lane; e < nd; e += 32) {
-                float ph;
-                if (e < nloop) {
-                    const int jj = up ? e + p.npair + p.nexup : e;
-                    // two chains, loads unrolled ahead of the multiply-adds
-                    float acc = v0, acc2 = 0.0f;
-                    int q = 0;
-#pragma unroll 4
-                    for (; q + 1 < nq; q += 2) {
-                        const float2 a = onew[q], b = T[q * P + jj];
-                        const float2 a2 = onew[q + 1], b2 = T[(q + 1) * P + jj];
-                        acc = fmaf(a.x, b.x, fmaf(a.y, b.y, acc));
-                        acc2 = fmaf(a2.x, b2.x, fmaf(a2.y, b2.y, acc2));
-                    }
-                    if (q < nq) {
-                        const float2 a = onew[q], b = T[q * P + jj];
-                        acc = fmaf(a.x, b.x, fmaf(a.y, b.y, acc));
-                    }
-                    acc += acc2;
-                    float d2 = 0.0f;
-                    for (int c = 0; c < 3; ++c) {
-                        const float d = min_image_f(xf[c] - xsf[3 * jj + c], elf, elif);
-                        d2 = fmaf(d, d, d2);
-                    }
-                    ph = acc + beta_f(p, tud, sqrtf(d2));
-                } else {
-                    const int u = e - nloop;
-                    const double* a = up ? p.akup[u] : p.akdn[u];
-                    const int sn = up ? p.sinup[u] : p.sindn[u];
-                    const float arg = (float)a[0] * xf[0] + (float)a[1] * xf[1] + (float)a[2] * xf[2];
-                    ph = sn ? sinf(arg) : cosf(arg);
+            if (tid < NR) {
+                // the moved particle's plane waves
+                for (int q = tid; q < nq; q += NR) {
+                    const KVecMP& K = kv[q + 1];
+                    float sn, cs;
+                    sincosf(K.k[0].hi * xf[0] + K.k[1].hi * xf[1] + K.k[2].hi * xf[2], &sn, &cs);
+                    oraw[q] = make_float2(cs, sn);
+                    const float vq = K.v.hi;
+                    onew[q] = make_float2(vq * cs, vq * sn);
                 }
-                snew[e] = ph;
-            }
-            __syncwarp();
-            // v_k = sum_q s'_q X(q, k) (row i replaced) or w_k = sum_q X(k, q) s'_q
-            // (column c replaced); the ratio is v_i or w_c
-            const int cix = up ? i : i - nup;
-            for (int k = lane; k < nd; k += 32) {
-                // four partial sums: the chain is shared-memory latency bound
-                float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                const int rs = up ? 1 : ldx, cs = up ? ldx : 1;   // X(q, k) or X(k, q)
-                const float* xb = X + k * cs;
-                int q = 0;
-                for (; q + 3 < nd; q += 4) {
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) a[u] = fmaf(snew[q + u], xb[(q + u) * rs], a[u]);
-                }
-                for (; q < nd; ++q) a[0] = fmaf(snew[q], xb[q * rs], a[0]);
-                vw[k] = (a[0] + a[1]) + (a[2] + a[3]);
-            }
-            // Jastrow: U(r_i') - U(r_i) over the pairs getphione counts.  A
-            // lane takes its partners j = lane + 32 u kJasLanes at a time, all
-            // their table lookups in flight before any is used; the
-            // differences are added in partner order (skipped pairs add 0).
-            constexpr int kJasLanes = 3;
-            float du = 0.0f;
-            for (int j0 = lane; j0 < P; j0 += 32 * kJasLanes) {
-                float dj[kJasLanes];
-#pragma unroll
-                for (int u = 0; u < kJasLanes; ++u) {
-                    const int j = j0 + 32 * u;
-                    dj[u] = 0.0f;
-                    const bool opp = up != (j < nup);
-                    if (j < P && j != i && (opp || p.ieq)) {
-                        float dn = 0.0f, dold = 0.0f;
+                row_sync<W>();
+                // the new row (up) or column (down) of the pair matrix: two
+                // threads per entry, the chain over the even and the one over
+                // the odd k vectors
+                const int nloop = up ? p.npair + p.nexdn : p.npair + p.nexup;
+                for (int t0 = 0; t0 < 2 * nd; t0 += NR) {
+                    const int e = (t0 + tid) >> 1, h = tid & 1;
+                    float acc = h == 0 ? v0 : 0.0f, rest = 0.0f;
+                    if (e < nloop && e < nd) {
+                        const int jj = up ? e + p.npair + p.nexup : e;
+                        float d2 = 0.0f;
                         for (int c = 0; c < 3; ++c) {
-                            const float a = min_image_f(xf[c] - xsf[3 * j + c], elf, elif);
-                            const float b = min_image_f(xsf[3 * i + c] - xsf[3 * j + c], elf, elif);
-                            dn = fmaf(a, a, dn);
-                            dold = fmaf(b, b, dold);
+                            const float d = min_image_f(xf[c] - xsf[3 * jj + c], elf, elif);
+                            d2 = fmaf(d, d, d2);
                         }
-                        dj[u] = jas_u(p, tud, tss, opp, fmaxf(sqrtf(dn), 1.0e-14f)) -
-                                jas_u(p, tud, tss, opp, fmaxf(sqrtf(dold), 1.0e-14f));
+                        rest = beta_f(p, tud, sqrtf(d2));
+#pragma unroll 10
+                        for (int q = h; q < nq; q += 2) {
+                            const float2 a = onew[q], b = T[q * P + jj];
+                            acc = fmaf(a.x, b.x, fmaf(a.y, b.y, acc));
+                        }
+                    } else if (e < nd) {
+                        const int u = e - nloop;
+                        const double* a = up ? p.akup[u] : p.akdn[u];
+                        const int sn = up ? p.sinup[u] : p.sindn[u];
+                        const float arg = (float)a[0] * xf[0] + (float)a[1] * xf[1] + (float)a[2] * xf[2];
+                        rest = sn ? sinf(arg) : cosf(arg);
                     }
+                    const float odd = __shfl_xor_sync(0xffffffffu, acc, 1);
+                    if (h == 0 && e < nd) snew[e] = e < nloop ? (acc + odd) + rest : rest;
                 }
+            } else {
+                // Jastrow: U(r_i') - U(r_i) over the pairs getphione counts.  A
+                // lane takes its partners j = lane + 32 u kJasLanes at a time, all
+                // their table lookups in flight before any is used; the
+                // differences are added in partner order (skipped pairs add 0).
+                constexpr int kJasLanes = 3;
+                float du = 0.0f;
+                for (int j0 = lane; j0 < P; j0 += 32 * kJasLanes) {
+                    float dj[kJasLanes];
 #pragma unroll
-                for (int u = 0; u < kJasLanes; ++u)
-                    if (j0 + 32 * u < P) du += dj[u];
+                    for (int u = 0; u < kJasLanes; ++u) {
+                        const int j = j0 + 32 * u;
+                        dj[u] = 0.0f;
+                        const bool opp = up != (j < nup);
+                        if (j < P && j != i && (opp || p.ieq)) {
+                            float dn = 0.0f, dold = 0.0f;
+                            for (int c = 0; c < 3; ++c) {
+                                const float a = min_image_f(xf[c] - xsf[3 * j + c], elf, elif);
+                                const float b = min_image_f(xsf[3 * i + c] - xsf[3 * j + c], elf, elif);
+                                dn = fmaf(a, a, dn);
+                                dold = fmaf(b, b, dold);
+                            }
+                            dj[u] = jas_u(p, tud, tss, opp, fmaxf(sqrtf(dn), 1.0e-14f)) -
+                                    jas_u(p, tud, tss, opp, fmaxf(sqrtf(dold), 1.0e-14f));
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < kJasLanes; ++u)
+                        if (j0 + 32 * u < P) du += dj[u];
+                }
+                du = warp_sum_f(du);
+                if (lane == 0) s_du[i & 1] = du;
             }
-            du = warp_sum_f(du);
-            __syncwarp();
+            __syncthreads();
+            // v_k = sum_q s'_q X(q, k) (row i replaced) or w_k = sum_q X(k, q) s'_q
+            // (column c replaced); the ratio is v_i or w_c.  Four partial sums
+            // an entry, two on each of its two threads.
+            const int cix = up ? i : i - nup;
+            const int rs = up ? 1 : ldx, cs = up ? ldx : 1;   // X(q, k) or X(k, q)
+            for (int t0 = 0; t0 < 2 * nd; t0 += NT) {
+                const int k = (t0 + tid) >> 1, h = tid & 1;
+                float a = 0.0f, b = 0.0f;
+                if (k < nd) {
+                    const float* xb = X + k * cs;
+                    int q = 2 * h;
+#pragma unroll 4
+                    for (; q - 2 * h + 3 < nd; q += 4) {
+                        a = fmaf(snew[q], xb[q * rs], a);
+                        b = fmaf(snew[q + 1], xb[(q + 1) * rs], b);
+                    }
+                    if (h == 0)
+                        for (; q < nd; ++q) a = fmaf(snew[q], xb[q * rs], a);
+                }
+                a += b;
+                const float other = __shfl_xor_sync(0xffffffffu, a, 1);
+                if (h == 0 && k < nd) vw[k] = a + other;
+            }
+            __syncthreads();
             const float R = vw[cix];
-            const float prob = R * R * expf(2.0f * du);
+            const float prob = R * R * expf(2.0f * s_du[i & 1]);
             const bool acc = rn < (double)prob;   // R = 0 or NaN: rejected
             if (acc) {
                 const float iR = 1.0f / R;
                 // Sherman-Morrison (rank one): every column (row) but cix first
-                if (up) {
-                    for (int k = lane; k < nd; k += 32) {
-                        if (k == cix) continue;
-                        const float f = vw[k] * iR;
-                        for (int q = 0; q < nd; ++q) X[q + k * ldx] = fmaf(-X[q + cix * ldx], f, X[q + k * ldx]);
-                    }
-                    __syncwarp();
-                    for (int q = lane; q < nd; q += 32) X[q + cix * ldx] *= iR;
-                } else {
-                    for (int k = lane; k < nd; k += 32) {
-                        if (k == cix) continue;
-                        const float f = vw[k] * iR;
-                        for (int q = 0; q < nd; ++q) X[k + q * ldx] = fmaf(-X[cix + q * ldx], f, X[k + q * ldx]);
-                    }
-                    __syncwarp();
-                    for (int q = lane; q < nd; q += 32) X[cix + q * ldx] *= iR;
+                for (int e = tid; e < nd * nd; e += NT) {
+                    const int c = dv.quo(e), r = e - c * nd;
+                    const int k = up ? c : r;
+                    if (k == cix) continue;
+                    const float f = vw[k] * iR;
+                    float* x = X + r + c * ldx;
+                    *x = fmaf(-(up ? X[r + cix * ldx] : X[cix + c * ldx]), f, *x);
                 }
-                for (int q = lane; q < nq; q += 32) T[q * P + i] = oraw[q];
-                if (lane < 3) {
-                    xs[3 * i + lane] = pcur;
-                    xsf[3 * i + lane] = (float)pcur;
+                __syncthreads();
+                for (int q = tid; q < nd; q += NT) X[up ? q + cix * ldx : cix + q * ldx] *= iR;
+                for (int q = tid; q < nq; q += NT) T[q * P + i] = oraw[q];
+                if (tid < 3) {
+                    xs[3 * i + tid] = pcur;
+                    xsf[3 * i + tid] = (float)pcur;
                 }
                 ++nacc;
+                __syncthreads();
             }
-            __syncwarp();
         }
     }
     // ---- write back (the positions are already in the stack) ----
-    for (int e = lane; e < nd * nd; e += 32) {
+    __syncthreads();
+    for (int e = tid; e < nd * nd; e += NT) {
         const int r = e % nd, c = e / nd;
         inv32[(size_t)w * nd * nd + e] = X[r + c * ldx];
     }
-    if (lane == 0) {
+    if (tid == 0) {
         st.irn[w] = s;
         accepted[w] += nacc;
     }
 }
 
 }  // namespace
-
-size_t sweep_smem_bytes(const DevParams& p, int wpc) { return (size_t)wpc * (sweep_warp_floats(p) / 2 + 1) * 8; }
 
 cudaError_t launch_sweeps(const DevParams& p, const DevStack& st, int n, int nsweep, const double* inv64,
                           float* inv32, float2* tab, const KVecMP* kv, const TabUDmp* tud, const TabSSmp* tss,
@@ -336,28 +352,53 @@ cudaError_t launch_sweeps(const DevParams& p, const DevStack& st, int n, int nsw
 {
     if (n <= 0 || nsweep <= 0) return cudaSuccess;
     if (!prop) return cudaErrorInvalidValue;
-    // walkers per CTA: four, or fewer where a walker's shared memory (its
-    // inverse is nd^2 floats) would not fit four times
-    int dev = 0, optin = 0;
+    int dev = 0, optin = 0, nsm = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    int wpc = kSweepWarps;
-    while (wpc > 1 && sweep_smem_bytes(p, wpc) > (size_t)optin) wpc /= 2;
-    const size_t smem = sweep_smem_bytes(p, wpc);
-    if (smem > (size_t)optin) return cudaErrorInvalidValue;
-    if (smem > 48 * 1024) {
-        e = cudaFuncSetAttribute(sweep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // Four warps with the table on chip are the fastest while every walker is
+    // resident.  Beyond that the rounds count: two warps (1.0 to 1.7 of the
+    // time of a round) let twice as many small walkers in, the table in global
+    // memory (1.25 to 1.6) more of the large ones.  us per sweep, four on chip /
+    // two on chip / four with a global table / one warp per walker as before:
+    //   7/7   1024:  39 / 35 / 73 / 76        4096: 155 / 88 / 209 / 90
+    //   19/19 1024: 120 / 147 / 173 / 322     4096: 457 / 369 / 522 / 373
+    //   33/33 1024: 274 / 393 / 330 / 822     1300: 457 / 716 / 377 / 823
+    //         4096: 1022 / 1500 / 1093 / 1029
+    //   66/66  256: 798 / 1322 / 1027 / 2607  1024: 2419 / 3983 / 1347 / 2671
+    struct Variant {
+        decltype(&sweep_kernel<4, true>) kern;
+        int warps;
+        bool onchip;
+        double round;
+    };
+    const Variant variants[3] = {{sweep_kernel<4, true>, 4, true, 1.0},
+                                 {sweep_kernel<2, true>, 2, true, 1.3},
+                                 {sweep_kernel<4, false>, 4, false, 1.35}};
+    const Variant* best = nullptr;
+    double least = 0.0;
+    for (const Variant& v : variants) {
+        const size_t smem = (size_t)walker_floats(p, v.onchip) * 4;
+        if (smem > (size_t)optin) continue;
+        int per_sm = 0;
+        e = cudaFuncSetAttribute(v.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(v.kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                     (int)cudaSharedmemCarveoutMaxShared);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, v.kern, 32 * v.warps, smem);
         if (e != cudaSuccess) return e;
+        if (per_sm < 1) continue;
+        const long long room = (long long)nsm * per_sm;
+        const double cost = (double)((n + room - 1) / room) * v.round;
+        if (!best || cost < least) {
+            best = &v;
+            least = cost;
+        }
     }
-    // the largest shared-memory share of the SM: eight 4-walker CTAs per SM
-    // at N = 66, so that 4096 walkers are resident at once
-    e = cudaFuncSetAttribute(sweep_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             (int)cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return e;
-    const int grid = (n + wpc - 1) / wpc;
-    sweep_kernel<<<grid, 32 * wpc, smem, stream>>>(p, st, n, nsweep, inv64, inv32, tab, kv, tud, tss, jA, jC,
-                                                   accepted, wpc, prop);
+    if (!best) return cudaErrorInvalidValue;
+    best->kern<<<n, 32 * best->warps, (size_t)walker_floats(p, best->onchip) * 4, stream>>>(
+        p, st, nsweep, inv64, inv32, tab, kv, tud, tss, jA, jC, accepted, prop);
     return cudaGetLastError();
 }
 
