@@ -560,6 +560,54 @@ __device__ void fix_positions(const Ctx<double, NT, BIG>& c)
     __syncthreads();
 }
 
+// A pair's distance on the FP64 path: difference vector, length and reciprocal
+// length in units of L 2^-64.  nan: a coordinate of the pair is not finite.
+__device__ __forceinline__ void pair_dist(const DevParams& p, const double* x, const long long* xf, int i, int pj,
+                                          double unit, bool nan, double (&d)[3], double& r, double& ri)
+{
+    const long long e0 = fsub(xf[3 * i], xf[3 * pj]), e1 = fsub(xf[3 * i + 1], xf[3 * pj + 1]);
+    const long long e2 = fsub(xf[3 * i + 2], xf[3 * pj + 2]);
+    d[0] = (double)e0;
+    d[1] = (double)e1;
+    d[2] = (double)e2;
+    if (nan) d[0] = __longlong_as_double(0x7ff8000000000000ll);
+    if (((e0 | e1) | e2) != 0 || nan) {
+        inv_dist(fma(d[0], d[0], fma(d[1], d[1], d[2] * d[2])), r, ri);
+    } else {   // closer than a unit, or coincident: 1/r is large or infinite
+        for (int a = 0; a < 3; ++a) d[a] = min_image(x[3 * i + a] - x[3 * pj + a], p) / unit;
+        r = sqrt(norm2(d[0], d[1], d[2]));
+        ri = 1.0 / r;
+    }
+}
+
+// Jastrow and potential of a pair inside L/2: the sums, and u'/r in gf.
+__device__ __forceinline__ void pair_jastrow(const TabPoly* tpoly, const TabPoly* T, double t, double r, double ri,
+                                             double tscale, double r_min, double two_iu, int ntab, double& tu, double& tv,
+                                             double& td, double& gf)
+{
+    if (r < r_min) {   // the reference's clamp, coshpot.f90:170
+        T = tpoly + grid_split(r_min * tscale, ntab, t);
+        ri = 1.0 / r_min;
+    }
+    tv += poly3(T->c[3], t);
+    tu += poly3(T->c[4], t);
+    gf = poly3(T->c[5], t) * ri;
+    td += fma(gf, two_iu, poly3(T->c[6], t));
+}
+
+// Whether the Jastrow terms of the up-down pairs are taken from a list of the
+// pairs inside the healing distance (grid points up to ntab0 differ from zero)
+// rather than with each pair.  A pair beyond it costs 16 FP64 instructions for
+// nothing, and one pair inside keeps its whole warp there; a listed pair's
+// distance is taken twice (16 again) and the list costs two barriers.  So: at
+// least two pairs a thread, and a healing sphere of at most a sixteenth of the
+// box, (pi/6) (ntab0 / ntab)^3.  A generation of 4096 walkers at N = 66: 1.88 ->
+// 1.73 ms; 1024 at N = 90: 1.08 -> 1.01 ms.
+__device__ __forceinline__ bool jastrow_list(const DevParams& p, int nt)
+{
+    return p.nup * p.ndn >= 2 * nt && 2 * p.ntab0 <= p.ntab;
+}
+
 // ---------------------------------------------------------------------------
 // FP64 path, stages 1 to 3 in one pass over the up-down pairs: Jastrow and
 // potential (coshpot.f90:154-205) and the pair function with beta
@@ -600,81 +648,127 @@ __device__ bool pair_stage64(const Ctx<double, NT, BIG>& c, int mode, double (&j
     if (jas)
         for (int i = threadIdx.x; i < 3 * P; i += NT) du[i] = 0.0;
     __syncthreads();
+    const bool list = jas && jastrow_list(p, NT);
+    // the list and its ballots, in the inverse's second buffer (not in use yet)
+    int* near_q = c.template uat<int>(c.L.S2);
+    unsigned* words = reinterpret_cast<unsigned*>(near_q + pairs);
     const int rows = jas ? c.L.rows64 : nup;
     for (int r0 = 0; r0 < nup; r0 += rows) {
         const int r1 = min(nup, r0 + rows);
         const int npc = (r1 - r0) * ndn;
         const UDiv dv(ndn);
-        for (int q = threadIdx.x; q < npc; q += NT) {
-            const int qi = dv.quo(q);
-            const int i = r0 + qi, j = q - qi * ndn, pj = nup + j;
-            // the integer part first: its temporaries are dead before the distances
-            PhiPair o;
-            if (det) {
-                if (F->fast)
-                    phi_sym(F, tr, P, i, pj, grad, o);
+        for (int q0 = threadIdx.x & ~31; q0 < npc; q0 += NT) {
+            const int q = q0 + (int)(threadIdx.x & 31);
+            bool near = false;
+            if (q < npc) {
+                const int qi = dv.quo(q);
+                const int i = r0 + qi, j = q - qi * ndn, pj = nup + j;
+                // the integer part first: its temporaries are dead before the distances
+                PhiPair o;
+                if (det) {
+                    if (F->fast)
+                        phi_sym(F, tr, P, i, pj, grad, o);
+                    else
+                        phi_octant(F, c.a.phi_oct, tr, P, i, pj, o);
+                }
+                const bool nan = (nf[i] | nf[pj]) != 0;
+                double d[3], r, ri;
+                pair_dist(p, x, xf, i, pj, unit, nan, d, r, ri);
+                const long long rb = __double_as_longlong(r);
+                double t;
+                const int ic = grid_split(r * tscale, p.ntab, t);
+                const TabPoly* T = c.a.tpoly + ic;
+                if (jas) {
+                    double g0 = 0.0, g1 = 0.0, g2 = 0.0;
+                    if (rb < half) {   // r < L/2 (false for NaN)
+                        if (list) {
+                            near = ic - 1 <= p.ntab0;
+                            if (!near) tv += poly3(T->c[3], t);
+                        } else {
+                            pair_jastrow(c.a.tpoly, T, t, r, ri, tscale, r_min, two_iu, p.ntab, tu, tv, td, g0);
+                            g2 = d[2] * g0;
+                            g1 = d[1] * g0;
+                            g0 = d[0] * g0;
+                        }
+                    }
+                    if (!list) {
+                        pv[3 * q + 0] = g0;
+                        pv[3 * q + 1] = g1;
+                        pv[3 * q + 2] = g2;
+                    }
+                }
+                if (det) {
+                    const bool in_b = !p.nobeta && (rb <= half || nan);
+                    double f = in_b ? poly3(T->c[0], t) : 0.0;
+                    if (nan) f = d[0];
+                    S[i * ldS + j] = fma((double)o.f, F->sphi, f);
+                    if (grad) {
+                        double gr = 0.0, lp = 0.0;
+                        if (in_b) {
+                            gr = poly3(T->c[1], t) * ri;
+                            lp = poly3(T->c[2], t);
+                        }
+                        if (nan) gr = lp = d[0];
+                        double* w = w0 + i * ndn + j;
+                        w[0] = fma((double)o.g[0], F->sgrad, gr * d[0]);
+                        w[pairs] = fma((double)o.g[1], F->sgrad, gr * d[1]);
+                        w[2 * pairs] = fma((double)o.g[2], F->sgrad, gr * d[2]);
+                        w[3 * pairs] = fma((double)o.l, F->slap, lp);
+                    } else if (in_b && !isfinite(ri)) {
+                        bad = true;   // the drift would not be finite
+                    }
+                }
+            }
+            if (list) {
+                const unsigned word = __ballot_sync(0xffffffffu, near);
+                if ((threadIdx.x & 31) == 0) words[q0 >> 5] = word;
+            }
+        }
+        if (list) {
+            // the listed pairs in order, then their terms, one pair a thread
+            __syncthreads();
+            const int nwords = (npc + 31) / 32, lane = threadIdx.x & 31;
+            int count = 0;   // every warp counts; each writes its own words' pairs
+            for (int b = 0; b < nwords; b += 32) {
+                unsigned m = b + lane < nwords ? words[b + lane] : 0u;
+                int incl = __popc(m);
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int up = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += up;
+                }
+                if ((lane & (NT / 32 - 1)) == (int)(threadIdx.x >> 5)) {
+                    int at_ = count + incl - __popc(m);
+                    for (; m; m &= m - 1) near_q[at_++] = 32 * (b + lane) + __ffs(m) - 1;
+                }
+                count += __shfl_sync(0xffffffffu, incl, 31);
+            }
+            __syncthreads();
+            for (int k = threadIdx.x; k < count; k += NT) {
+                const int q = near_q[k], qi = dv.quo(q), i = r0 + qi, pj = nup + q - qi * ndn;
+                double d[3], r, ri, t, gf;
+                pair_dist(p, x, xf, i, pj, unit, false, d, r, ri);
+                const TabPoly* T = c.a.tpoly + grid_split(r * tscale, p.ntab, t);
+                pair_jastrow(c.a.tpoly, T, t, r, ri, tscale, r_min, two_iu, p.ntab, tu, tv, td, gf);
+                for (int a = 0; a < 3; ++a) pv[3 * k + a] = d[a] * gf;
+            }
+            __syncthreads();
+            // one thread per (particle, component) adds its pairs in order
+            const int nr = r1 - r0;
+            for (int tc = threadIdx.x; tc < 3 * (nr + ndn); tc += NT) {
+                const int t = tc / 3, cmp = tc % 3;
+                const bool up = t < nr;
+                double s0 = 0.0;
+                for (int k = 0; k < count; ++k) {
+                    const int q = near_q[k], qi = dv.quo(q);
+                    if ((up ? qi : q - qi * ndn + nr) == t) s0 += pv[3 * k + cmp];
+                }
+                if (up)
+                    du[3 * (r0 + t) + cmp] += s0 * p.isqm[0];
                 else
-                    phi_octant(F, c.a.phi_oct, tr, P, i, pj, o);
+                    du[3 * (nup + t - nr) + cmp] -= s0 * p.isqm[1];
             }
-            const bool nan = (nf[i] | nf[pj]) != 0;
-            const long long e0 = fsub(xf[3 * i], xf[3 * pj]), e1 = fsub(xf[3 * i + 1], xf[3 * pj + 1]);
-            const long long e2 = fsub(xf[3 * i + 2], xf[3 * pj + 2]);
-            double d0 = (double)e0, d1 = (double)e1, d2 = (double)e2, r, ri;
-            if (nan) d0 = __longlong_as_double(0x7ff8000000000000ll);
-            if (((e0 | e1) | e2) != 0 || nan) {
-                inv_dist(fma(d0, d0, fma(d1, d1, d2 * d2)), r, ri);
-            } else {   // closer than a unit, or coincident: 1/r is large or infinite
-                d0 = min_image(x[3 * i] - x[3 * pj], p) / unit;
-                d1 = min_image(x[3 * i + 1] - x[3 * pj + 1], p) / unit;
-                d2 = min_image(x[3 * i + 2] - x[3 * pj + 2], p) / unit;
-                r = sqrt(norm2(d0, d1, d2));
-                ri = 1.0 / r;
-            }
-            const long long rb = __double_as_longlong(r);
-            double t;
-            const TabPoly* T = c.a.tpoly + grid_split(r * tscale, p.ntab, t);
-            if (jas) {
-                double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-                if (rb < half) {   // r < L/2 (false for NaN)
-                    const TabPoly* TJ = T;
-                    double tj = t, rj = ri;
-                    if (r < r_min) {   // the reference's clamp, coshpot.f90:170
-                        TJ = c.a.tpoly + grid_split(r_min * tscale, p.ntab, tj);
-                        rj = 1.0 / r_min;
-                    }
-                    tv += poly3(TJ->c[3], tj);
-                    tu += poly3(TJ->c[4], tj);
-                    const double gf = poly3(TJ->c[5], tj) * rj;
-                    td += fma(gf, two_iu, poly3(TJ->c[6], tj));
-                    g0 = d0 * gf;
-                    g1 = d1 * gf;
-                    g2 = d2 * gf;
-                }
-                pv[3 * q + 0] = g0;
-                pv[3 * q + 1] = g1;
-                pv[3 * q + 2] = g2;
-            }
-            if (det) {
-                const bool in_b = !p.nobeta && (rb <= half || nan);
-                double f = in_b ? poly3(T->c[0], t) : 0.0;
-                if (nan) f = d0;
-                S[i * ldS + j] = fma((double)o.f, F->sphi, f);
-                if (grad) {
-                    double gr = 0.0, lp = 0.0;
-                    if (in_b) {
-                        gr = poly3(T->c[1], t) * ri;
-                        lp = poly3(T->c[2], t);
-                    }
-                    if (nan) gr = lp = d0;
-                    double* w = w0 + i * ndn + j;
-                    w[0] = fma((double)o.g[0], F->sgrad, gr * d0);
-                    w[pairs] = fma((double)o.g[1], F->sgrad, gr * d1);
-                    w[2 * pairs] = fma((double)o.g[2], F->sgrad, gr * d2);
-                    w[3 * pairs] = fma((double)o.l, F->slap, lp);
-                } else if (in_b && !isfinite(ri)) {
-                    bad = true;   // the drift would not be finite
-                }
-            }
+            __syncthreads();
+            continue;
         }
         __syncthreads();
         if (!jas) continue;
