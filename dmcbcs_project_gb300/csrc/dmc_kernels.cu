@@ -97,7 +97,8 @@ __global__ void __launch_bounds__(256) estimator_kernel(const double* est, int n
     if ((int)threadIdx.x < 3 * nest) {
         const int ee = (int)threadIdx.x / 3, q = (int)threadIdx.x % 3;
         double t = 0.0;
-        for (int u = 0; u < nsub; ++u) t += red[(u * nest + ee) * 3 + q];
+        const int used = min(nsub, max(k1 - k0, 0));   // the other partial sums are zero
+        for (int u = 0; u < used; ++u) t += red[(u * nest + ee) * 3 + q];
         part[((size_t)blockIdx.x * DMC_NEST_MAX + ee) * 3 + q] = t;
     }
     // the last CTA to finish (threadFenceReduction pattern) combines them
@@ -111,7 +112,10 @@ __global__ void __launch_bounds__(256) estimator_kernel(const double* est, int n
     if ((int)threadIdx.x < 3 * nest) {
         const int ee = (int)threadIdx.x / 3, q = (int)threadIdx.x % 3;
         double t = 0.0;
-        for (int blk = 0; blk < (int)gridDim.x; ++blk) t += __ldcg(part + ((size_t)blk * DMC_NEST_MAX + ee) * 3 + q);
+        // shares without walkers are zero; sixteen loads in flight
+        const int used = per > 0 ? (n + per - 1) / per : 0;
+#pragma unroll 16
+        for (int blk = 0; blk < used; ++blk) t += __ldcg(part + ((size_t)blk * DMC_NEST_MAX + ee) * 3 + q);
         double* dst = q == 0 ? valblk : (q == 1 ? valblk2 : wtblk);
         comp_add(dst[ee], comp[q * DMC_NEST_MAX + ee], t);
     }
@@ -222,6 +226,44 @@ __device__ __forceinline__ unsigned long long ran2_jump(unsigned long long s, un
     return (A * s + C) & kMask48;
 }
 
+// A warp's copy of a walker's vectors, four elements a lane in flight (source
+// and destination may alias for the compiler: a load behind each store waits
+// for memory once per element otherwise).
+__device__ __forceinline__ void copy_vectors(const DevStack& in, const DevStack& out, size_t j, size_t d, int n3, int lane)
+{
+    const double* const src[3] = {in.x + j * n3, in.dpsi + j * n3, in.dpsig + j * n3};
+    double* const dst[3] = {out.x + d * n3, out.dpsi + d * n3, out.dpsig + d * n3};
+    for (int e0 = lane; e0 < n3; e0 += 128) {
+        double v[3][4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (e0 + 32 * u < n3)
+#pragma unroll
+                for (int f = 0; f < 3; ++f) v[f][u] = src[f][e0 + 32 * u];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (e0 + 32 * u < n3)
+#pragma unroll
+                for (int f = 0; f < 3; ++f) dst[f][e0 + 32 * u] = v[f][u];
+    }
+}
+
+// The nine scalars in FP64 that a copied walker keeps, by number.
+__device__ __forceinline__ double* scalar_field(const DevStack& s, int f)
+{
+    switch (f) {
+        case 0: return s.psil;
+        case 1: return s.psigl;
+        case 2: return s.d2psi;
+        case 3: return s.d2psig;
+        case 4: return s.v;
+        case 5: return s.vext;
+        case 6: return s.psil0;
+        case 7: return s.psigl0;
+        default: return s.weight;
+    }
+}
+
 // One warp per output slot d < min(total, cap), so that a walker with many
 // copies is spread over many warps: its source is the pop index m with
 // offs[m] <= d < offs[m + 1] (binary search over the non-decreasing offsets;
@@ -250,25 +292,18 @@ __global__ void branch_scatter_kernel(DevStack in, DevStack out, int n, int n3, 
                 hi = mid - 1;
         }
         const int m = lo, j = n - 1 - m;
-        for (int e = lane; e < n3; e += 32) {
-            out.x[(size_t)d * n3 + e] = in.x[(size_t)j * n3 + e];
-            out.dpsi[(size_t)d * n3 + e] = in.dpsi[(size_t)j * n3 + e];
-            out.dpsig[(size_t)d * n3 + e] = in.dpsig[(size_t)j * n3 + e];
-        }
-        if (lane == 0) {
-            out.psil[d] = in.psil[j];
-            out.psigl[d] = in.psigl[j];
-            out.d2psi[d] = in.d2psi[j];
-            out.d2psig[d] = in.d2psig[j];
-            out.v[d] = in.v[j];
-            out.vext[d] = in.vext[j];
-            out.weight[d] = copysign(1.0, in.weight[j]);
-            out.psil0[d] = in.psil0[j];
-            out.psigl0[d] = in.psigl0[j];
+        // a field a lane: one load and one store deep
+        if (lane < 9) {
+            const double v = scalar_field(in, lane)[j];
+            scalar_field(out, lane)[d] = lane == 8 ? copysign(1.0, v) : v;
+        } else if (lane == 9) {
             out.wt0[d] = in.wt0[j];
+        } else if (lane == 10) {
             out.is[d] = in.is[j];
+        } else if (lane == 11) {
             out.irn[d] = ran2_jump(irn1[m], (unsigned)(d - offs[m]) + 1u);
         }
+        copy_vectors(in, out, j, d, n3, lane);
     }
 }
 
@@ -282,25 +317,15 @@ __global__ void stack_copy_kernel(DevStack from, DevStack to, const int* pn, con
     const int lane = threadIdx.x & 31;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     for (int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < n; j += nwarps) {
-        for (int e = lane; e < n3; e += 32) {
-            to.x[(size_t)j * n3 + e] = from.x[(size_t)j * n3 + e];
-            to.dpsi[(size_t)j * n3 + e] = from.dpsi[(size_t)j * n3 + e];
-            to.dpsig[(size_t)j * n3 + e] = from.dpsig[(size_t)j * n3 + e];
-        }
-        if (lane == 0) {
-            to.psil[j] = from.psil[j];
-            to.psigl[j] = from.psigl[j];
-            to.d2psi[j] = from.d2psi[j];
-            to.d2psig[j] = from.d2psig[j];
-            to.v[j] = from.v[j];
-            to.vext[j] = from.vext[j];
-            to.weight[j] = from.weight[j];
-            to.psil0[j] = from.psil0[j];
-            to.psigl0[j] = from.psigl0[j];
+        if (lane < 9)
+            scalar_field(to, lane)[j] = scalar_field(from, lane)[j];
+        else if (lane == 9)
             to.wt0[j] = from.wt0[j];
+        else if (lane == 10)
             to.is[j] = from.is[j];
+        else if (lane == 11)
             to.irn[j] = from.irn[j];
-        }
+        copy_vectors(from, to, j, j, n3, lane);
     }
 }
 
@@ -435,10 +460,15 @@ cudaError_t launch_branch_dev(const DevStack& in, const DevStack& out, const int
                               unsigned long long* irn1, unsigned long long* wtisto, cudaStream_t st)
 {
     const BranchDev bd{pn, pn_out, need, dfactor, flags};
-    branch_count_kernel<<<nsm * 4, 256, 0, st>>>(in, 0, 1.0, counts, irn1, wtisto, bd, cap);
+    // warps (threads) for a quarter of the stack, which is ten target populations
+    // by default; more walkers go round again.  CTAs without work cost: 2432 of
+    // them 3.4 us a launch.
+    const int quarter = (cap + 3) / 4, warps_grid = max(1, min(nsm * 16, (quarter + 7) / 8));
+    branch_count_kernel<<<max(1, min(nsm * 4, (quarter + 255) / 256)), 256, 0, st>>>(in, 0, 1.0, counts, irn1, wtisto, bd,
+                                                                                     cap);
     scan_kernel<<<1, 1024, 0, st>>>(counts, 0, offs, cap, bd);
-    branch_scatter_kernel<<<nsm * 16, 256, 0, st>>>(in, out, 0, n3, cap, counts, offs, irn1, bd);
-    if (need) stack_copy_kernel<<<nsm * 16, 256, 0, st>>>(out, in, pn_out, need, n3);
+    branch_scatter_kernel<<<warps_grid, 256, 0, st>>>(in, out, 0, n3, cap, counts, offs, irn1, bd);
+    if (need) stack_copy_kernel<<<warps_grid, 256, 0, st>>>(out, in, pn_out, need, n3);
     return cudaGetLastError();
 }
 
@@ -448,28 +478,43 @@ cudaError_t launch_branch_dev(const DevStack& in, const DevStack& out, const int
 // directly; the reference's single-precision wt0 (stack.f90:12) is converted
 // here.  put also leaves the walker count in the device count slot.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ double* host_field(const HostWalkers& h, int f)   // as scalar_field
+{
+    switch (f) {
+        case 0: return h.psil;
+        case 1: return h.psigl;
+        case 2: return h.d2psi;
+        case 3: return h.d2psig;
+        case 4: return h.v;
+        case 5: return h.vext;
+        case 6: return h.psil0;
+        case 7: return h.psigl0;
+        default: return h.weight;
+    }
+}
+
 __global__ void walkers_put_kernel(HostWalkers h, DevStack d, int n, int n3, int* pn)
 {
     const size_t t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (size_t)gridDim.x * blockDim.x;
     const size_t nb = (size_t)n * n3;
     for (size_t e = t0; e < nb; e += nt) {
-        d.x[e] = h.x[e];
-        d.dpsi[e] = h.dpsi[e];
-        d.dpsig[e] = h.dpsig[e];
+        const double a = h.x[e], b = h.dpsi[e], c = h.dpsig[e];
+        d.x[e] = a;
+        d.dpsi[e] = b;
+        d.dpsig[e] = c;
     }
-    for (size_t k = t0; k < (size_t)n; k += nt) {
-        d.psil[k] = h.psil[k];
-        d.psigl[k] = h.psigl[k];
-        d.d2psi[k] = h.d2psi[k];
-        d.d2psig[k] = h.d2psig[k];
-        d.v[k] = h.v[k];
-        d.vext[k] = h.vext[k];
-        d.weight[k] = h.weight[k];
-        d.psil0[k] = h.psil0[k];
-        d.psigl0[k] = h.psigl0[k];
-        d.wt0[k] = (float)h.wt0[k];
-        d.is[k] = h.is[k];
-        d.irn[k] = (unsigned long long)h.irn[k];
+    // a (field, walker) a thread
+    for (size_t t = t0; t < (size_t)n * 12; t += nt) {
+        const int f = (int)(t / n);
+        const size_t k = t - (size_t)f * n;
+        if (f < 9)
+            scalar_field(d, f)[k] = host_field(h, f)[k];
+        else if (f == 9)
+            d.wt0[k] = (float)h.wt0[k];
+        else if (f == 10)
+            d.is[k] = h.is[k];
+        else
+            d.irn[k] = (unsigned long long)h.irn[k];
     }
     if (t0 == 0 && pn) *pn = n;
 }
@@ -482,23 +527,25 @@ __global__ void walkers_get_kernel(DevStack d, HostWalkers h, int n, const int* 
     const size_t t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (size_t)gridDim.x * blockDim.x;
     const size_t nb = (size_t)n * n3;
     for (size_t e = t0; e < nb; e += nt) {
-        if (h.x) h.x[e] = d.x[e];
-        if (h.dpsi) h.dpsi[e] = d.dpsi[e];
-        if (h.dpsig) h.dpsig[e] = d.dpsig[e];
+        const double a = d.x[e], b = d.dpsi[e], c = d.dpsig[e];
+        if (h.x) h.x[e] = a;
+        if (h.dpsi) h.dpsi[e] = b;
+        if (h.dpsig) h.dpsig[e] = c;
     }
-    for (size_t k = t0; k < (size_t)n; k += nt) {
-        if (h.psil) h.psil[k] = d.psil[k];
-        if (h.psigl) h.psigl[k] = d.psigl[k];
-        if (h.d2psi) h.d2psi[k] = d.d2psi[k];
-        if (h.d2psig) h.d2psig[k] = d.d2psig[k];
-        if (h.v) h.v[k] = d.v[k];
-        if (h.vext) h.vext[k] = d.vext[k];
-        if (h.weight) h.weight[k] = d.weight[k];
-        if (h.psil0) h.psil0[k] = d.psil0[k];
-        if (h.psigl0) h.psigl0[k] = d.psigl0[k];
-        if (h.wt0) h.wt0[k] = (double)d.wt0[k];
-        if (h.is) h.is[k] = d.is[k];
-        if (h.irn) h.irn[k] = (long long)d.irn[k];
+    // a (field, walker) a thread
+    for (size_t t = t0; t < (size_t)n * 12; t += nt) {
+        const int f = (int)(t / n);
+        const size_t k = t - (size_t)f * n;
+        if (f < 9) {
+            double* to = host_field(h, f);
+            if (to) to[k] = scalar_field(d, f)[k];
+        } else if (f == 9) {
+            if (h.wt0) h.wt0[k] = (double)d.wt0[k];
+        } else if (f == 10) {
+            if (h.is) h.is[k] = d.is[k];
+        } else if (h.irn) {
+            h.irn[k] = (long long)d.irn[k];
+        }
     }
 }
 
