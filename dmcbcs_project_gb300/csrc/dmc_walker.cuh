@@ -1115,24 +1115,47 @@ __device__ __forceinline__ void bar1_sync() { asm volatile("bar.sync 1, %0;" ::"
 template <int NT>
 __device__ __forceinline__ void bar1_arrive() { asm volatile("bar.arrive 1, %0;" ::"n"(NT) : "memory"); }
 
-constexpr int kPanelWarps = 1;
+// Barrier 2 over the PW panel warps.
+template <int PW>
+__device__ __forceinline__ void bar2_sync() { asm volatile("bar.sync 2, %0;" ::"n"(32 * PW) : "memory"); }
+
+// 1 / p of a pivot: a single-precision reciprocal (converted by shifting
+// exponents, on the integer pipe), then one step of the third-order iteration
+// y <- y + y (e + e^2), e = 1 - p y; three FP64 instructions.  Outside FP32's
+// range the division.
+__device__ __forceinline__ double pivot_rcp(double p)
+{
+    const unsigned hi = (unsigned)__double2hiint(p), lo = (unsigned)__double2loint(p), mag = hi & 0x7fffffffu;
+    if (mag < 0x39000000u || mag >= 0x46c00000u) return 1.0 / p;
+    const unsigned yb = __float_as_uint(__fdividef(1.0f, __uint_as_float(((mag - 0x38000000u) << 3) | (lo >> 29))));
+    const double y = __hiloint2double((int)(((yb >> 3) + 0x38000000u) | (hi & 0x80000000u)), (int)(yb << 29));
+    const double e = fma(-p, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ df pivot_rcp(df p) { return rcp(p); }
 
 // Factor columns k0..k0+bw-1 of A (all n rows, rows pivoted in earlier
 // blocks excluded from the pivot search) by Gauss-Jordan steps restricted
-// to the panel.  Called by warp 0; lane t holds rows t + 32 s (s < RPL) in
-// registers, so the pivot search is a warp reduction (REDUX max of the
-// magnitude keys, then min of the rows that reach it: the first maximum, as
-// idamax) and the pivot row reaches every lane by shuffles.  Records piv[k],
+// to the panel.  Called by the first PW warps; thread t holds rows t + 32 PW s
+// (s < RPL) in registers, so the pivot search is a warp reduction (REDUX max of
+// the magnitude keys, then min of the rows that reach it: the first maximum, as
+// idamax) and the pivot row reaches every lane by shuffles, with PW > 1 both
+// through xch (2 PW (B + 2) values, by the column's parity).  Records piv[k],
 // pvals[k] and rowpos[piv[k]] = k.  Returns false on a zero pivot.
-template <class R, int RPL, int B>
-__device__ __forceinline__ bool gj_panel(R* A, int ld, int n, int k0, int bw, int* piv, R* pvals, int* rowpos)
+// Bound: the column's serial chain, whose FP64 instructions take 64 cycles each
+// however few rows a warp holds; so a warp has one row a lane where that leaves
+// enough warps for the update.  us per generation, one panel warp with all
+// rows and a division per pivot before: FP64 n = 33, 4096 walkers 1733 -> 1700;
+// n = 19, 1024 walkers 304 -> 288; n = 66, 1024 walkers 2048 -> 2030.
+template <class R, int RPL, int B, int PW>
+__device__ __forceinline__ bool gj_panel(R* A, int ld, int n, int k0, int bw, int* piv, R* pvals, int* rowpos, R* xch)
 {
-    const int t = threadIdx.x;
+    const int t = threadIdx.x, warp = t >> 5;
     R v[RPL][B];
     bool done[RPL];
 #pragma unroll
     for (int s = 0; s < RPL; ++s) {
-        const int r = t + 32 * s;
+        const int r = t + 32 * PW * s;
         const bool ok = r < n;
         done[s] = !ok || rowpos[r] < k0;
 #pragma unroll
@@ -1164,22 +1187,55 @@ __device__ __forceinline__ bool gj_panel(R* A, int ld, int n, int k0, int bw, in
                     }
                 gl = __reduce_max_sync(0xffffffffu, ml);
             }
-            if (gh == 0u && gl == 0u) return false;   // no non-zero candidate
+            if (PW == 1 && gh == 0u && gl == 0u) return false;   // no non-zero candidate
             unsigned mine = 0xffffffffu;
 #pragma unroll
             for (int s = RPL - 1; s >= 0; --s)
-                if (!done[s] && kh[s] == gh && mag_lo(v[s][0]) == gl) mine = (unsigned)(t + 32 * s);
-            const int pr = (int)__reduce_min_sync(0xffffffffu, mine);
-            // the pivot row from its lane (slot pr / 32 is the same on every lane)
-            const int ps = pr >> 5, pl = pr & 31;
+                if (!done[s] && kh[s] == gh && mag_lo(v[s][0]) == gl) mine = (unsigned)(t + 32 * PW * s);
+            int pr = (int)__reduce_min_sync(0xffffffffu, mine);
             R rr[B];
+            if constexpr (PW == 1) {
+                // the pivot row from its lane (slot pr / 32 is the same on every lane)
+                const int ps = pr >> 5, pl = pr & 31;
 #pragma unroll
-            for (int c2 = 0; c2 < B; ++c2) {
-                R own = v[0][c2];
+                for (int c2 = 0; c2 < B; ++c2) {
+                    R own = v[0][c2];
 #pragma unroll
-                for (int s = 1; s < RPL; ++s)
-                    if (ps == s) own = v[s][c2];
-                rr[c2] = shfl_r(own, pl);
+                    for (int s = 1; s < RPL; ++s)
+                        if (ps == s) own = v[s][c2];
+                    rr[c2] = shfl_r(own, pl);
+                }
+            } else {
+                // this warp's candidate and its row, then the largest of them
+                R* const x = xch + (c & 1) * PW * (B + 2);
+                unsigned* const key = reinterpret_cast<unsigned*>(x + PW * B);   // [PW][4]
+#pragma unroll
+                for (int s = 0; s < RPL; ++s)
+                    if (t + 32 * PW * s == pr)
+#pragma unroll
+                        for (int c2 = 0; c2 < B; ++c2) x[warp * B + c2] = v[s][c2];
+                if ((t & 31) == 0) {
+                    key[4 * warp] = gh;
+                    key[4 * warp + 1] = gl;
+                    key[4 * warp + 2] = (unsigned)pr;
+                }
+                bar2_sync<PW>();
+                unsigned bh = key[0], bl = key[1], br = key[2];
+                int from = 0;
+#pragma unroll
+                for (int w = 1; w < PW; ++w) {
+                    const unsigned h = key[4 * w], l = key[4 * w + 1], r = key[4 * w + 2];
+                    if (h > bh || (h == bh && (l > bl || (l == bl && r < br)))) {
+                        bh = h;
+                        bl = l;
+                        br = r;
+                        from = w;
+                    }
+                }
+                if (bh == 0u && bl == 0u) return false;
+                pr = (int)br;
+#pragma unroll
+                for (int c2 = 0; c2 < B; ++c2) rr[c2] = x[from * B + c2];
             }
             // Gauss-Jordan step with the unscaled pivot row p and multiplier
             // m = a_c / p_c per row (m = -1/p_c for the pivot row itself):
@@ -1187,10 +1243,10 @@ __device__ __forceinline__ bool gj_panel(R* A, int ld, int n, int k0, int bw, in
             //   a_c  <- -m              (pivot row: 1 / p_c)
             // one multiply per row instead of scaling the pivot row on every lane
             const R pv = rr[0];
-            const R pinv = rcp(pv);
+            const R pinv = pivot_rcp(pv);
 #pragma unroll
             for (int s = 0; s < RPL; ++s) {
-                const bool isp = t + 32 * s == pr;
+                const bool isp = t + 32 * PW * s == pr;
                 const R m = isp ? -pinv : v[s][0] * pinv;
 #pragma unroll
                 for (int c2 = 1; c2 < B; ++c2) v[s][c2] = fms(isp ? rzero<R>() : v[s][c2], m, rr[c2]);
@@ -1214,7 +1270,7 @@ __device__ __forceinline__ bool gj_panel(R* A, int ld, int n, int k0, int bw, in
     }
 #pragma unroll
     for (int s = 0; s < RPL; ++s) {
-        const int r = t + 32 * s;
+        const int r = t + 32 * PW * s;
         if (r < n)
 #pragma unroll
             for (int c = 0; c < B; ++c)
@@ -1240,7 +1296,7 @@ __device__ __forceinline__ R gj_apply(const R* cur, int ld, int i, int j, int k0
     return acc_value(a);
 }
 
-template <class R, int RPL, int B, int NT, bool BIG>
+template <class R, int RPL, int B, int PW, int NT, bool BIG>
 __device__ bool inverse_blocked(const Ctx<R, NT, BIG>& c, double& logdet, int& sgn)
 {
     const DevParams& p = c.p;
@@ -1250,6 +1306,7 @@ __device__ bool inverse_blocked(const Ctx<R, NT, BIG>& c, double& logdet, int& s
     int* piv = reinterpret_cast<int*>(sm + c.L.red + 512);                           // nd ints
     R* pvals = reinterpret_cast<R*>(sm + c.L.red + 512 + 2 * DMC_MAX_PART);          // nd pivots
     int* rowpos = reinterpret_cast<int*>(sm + c.L.red + 512 + 4 * DMC_MAX_PART);     // nd ints
+    R* xch = at<R>(sm, c.L.red);   // the panel warps' exchange
     __shared__ int s_sing;
     __shared__ double s_logdet;
     const int n = p.nd, ld = p.ldS;
@@ -1283,17 +1340,17 @@ __device__ bool inverse_blocked(const Ctx<R, NT, BIG>& c, double& logdet, int& s
                 const int i = db.quo(e), j = k1 + e - i * bw1;
                 nxt[i * ld + j] = gj_apply<R, B>(cur, ld, i, j, k0, bw, prow, rowpos);
             }
-            if (warp < kPanelWarps) {
+            if (warp < PW) {
                 bar1_sync<NT>();
-                if (!gj_panel<R, RPL, B>(nxt, ld, n, k1, bw1, piv, pvals, rowpos) && threadIdx.x == 0) s_sing = 1;
+                if (!gj_panel<R, RPL, B, PW>(nxt, ld, n, k1, bw1, piv, pvals, rowpos, xch) && threadIdx.x == 0) s_sing = 1;
             } else {
                 bar1_arrive<NT>();
             }
         }
-        if (bw1 == 0 || warp >= kPanelWarps) {
+        if (bw1 == 0 || warp >= PW) {
             // every other column: the non-panel warps (all warps in the last block)
-            const int nt = bw1 > 0 ? NT - 32 * kPanelWarps : NT;
-            const int t0 = bw1 > 0 ? (int)threadIdx.x - 32 * kPanelWarps : (int)threadIdx.x;
+            const int nt = bw1 > 0 ? NT - 32 * PW : NT;
+            const int t0 = bw1 > 0 ? (int)threadIdx.x - 32 * PW : (int)threadIdx.x;
             const int nc = n - bw1;
             const UDiv dc(nc);
             for (int e = t0; e < n * nc; e += nt) {
@@ -1522,9 +1579,20 @@ __device__ bool inverse_stage(const Ctx<R, NT, BIG>& c, double& logdet, int& sgn
 {
     const int n = c.p.nd;
     if (c.L.S2 >= 0) {
-        if (n <= 64) return inverse_blocked<R, 2, 6>(c, logdet, sgn);
-        if (n <= 96) return inverse_blocked<R, 3, 8>(c, logdet, sgn);
-        if (n <= 128) return inverse_blocked<R, 4, 8>(c, logdet, sgn);
+        // double-float instructions do not hold the pipe as FP64's do: below 65
+        // rows and above 96 the exchange costs more than the second row (us per
+        // generation with it and without: n = 33, 4096 walkers 1560 and 1531;
+        // n = 100, 512 walkers 3442 and 3295; n = 66, 1024 walkers 1459 and 1524)
+        if constexpr (is_df<R>::value) {
+            if (n <= 64) return inverse_blocked<R, 2, 6, 1>(c, logdet, sgn);
+            if (n <= 96) return inverse_blocked<R, 1, 8, 3>(c, logdet, sgn);
+            if (n <= 128) return inverse_blocked<R, 4, 8, 1>(c, logdet, sgn);
+        } else {
+            if (n <= 32) return inverse_blocked<R, 1, 6, 1>(c, logdet, sgn);
+            if (n <= 64) return inverse_blocked<R, 1, 6, 2>(c, logdet, sgn);
+            if (n <= 96) return inverse_blocked<R, 1, 8, 3>(c, logdet, sgn);
+            if (n <= 128) return inverse_blocked<R, 2, 8, 2>(c, logdet, sgn);
+        }
     }
     return inverse_unblocked<R>(c, logdet, sgn);
 }
@@ -2285,11 +2353,12 @@ __device__ HRes hpsi_eval(const Ctx<R, NT, BIG>& c, int mode)
         for (int i = threadIdx.x; i < n3; i += NT) xr[i] = from_dbl<R>(x[i]);
         __syncthreads();
         pair_stage<R>(c, jt);
+        if (p.ieq) same_spin_stage(c, ss);
     } else {
         fix_positions(c);
         bad = pair_stage64(c, mode, jt);
+        if (p.ieq && mode != MODE_BCS) same_spin_stage(c, ss);
     }
-    if (p.ieq && mode != MODE_BCS) same_spin_stage(c, ss);
     double su = 0.0, sv = 0.0, sd2 = 0.0;
     if (mode == MODE_BCS) {
         for (int i = threadIdx.x; i < n3; i += NT) du[i] = 0.0;
@@ -2327,7 +2396,8 @@ __device__ HRes hpsi_eval(const Ctx<R, NT, BIG>& c, int mode)
             __syncthreads();
         }
         ok = inverse_stage<R>(c, logdet, sgn);
-        if (ok && !(mode == MODE_BCS && c.a.inv_only)) {
+        // (the mixed path always forms the derivatives)
+        if (ok && (is_df<R>::value || !(mode == MODE_BCS && c.a.inv_only))) {
             if constexpr (is_df<R>::value) {
                 drift_stage<R>(c);
                 beta_drift_stage<R>(c);
