@@ -65,8 +65,8 @@ cudaError_t launch_popctl(const int* pn, double nwalk, double popup, double popd
 // Single-particle ratios and parameter derivatives (dmc_single.cu)
 // (sym: the shells are in the symmetric fixed-point form, phi->fast)
 cudaError_t launch_bcsone(const DevParams& p, const KVecDev* kv, const TabUD* tud, const PhiFix* phi,
-                          const TabPoly* tpoly, bool sym, const double* x, const double* smati, const int* ipart,
-                          const double* dr, double* ratio, int nw, cudaStream_t st);
+                          const TabPoly* tpoly, bool sym, const double* x, const double* inv, const int* ipart,
+                          const double* dr, double* ratio, int nw, cudaStream_t st);   // inv: [nw][nd]
 cudaError_t launch_getphione(const DevParams& p, const TabPoly* tpoly, const TabUD* tud, const TabSS* tss,
                              const double* x, const int* ipart, const double* drr, double* ratio, int nw,
                              cudaStream_t st);

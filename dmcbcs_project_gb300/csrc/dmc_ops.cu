@@ -448,7 +448,8 @@ __global__ void __launch_bounds__(kThreads) ops_enk_kernel(const __grid_constant
                 __syncwarp();
             } else {
                 rat1 = single::warp_getphione(p, tud, tss, xs, i, drr);
-                rat2 = single::warp_bcsone(p, kv, tud, xs, S, i, xi);
+                rat2 = i < p.nup ? single::warp_bcsone(p, kv, tud, xs, S + (size_t)i * p.nd, 1, i, xi)
+                                : single::warp_bcsone(p, kv, tud, xs, S + (i - p.nup), p.nd, i, xi);
             }
             const double psirat = rat1 * rat2;
             // cos(dk m dx_c) for m = 0..nnk, c = 0..2, one per lane

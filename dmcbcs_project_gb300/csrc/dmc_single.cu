@@ -46,19 +46,19 @@ __device__ __forceinline__ double move_sum(double v)
 
 // bcsone (psislaterbcs.f90:296-376) with the shells in the symmetric form: an
 // entry is one polynomial of the displacement's axis cosines in fixed point
-// instead of a cosine per k vector (64 walkers at N = 66: 144 -> 10 us)
+// instead of a cosine per k vector (64 walkers at N = 66: 144 -> 10 us).  inv:
+// the moved particle's column (up) or row (down) of the inverse, [nw][nd].
 __global__ void __launch_bounds__(kMoveThreads) bcsone_sym_kernel(const __grid_constant__ DevParams p,
                                                                  const PhiFix* __restrict__ F,
                                                                  const TabPoly* __restrict__ tpoly,
                                                                  const double* __restrict__ x,
-                                                                 const double* __restrict__ smati,
+                                                                 const double* __restrict__ inv,
                                                                  const int* __restrict__ ipart,
                                                                  const double* __restrict__ dr,
                                                                  double* __restrict__ ratio)
 {
     const int w = blockIdx.x, P = p.npart, nd = p.nd;
     const double* xw = x + (size_t)w * 3 * P;
-    const double* S = smati + (size_t)w * nd * nd;
     const int i = ipart[w] - 1;   // checked on the host
     const bool up = i < p.nup;
     const double xi[3] = {xw[3 * i] - dr[3 * w], xw[3 * i + 1] - dr[3 * w + 1], xw[3 * i + 2] - dr[3 * w + 2]};
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(kMoveThreads) bcsone_sym_kernel(const __grid_c
             ph = (up ? p.sinup[u] : p.sindn[u]) ? sin(arg) : cos(arg);
         }
         // up: row i of S replaced, ratio = sum_q Sinv(q,i) phi_q; down: column
-        acc = fma(up ? S[q + (size_t)i * nd] : S[(i - p.nup) + (size_t)q * nd], ph, acc);
+        acc = fma(inv[(size_t)w * nd + q], ph, acc);
     }
     const double r = move_sum(acc);
     if (threadIdx.x == 0) ratio[w] = r;
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(kMoveThreads) bcsone_sym_kernel(const __grid_c
 
 __global__ void bcsone_kernel(const __grid_constant__ DevParams p, const KVecDev* __restrict__ kv,
                               const TabUD* __restrict__ tud, const double* __restrict__ x,
-                              const double* __restrict__ smati, const int* __restrict__ ipart,
+                              const double* __restrict__ inv, const int* __restrict__ ipart,
                               const double* __restrict__ dr, double* __restrict__ ratio, int nw)
 {
     const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -96,7 +96,7 @@ __global__ void bcsone_kernel(const __grid_constant__ DevParams p, const KVecDev
     const double* xw = x + (size_t)w * 3 * P;
     const int i = ipart[w] - 1;   // checked on the host
     const double xi[3] = {xw[3 * i] - dr[3 * w], xw[3 * i + 1] - dr[3 * w + 1], xw[3 * i + 2] - dr[3 * w + 2]};
-    const double r = single::warp_bcsone(p, kv, tud, xw, smati + (size_t)w * nd * nd, i, xi);
+    const double r = single::warp_bcsone(p, kv, tud, xw, inv + (size_t)w * nd, 1, i, xi);
     if (lane == 0) ratio[w] = r;
 }
 
@@ -821,16 +821,16 @@ __global__ void __launch_bounds__(128) sr_sums_kernel(const double* __restrict__
 }  // namespace
 
 cudaError_t launch_bcsone(const DevParams& p, const KVecDev* kv, const TabUD* tud, const PhiFix* phi,
-                          const TabPoly* tpoly, bool sym, const double* x, const double* smati, const int* ipart,
+                          const TabPoly* tpoly, bool sym, const double* x, const double* inv, const int* ipart,
                           const double* dr, double* ratio, int nw, cudaStream_t st)
 {
     if (nw <= 0) return cudaSuccess;
     if (sym) {
-        bcsone_sym_kernel<<<nw, kMoveThreads, 0, st>>>(p, phi, tpoly, x, smati, ipart, dr, ratio);
+        bcsone_sym_kernel<<<nw, kMoveThreads, 0, st>>>(p, phi, tpoly, x, inv, ipart, dr, ratio);
         return cudaGetLastError();
     }
     const int warps = 8;
-    bcsone_kernel<<<(nw + warps - 1) / warps, 32 * warps, 0, st>>>(p, kv, tud, x, smati, ipart, dr, ratio, nw);
+    bcsone_kernel<<<(nw + warps - 1) / warps, 32 * warps, 0, st>>>(p, kv, tud, x, inv, ipart, dr, ratio, nw);
     return cudaGetLastError();
 }
 

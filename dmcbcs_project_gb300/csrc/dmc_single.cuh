@@ -38,10 +38,10 @@ __device__ __forceinline__ double jastrow_u(const DevParams& p, const TabUD* tud
 }
 
 // bcsone (psislaterbcs.f90:296-376) for particle i (0-based) of the walker at
-// xw moved to xi; S is the walker's inverse, column-major as smati.  Called
-// by a whole warp; every lane returns the ratio.
+// xw moved to xi; s[q rs] is entry q of the inverse's column i (up) or of the row
+// of down particle i.  Called by a whole warp; every lane returns the ratio.
 __device__ __forceinline__ double warp_bcsone(const DevParams& p, const KVecDev* __restrict__ kv,
-                                              const TabUD* __restrict__ tud, const double* xw, const double* S, int i,
+                                              const TabUD* __restrict__ tud, const double* xw, const double* s, size_t rs, int i,
                                               const double (&xi)[3])
 {
     const int lane = threadIdx.x & 31, nd = p.nd;
@@ -70,8 +70,7 @@ __device__ __forceinline__ double warp_bcsone(const DevParams& p, const KVecDev*
             ph = sn ? sin(arg) : cos(arg);
         }
         // up: row i of S replaced, ratio = sum_q Sinv(q,i) phi_q; down: column
-        const double s = isup ? S[q + (size_t)i * nd] : S[(i - p.nup) + (size_t)q * nd];
-        acc = fma(s, ph, acc);
+        acc = fma(s[q * rs], ph, acc);
     }
     return walker::warp_sum(acc);
 }
