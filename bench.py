@@ -64,11 +64,12 @@ def algorithmic_flops(nup, ndn, nd, K, npart):
     return 10 * nup * ndn * K + 2 * nd ** 3 + 8 * nd * (nup + ndn) + 60 * P + 40 * nup * ndn + 30 * npart
 
 
-def executed_flops(nup, ndn, nd, K, npart, nk, npairs_active):
-    """FP64 flops of one walker-step as this library computes it: S = U D^T,
-    Gauss-Jordan inverse (nd^3 multiply-adds), the two contraction products
-    G and H (2 nd^2 K multiply-adds each) and about 90 flops per active pair."""
-    return 2 * nup * ndn * K + 2 * nd ** 3 + 4 * nup * ndn * K + 90 * npairs_active + 30 * npart * nk
+def executed_flops(nd, npart, npairs):
+    """FP64 flops of one walker-step as the FP64 path computes it: Gauss-Jordan
+    inverse (nd^3 multiply-adds), about 70 flops per up-down pair, eight
+    multiply-adds per pair against the inverse and about 300 flops per particle
+    (the pair function itself is integer arithmetic)."""
+    return 2 * nd ** 3 + 86 * npairs + 300 * npart
 
 
 class ClockSampler:
@@ -535,7 +536,7 @@ def run_gpu(args):
     e2e = e2e_rate(ctx, info, args, world, barrier)
 
     flops_alg = algorithmic_flops(info.nup, info.ndn, info.nd, info.ncol, info.npart)
-    flops_exe = executed_flops(info.nup, info.ndn, info.nd, info.ncol, info.npart, info.nk, info.nup * info.ndn)
+    flops_exe = executed_flops(info.nd, info.npart, info.nup * info.ndn)
     peak64 = capi.probe_peak("fp64") if rank == 0 else None
     peak32 = capi.probe_peak("fp32") if rank == 0 else None
     dgemm = fp64_peak_tflops(torch) if rank == 0 else None

@@ -12,7 +12,7 @@
 //    for theta = (vorb(1..norb), bfact, b, d) of the pair function
 //    (psislaterbcs.f90:249-293, betafun.f90:12-125) and the 16 knots of the
 //    opt-in Jastrow spline.
-// One warp per walker for the ratios (a few hundred flops each); one CTA per
+// Two warps per walker for the ratios (a few hundred flops each); one CTA per
 // walker for the derivatives, which contract the whole inverse.
 #include <cuda_runtime.h>
 #include <math.h>

@@ -619,8 +619,9 @@ __device__ __forceinline__ bool jastrow_list(const DevParams& p, int nt)
 // and the Jastrow gradients' sums to acc.  jt[] gets the per-thread sums of
 // u, v and the pair Laplacian part; returns whether a pair at distance zero
 // left the derivatives not finite (inv_only, which does not form them).
-// Bound: the FP64 pipe, about 60 of its instructions a pair; the 64 high
-// products run beside it on the integer pipe.
+// Bound: the FP64 pipe, 59 of its instructions a pair (43 where the Jastrow
+// terms come from the list); the 64 high products run beside it on the integer
+// pipe.
 // ---------------------------------------------------------------------------
 template <int NT, bool BIG>
 __device__ bool pair_stage64(const Ctx<double, NT, BIG>& c, int mode, double (&jt)[3])
