@@ -561,7 +561,8 @@ __device__ void fix_positions(const Ctx<double, NT, BIG>& c)
 }
 
 // A pair's distance on the FP64 path: difference vector, length and reciprocal
-// length in units of L 2^-64.  nan: a coordinate of the pair is not finite.
+// length in units of L 2^-64.  nan: a coordinate of the pair is not finite; the
+// vector is then NaN in that component, as are the lengths.
 __device__ __forceinline__ void pair_dist(const DevParams& p, const double* x, const long long* xf, int i, int pj,
                                           double unit, bool nan, double (&d)[3], double& r, double& ri)
 {
@@ -570,8 +571,7 @@ __device__ __forceinline__ void pair_dist(const DevParams& p, const double* x, c
     d[0] = (double)e0;
     d[1] = (double)e1;
     d[2] = (double)e2;
-    if (nan) d[0] = __longlong_as_double(0x7ff8000000000000ll);
-    if (((e0 | e1) | e2) != 0 || nan) {
+    if (((e0 | e1) | e2) != 0 && !nan) {
         inv_dist(fma(d[0], d[0], fma(d[1], d[1], d[2] * d[2])), r, ri);
     } else {   // closer than a unit, or coincident: 1/r is large or infinite
         for (int a = 0; a < 3; ++a) d[a] = min_image(x[3 * i + a] - x[3 * pj + a], p) / unit;
@@ -580,12 +580,13 @@ __device__ __forceinline__ void pair_dist(const DevParams& p, const double* x, c
     }
 }
 
-// Jastrow and potential of a pair inside L/2: the sums, and u'/r in gf.
+// Jastrow and potential of a pair inside L/2, or of one whose distance is not a
+// number: the sums, and u'/r in gf.
 __device__ __forceinline__ void pair_jastrow(const TabPoly* tpoly, const TabPoly* T, double t, double r, double ri,
                                              double tscale, double r_min, double two_iu, int ntab, double& tu, double& tv,
                                              double& td, double& gf)
 {
-    if (r < r_min) {   // the reference's clamp, coshpot.f90:170
+    if (!(r >= r_min)) {   // the reference's clamp, coshpot.f90:170; of NaN, too: its NaN is the vector's
         T = tpoly + grid_split(r_min * tscale, ntab, t);
         ri = 1.0 / r_min;
     }
@@ -681,9 +682,9 @@ __device__ bool pair_stage64(const Ctx<double, NT, BIG>& c, int mode, double (&j
                 const TabPoly* T = c.a.tpoly + ic;
                 if (jas) {
                     double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-                    if (rb < half) {   // r < L/2 (false for NaN)
+                    if (rb < half || nan) {   // r < L/2 (false for NaN)
                         if (list) {
-                            near = ic - 1 <= p.ntab0;
+                            near = ic - 1 <= p.ntab0 || nan;
                             if (!near) tv += poly3(T->c[3], t);
                         } else {
                             pair_jastrow(c.a.tpoly, T, t, r, ri, tscale, r_min, two_iu, p.ntab, tu, tv, td, g0);
@@ -701,7 +702,7 @@ __device__ bool pair_stage64(const Ctx<double, NT, BIG>& c, int mode, double (&j
                 if (det) {
                     const bool in_b = !p.nobeta && (rb <= half || nan);
                     double f = in_b ? poly3(T->c[0], t) : 0.0;
-                    if (nan) f = d[0];
+                    if (nan) f = r;
                     S[i * ldS + j] = fma((double)o.f, F->sphi, f);
                     if (grad) {
                         double gr = 0.0, lp = 0.0;
@@ -709,7 +710,7 @@ __device__ bool pair_stage64(const Ctx<double, NT, BIG>& c, int mode, double (&j
                             gr = poly3(T->c[1], t) * ri;
                             lp = poly3(T->c[2], t);
                         }
-                        if (nan) gr = lp = d[0];
+                        if (nan) gr = lp = r;
                         double* w = w0 + i * ndn + j;
                         w[0] = fma((double)o.g[0], F->sgrad, gr * d[0]);
                         w[pairs] = fma((double)o.g[1], F->sgrad, gr * d[1]);
@@ -747,7 +748,7 @@ __device__ bool pair_stage64(const Ctx<double, NT, BIG>& c, int mode, double (&j
             for (int k = threadIdx.x; k < count; k += NT) {
                 const int q = near_q[k], qi = dv.quo(q), i = r0 + qi, pj = nup + q - qi * ndn;
                 double d[3], r, ri, t, gf;
-                pair_dist(p, x, xf, i, pj, unit, false, d, r, ri);
+                pair_dist(p, x, xf, i, pj, unit, (nf[i] | nf[pj]) != 0, d, r, ri);
                 const TabPoly* T = c.a.tpoly + grid_split(r * tscale, p.ntab, t);
                 pair_jastrow(c.a.tpoly, T, t, r, ri, tscale, r_min, two_iu, p.ntab, tu, tv, td, gf);
                 for (int a = 0; a < 3; ++a) pv[3 * k + a] = d[a] * gf;
