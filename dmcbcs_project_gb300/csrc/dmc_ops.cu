@@ -31,10 +31,29 @@ __device__ __forceinline__ double fix_dist(long long e0, long long e1, long long
     return r;
 }
 
+// The distance that decides a bin near an edge: r, or within 2^-46 of the range
+// (and with `wide` anywhere) the minimum-image distance in FP64 from the
+// positions themselves.
+__device__ __noinline__ double edge_dist(double r, double pos, const double* xi, const double* xj, double el, int ntabg, bool wide)
+{
+    if (!wide && fabs(pos - rint(pos)) > 1.4210854715202004e-14 * ntabg) return r;
+    double r2 = 0.0;
+    for (int c = 0; c < 3; ++c) {
+        double dx = xi[c] - xj[c];
+        dx = dx - el * single::fnint(dx / el);
+        r2 += dx * dx;
+    }
+    return sqrt(r2);
+}
+
 // One CTA per walker.  Distances and plane waves come from positions as
 // 64-bit fractions of the box (dmc_pairfix.cuh): a pair's difference wraps to
 // the minimum image, q.x is an integer combination of a particle's fractions,
 // and rho_q is summed in fixed point (2^54 = 1) by a few threads per q vector.
+// A bin is the direct distance's: the two agree to 2^-47 of the range with both
+// particles within eight boxes, so within 2^-46 of a bin's edge (lattice sites
+// meet the edges exactly), or with a particle farther out, the direct form
+// decides.
 // The FP64 pipe bounds the direct form (three divisions and a root per pair, a
 // sincos per q and particle).
 __global__ void __launch_bounds__(kThreads) ops_walker_kernel(const __grid_constant__ DevParams p,
@@ -53,16 +72,22 @@ __global__ void __launch_bounds__(kThreads) ops_walker_kernel(const __grid_const
     for (int w = blockIdx.x; w < n; w += gridDim.x) {
         const double* xw = x + (size_t)w * 3 * P;
         unsigned long long* rho = reinterpret_cast<unsigned long long*>(sv + (size_t)w * o.nqtot * 4);
-        int nan = 0;   // bit 0, 1: an up, a down coordinate that is not finite
+        int nan = 0;   // bit 0, 1: an up, a down coordinate that is not finite; 2: one beyond eight boxes
         for (int t = threadIdx.x; t < 3 * P; t += kThreads) {
             const double xv = xw[t];
             xf[t] = walker::box_fraction(xv, p.el, p.eli);
             if (!isfinite(xv)) nan |= t < 3 * nup ? 1 : 2;
+            if (!(fabs(xv) <= 8.0 * o.el)) nan |= 4;
         }
         for (int t = threadIdx.x; t < 4 * o.nqtot; t += kThreads) rho[t] = 0ull;
         if (o.ntabg > 0)
             for (int t = threadIdx.x; t < ng + ndh; t += kThreads) g[t] = 0;
-        const bool nan_up = __syncthreads_or(nan & 1) != 0, nan_dn = __syncthreads_or(nan & 2) != 0;
+        bool nan_up = false, nan_dn = false, wide = false;
+        if (__syncthreads_or(nan)) {
+            nan_up = __syncthreads_or(nan & 1) != 0;
+            nan_dn = __syncthreads_or(nan & 2) != 0;
+            wide = __syncthreads_or(nan & 4) != 0;
+        }
         if (o.ntabg > 0) {
             // every pair once (gofr.f90:57-73): particle i with i + 1 .. i + P / 2 around the ring
             const int half = P / 2;
@@ -72,12 +97,15 @@ __global__ void __launch_bounds__(kThreads) ops_walker_kernel(const __grid_const
                 const int j0 = i0 + st < P ? i0 + st : i0 + st - P;
                 const int i = min(i0, j0), j = max(i0, j0);
                 const int itab = (i < nup && j < nup) ? 1 : ((i >= nup && j >= nup) ? 2 : 0);
-                const double r = unit * fix_dist(walker::fsub(xf[3 * i], xf[3 * j]), walker::fsub(xf[3 * i + 1], xf[3 * j + 1]),
-                                                 walker::fsub(xf[3 * i + 2], xf[3 * j + 2]));
-                const bool far = !(r < 0.5 * o.el) ||
-                                 ((nan_up || nan_dn) && !isfinite(xw[3 * i] + xw[3 * i + 1] + xw[3 * i + 2] + xw[3 * j] +
-                                                                  xw[3 * j + 1] + xw[3 * j + 2]));
-                const int index = far ? o.ntabg : (int)(o.scaleg * r);
+                double r = unit * fix_dist(walker::fsub(xf[3 * i], xf[3 * j]), walker::fsub(xf[3 * i + 1], xf[3 * j + 1]),
+                                           walker::fsub(xf[3 * i + 2], xf[3 * j + 2]));
+                double pos = o.scaleg * r;
+                const float at = (float)pos;   // FP32 looks first: 2^-22 of the range
+                if (wide || fabsf(at - rintf(at)) <= 2.3841858e-7f * o.ntabg) {
+                    r = edge_dist(r, pos, xw + 3 * i, xw + 3 * j, o.el, o.ntabg, wide);
+                    pos = o.scaleg * r;
+                }
+                const int index = r < 0.5 * o.el ? (int)pos : o.ntabg;   // NaN counts as far
                 atomicAdd(&g[itab * (o.ntabg + 1) + index], 1);
             }
             // density profile about the origin (gofr.f90:75-90)
