@@ -348,7 +348,8 @@ void fill_params(dmc_ctx* c)
 
 // The FP64 walker path's pair function (PhiFix): amplitudes A(n) of the
 // shells' octant vectors, in units of a power of two above the sum of their
-// magnitudes, so that no partial sum leaves the fixed-point range.  A sum
+// magnitudes, so that no partial sum leaves the fixed-point range (phi and the
+// gradient each in their own: A(0) takes no bits from the gradient).  A sum
 // that is not finite (an amplitude that is not) makes the units NaN.
 int upload_phi(dmc_ctx* c)
 {
@@ -364,11 +365,12 @@ int upload_phi(dmc_ctx* c)
         const int n2 = x * x + y * y + z * z;
         return n2 > n2max ? 0.0 : a[n2] * (1 << ((x != 0) + (y != 0) + (z != 0)));
     };
-    double sum = 0.0, suml = 0.0;
+    double sum = 0.0, sumg = 0.0, suml = 0.0;
     for (int x = 0; x <= M; ++x)
         for (int y = 0; y <= M; ++y)
             for (int z = 0; z <= M; ++z) {
                 sum += std::fabs(amp(x, y, z));
+                if (x + y + z > 0) sumg += std::fabs(amp(x, y, z));
                 suml += (x * x + y * y + z * z) * std::fabs(amp(x, y, z));
             }
     auto unit = [](double v) {   // the power of two above v
@@ -377,7 +379,7 @@ int upload_phi(dmc_ctx* c)
         std::frexp(v, &e);
         return std::ldexp(1.0, e);
     };
-    const double sc = unit(sum), sl = unit(suml), one = 4611686018427387904.0;   // 2^62
+    const double sc = unit(sum), sg = sumg > 0.0 ? std::min(unit(sumg), sc) : sc, sl = unit(suml), one = 4611686018427387904.0;   // 2^62
     const bool fin = std::isfinite(sum) && std::isfinite(suml);
     auto fix = [&](double v, double u) { return fin ? (long long)std::llrint(v / u * one) : 0ll; };
     PhiFix F;
@@ -394,22 +396,24 @@ int upload_phi(dmc_ctx* c)
         for (int m = 0; m < 7; ++m) F.f[m] = fix(w[m] * b[m], sc);
         for (int m = 1; m < 7; ++m) F.f[6 + m] = fix(w[m] * m * b[m], sl);
         const double g1[5] = {2 * b[1], 8 * b[2], 8 * b[3], 8 * b[5], 16 * b[6]}, g2[3] = {2 * b[4], 8 * b[5], 8 * b[6]};
-        for (int m = 0; m < 5; ++m) F.f[13 + m] = fix(g1[m], sc);
-        for (int m = 0; m < 3; ++m) F.f[18 + m] = fix(g2[m], sc);
+        for (int m = 0; m < 5; ++m) F.f[13 + m] = fix(g1[m], sg);
+        for (int m = 0; m < 3; ++m) F.f[18 + m] = fix(g2[m], sg);
     } else {
         const size_t n3 = (size_t)(M + 1) * (M + 1) * (M + 1);
         oct.assign(2 * n3, 0);
         size_t q = 0;
+        F.f[0] = fix(amp(0, 0, 0), sc);
+        F.kphi = std::min(63, std::ilogb(sc) - std::ilogb(sg));
         for (int x = 0; x <= M; ++x)
             for (int y = 0; y <= M; ++y)
                 for (int z = 0; z <= M; ++z, ++q) {
-                    oct[q] = fix(amp(x, y, z), sc);
+                    oct[q] = q ? fix(amp(x, y, z), sg) : 0;
                     oct[n3 + q] = fix((x * x + y * y + z * z) * amp(x, y, z), sl);
                 }
     }
     const double bad = fin ? 1.0 : std::nan("");
     F.sphi = bad * sc / one;
-    F.sgrad = bad * -kap * sc / one * (F.fast ? 4.0 : (double)(1 << F.kM));
+    F.sgrad = bad * -kap * sg / one * (F.fast ? 4.0 : (double)(1 << F.kM));
     F.slap = bad * -kap * kap * sl / one;
     c->phi_sym = F.fast != 0;
     CK(c->phi.alloc(1));

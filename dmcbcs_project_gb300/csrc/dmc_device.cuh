@@ -56,13 +56,15 @@ struct __align__(16) TabPoly {
 // f: coefficients of the symmetric form for |n|^2 <= 6 (walker::PhiPair):
 // [0..6] phi, [7..12] Laplacian, [13..17] and [18..20] the two brackets of
 // the gradient.  Otherwise (fast = 0) the octant tables: entry
-// (nx (M+1) + ny)(M+1) + nz of A / scale, and behind them |n|^2 A / scale.
+// (nx (M+1) + ny)(M+1) + nz of A / scale without n = 0, which is f[0] in units
+// of phi, and behind them |n|^2 A / scale.  The gradient's and the Laplacian's
+// scales leave n = 0 out: it may be the largest by far.
 // sphi, sgrad, slap: one unit of phi, of its gradient, of its Laplacian.
 constexpr int kPhiFast = 21;
 struct PhiFix {
     long long f[kPhiFast];
     double sphi, sgrad, slap;
-    int fast, M, kM, pad;     // octant form: the gradient's terms carry A / 2^kM
+    int fast, M, kM, kphi;    // octant form: the gradient's terms carry A / 2^kM, phi's units are the sum's times 2^kphi
 };
 static_assert(sizeof(PhiFix) == 26 * 8, "staged as 26 doubles");
 

@@ -91,7 +91,8 @@ __device__ __forceinline__ void pair_axes(const long long* tr, int P, int i, int
 }
 
 // The pair function's value, gradient with respect to x_i (without its
-// factor -2 pi / L) and Laplacian (without -(2 pi / L)^2), in PhiFix units.
+// factor -2 pi / L) and Laplacian (without -(2 pi / L)^2), each in its PhiFix
+// units.
 struct PhiPair {
     long long f, g[3], l;
 };
@@ -204,7 +205,7 @@ static __device__ __noinline__ void phi_octant(const PhiFix* F, const long long*
         cx = cn;
         sx = sn;
     }
-    o.f = f;
+    o.f = fadd(F->f[0], f >> F->kphi);
     o.g[0] = gx;
     o.g[1] = gy;
     o.g[2] = gz;
