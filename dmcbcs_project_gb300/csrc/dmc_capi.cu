@@ -711,12 +711,16 @@ static int apply_layout(dmc_ctx* c, const SmemLayout& L, int per_sm)
     const int st_big = std::max(0, walker_big_static_smem_bytes());
     SmemLayout L64{};
     bool found = false;
-    for (int level = 0; level < 3 && !found; ++level) {
-        const int st = level < 2 ? st_on : st_big;
-        const int limit = std::min(smem_sm / per_sm - st - 1024, std::min(optin, 227 * 1024) - 64 - st);
-        L64 = make_layout64(c->P, limit, level);
-        found = (long long)L64.total * 8 <= (long long)limit;
-    }
+    // (with one shell the mixed kernel's k vectors take less room than the pair
+    // function's coefficients, so that it can fit twice where the FP64 kernel
+    // fits once: half of the grid then waits its turn)
+    for (int fit = per_sm; fit > 0 && !found; --fit)
+        for (int level = 0; level < 3 && !found; ++level) {
+            const int st = level < 2 ? st_on : st_big;
+            const int limit = std::min(smem_sm / fit - st - 1024, std::min(optin, 227 * 1024) - 64 - st);
+            L64 = make_layout64(c->P, limit, level);
+            found = (long long)L64.total * 8 <= (long long)limit;
+        }
     if (!found) return fail(c, DMC_ERR_UNSUPPORTED, "the pair matrix does not fit one CTA's shared memory");
     const int stride = std::max(L.gstride, L64.gstride);
     if (stride > 0 && c->gscratch.alloc((size_t)grid * stride) != cudaSuccess)
