@@ -11,6 +11,7 @@
 #include "dmc_device.cuh"
 #include "dmc_kernels.h"
 #include "dmc_attr.h"
+#include "dmc_smem.cuh"
 #include "dmc_walker_kernel.cuh"
 
 namespace dmc {
@@ -619,6 +620,8 @@ int matinv_fits(int n, bool* two_buffers)
     return one <= (size_t)optin ? 1 : 0;
 }
 
+static AttrCache g_attr_inv;
+
 cudaError_t launch_matinv(const double* a, double* inv, double* detl, int* is, int n, int nb, cudaStream_t st)
 {
     DevParams p;
@@ -641,7 +644,7 @@ cudaError_t launch_matinv(const double* a, double* inv, double* detl, int* is, i
         L.total += round_up(n * p.ldS, 2);
     }
     const size_t smem = (size_t)L.total * 8;
-    cudaError_t e = cudaFuncSetAttribute(matinv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_smem(g_attr_inv, 0, matinv_kernel, smem);
     if (e != cudaSuccess) return e;
     matinv_kernel<<<nb, kThreads, smem, st>>>(a, inv, detl, is, n, p, L);
     return cudaGetLastError();

@@ -15,6 +15,7 @@
 #include "dmc_device.cuh"
 #include "dmc_kernels.h"
 #include "dmc_single.cuh"
+#include "dmc_smem.cuh"
 #include "dmc_walker.cuh"
 
 namespace dmc {
@@ -584,6 +585,9 @@ __global__ void __launch_bounds__(kReduceThreads) ops_reduce_kernel(const __grid
 
 }  // namespace
 
+static AttrCache g_attr;
+enum : int { kAttrWalker = 0, kAttrEnkSym, kAttrEnk };
+
 size_t ops_walker_smem(const DevParams& p, const OpsDev& o)
 {
     return sizeof(double) * 3 * p.npart + sizeof(int) * (size_t)(3 * (o.ntabg + 1) + 6 * (2 * o.ntabg + 1)) + 16;
@@ -594,7 +598,7 @@ cudaError_t launch_ops_walker(const DevParams& p, const OpsDev& o, const double*
 {
     if (n <= 0) return cudaSuccess;
     const size_t smem = ops_walker_smem(p, o);
-    cudaError_t e = cudaFuncSetAttribute(ops_walker_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(g_attr, kAttrWalker, ops_walker_kernel, smem);
     if (e != cudaSuccess) return e;
     ops_walker_kernel<<<grid < n ? grid : n, kThreads, smem, st>>>(p, o, x, n, hg, hd, sv);
     return cudaGetLastError();
@@ -614,7 +618,7 @@ cudaError_t launch_ops_enk(const DevParams& p, const OpsDev& o, const KVecDev* k
     cudaDeviceGetAttribute(&optin0, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev0);
     if (sym && (size_t)L.total * 8 <= (size_t)optin0) {
         const size_t smem = (size_t)L.total * 8;
-        cudaError_t e = cudaFuncSetAttribute(ops_enk_sym_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem(g_attr, kAttrEnkSym, ops_enk_sym_kernel, smem);
         int per_sm = 1;
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ops_enk_sym_kernel, kThreads, smem);
         if (e != cudaSuccess) return e;
@@ -630,7 +634,7 @@ cudaError_t launch_ops_enk(const DevParams& p, const OpsDev& o, const KVecDev* k
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     const int tab = with_tab <= (size_t)optin ? 1 : 0;   // plane-wave tables on chip when they fit
     const size_t smem = tab ? with_tab : base;
-    cudaError_t e = cudaFuncSetAttribute(ops_enk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(g_attr, kAttrEnk, ops_enk_kernel, smem);
     if (e != cudaSuccess) return e;
     ops_enk_kernel<<<2 * nsm < n ? 2 * nsm : n, kThreads, smem, st>>>(p, o, kv, tud, tss, x, irn, sinv, n, tk, tab);
     return cudaGetLastError();

@@ -21,6 +21,7 @@
 #include "dmc_kernels.h"
 #include "dmc_walker.cuh"
 #include "dmc_single.cuh"
+#include "dmc_smem.cuh"
 #include "dmc_spline.h"
 
 namespace dmc {
@@ -843,6 +844,9 @@ cudaError_t launch_getphione(const DevParams& p, const TabPoly* tpoly, const Tab
     return cudaGetLastError();
 }
 
+static AttrCache g_attr;
+enum : int { kAttrDerbcs = 0, kAttrPgrad = 1 };   // pgrad: + 1 in the symmetric form
+
 size_t derbcs_smem_bytes(const DevParams& p)
 {
     return sizeof(double) * ((size_t)p.nd * p.nd + 3 * p.npart + 2 * kChunk * p.ndn + (size_t)kChunk * p.nup +
@@ -859,7 +863,7 @@ cudaError_t launch_derbcs(const DevParams& p, const KVecDev* kv, const double* x
         return cudaGetLastError();
     }
     const size_t smem = derbcs_smem_bytes(p);
-    cudaError_t e = cudaFuncSetAttribute(derbcs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(g_attr, kAttrDerbcs, derbcs_kernel, smem);
     if (e != cudaSuccess) return e;
     derbcs_kernel<<<grid < nw ? grid : nw, kThreads, smem, st>>>(p, kv, x, smati, dpsi, nw, stride < 0 ? p.norb : stride,
                                                                  off);
@@ -895,8 +899,7 @@ int pgrad_grid(const DevParams& p, int nw, int nsm, int smem_limit, bool sym)
     const size_t need = pgrad_doubles(p) * 8;
     const int smem = need <= (size_t)smem_limit ? (int)need : 0;
     int per_sm = 1;
-    if (smem > 0 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-        return 0;
+    if (smem > 0 && allow_smem(g_attr, kAttrPgrad + (sym ? 1 : 0), kern, smem) != cudaSuccess) return 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem) != cudaSuccess) return 0;
     const long long g = (long long)(per_sm > 0 ? per_sm : 1) * nsm;
     return (int)(g < nw ? g : (nw > 0 ? nw : 1));
@@ -916,7 +919,7 @@ cudaError_t launch_pgrad(const DevParams& p, const KVecDev* kv, const TabPoly* t
     const bool on_chip = need * 8 <= (size_t)smem_limit;
     const size_t smem = on_chip ? need * 8 : 0;
     if (on_chip) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem(g_attr, kAttrPgrad + (sym ? 1 : 0), kern, smem);
         if (e != cudaSuccess) return e;
     } else if (!gscr) {
         return cudaErrorInvalidValue;

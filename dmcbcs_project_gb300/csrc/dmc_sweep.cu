@@ -32,6 +32,7 @@
 
 #include "dmc_device.cuh"
 #include "dmc_kernels.h"
+#include "dmc_smem.cuh"
 #include "dmc_walker.cuh"
 
 namespace dmc {
@@ -343,6 +344,8 @@ __global__ void __launch_bounds__(128) sweep_kernel(const __grid_constant__ DevP
     }
 }
 
+AttrCache g_attr;   // shared-memory limit and carveout of each variant
+
 }  // namespace
 
 cudaError_t launch_sweeps(const DevParams& p, const DevStack& st, int n, int nsweep, const double* inv64,
@@ -382,10 +385,9 @@ cudaError_t launch_sweeps(const DevParams& p, const DevStack& st, int n, int nsw
         const size_t smem = (size_t)walker_floats(p, v.onchip) * 4;
         if (smem > (size_t)optin) continue;
         int per_sm = 0;
-        e = cudaFuncSetAttribute(v.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(v.kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                     (int)cudaSharedmemCarveoutMaxShared);
+        const int kind = 2 * (int)(&v - variants);
+        e = allow_smem(g_attr, kind, v.kern, smem);
+        if (e == cudaSuccess) e = max_carveout(g_attr, kind + 1, v.kern);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, v.kern, 32 * v.warps, smem);
         if (e != cudaSuccess) return e;
         if (per_sm < 1) continue;
