@@ -83,10 +83,9 @@ struct PinBuf {
     }
 };
 
-// Page-locked staging of the single-particle moves: what a context starts with
-// (512 walkers at N = 66 take 1 MB; allocating it takes longer than the call),
-// and the most it keeps.
-constexpr size_t kMoveStart = 1u << 20, kMoveBytes = 8u << 20;
+// Page-locked staging of the single-particle moves: the largest call whose
+// inputs the kernels read from there, and the most a context keeps.
+constexpr size_t kMoveMapped = 512u << 10, kMoveBytes = 8u << 20;
 
 struct StackBufs {
     DevBuf<double> x, dpsi, dpsig, psil, psigl, d2psi, d2psig, v, vext, weight, psil0, psigl0;
@@ -212,7 +211,8 @@ struct dmc_ctx {
     DevBuf<int> bis;
     DevBuf<unsigned char> flush;
     // single-particle moves and parameter derivatives
-    DevBuf<double> sx, sder, ssinv, srsum, srene;
+    DevBuf<double> sx, sdr, sratio, sder, ssinv, srsum, srene;
+    DevBuf<int> sip;
     PinBuf hmove;                                               // single-particle moves: inputs and ratios
     DevBuf<double> pg_dpsi, pg_dphi, pg_dlog, pg_del, pg_scr;   // adjoint parameter gradients
     DevBuf<PgPoly> pg_btab;                                     // d beta / d b, d beta / d d by grid interval
@@ -769,7 +769,6 @@ int dmc_create(const dmc_system_desc* sd, const dmc_run_desc* rd, dmc_ctx** out)
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
-    if (e == cudaSuccess) e = c->hmove.alloc(kMoveStart / sizeof(double));
     if (e != cudaSuccess) {
         dmc_destroy(c);
         return DMC_ERR_CUDA;
@@ -1698,43 +1697,72 @@ static int check_moves(dmc_ctx* c, int nw, const double* x, const int* ipart, co
     return DMC_OK;
 }
 
+static cudaError_t launch_move(dmc_ctx* c, bool det, const double* x, const double* inv, const int* ip, const double* d,
+                               double* ratio, int n)
+{
+    ++c->launches;
+    return det ? launch_bcsone(c->P, c->kv.p, c->tud.p, c->phi.p, c->tpoly.p, c->phi_sym, x, inv, ip, d, ratio, n, c->stream)
+               : launch_getphione(c->P, c->tpoly.p, c->tud.p, c->tss.p, x, ip, d, ratio, n, c->stream);
+}
+
 // Ratios of nw single-particle moves: bcsone with smati, else getphione.  A
 // move needs its walker's positions and, of the inverse, the nd entries of the
-// moved particle's row or column; these are gathered in page-locked memory,
-// which the kernel reads and writes its ratios to (six copies of pageable arrays
-// and the whole inverses before; both ratios of 64 walkers at N = 66: 272 ->
-// 80 us, of 4096: 1.05 -> 0.96 ms).  Larger calls go in parts of kMoveBytes,
-// which bounds the page-locked memory a context keeps.
+// moved particle's row or column.  A small call gathers these in page-locked
+// memory, which the kernel reads and writes its ratios to: no copies (both
+// ratios of 64 walkers at N = 66: 262 -> 71 us, the kernels' own gain included).  The
+// kernel reads them across the link, once per partner, so beyond kMoveMapped
+// the positions are copied to the device and only the inverse is gathered.
+// getphione, us mapped / copied: N = 66, 512 walkers (0.8 MB) 62 / 57, 4096 339 /
+// 144; N = 132, 512 walkers (1.6 MB) 98 / 65, 4096 909 / 204.
 static int run_moves(dmc_ctx* c, int nw, const double* x, const double* smati, const int* ipart, const double* d,
                      double* ratio)
 {
-    const size_t n3 = (size_t)c->n3, nd = (size_t)c->S.nd, row = smati ? nd : 0, per = n3 + 3 + row + 2;
-    const int part = (int)std::min<size_t>((size_t)nw, std::max<size_t>(1, kMoveBytes / (per * sizeof(double))));
-    CK(c->hmove.alloc((size_t)part * per));
-    for (int w0 = 0; w0 < nw; w0 += part) {
-        const size_t n = (size_t)std::min(part, nw - w0);
+    const size_t n = (size_t)nw, n3 = (size_t)c->n3, nd = (size_t)c->S.nd, row = smati ? nd : 0, per = n3 + 3 + row + 2;
+    // up particle i: the inverse's column i (contiguous in smati); down: its row
+    auto gather = [&](size_t w0, size_t w1, double* to) {
+        for (size_t w = w0; w < w1; ++w, to += nd) {
+            const int i = ipart[w] - 1, nup = c->P.nup;
+            const double* s = smati + w * nd * nd + (i < nup ? (size_t)i * nd : (size_t)(i - nup));
+            const size_t step = i < nup ? 1 : nd;
+            for (size_t q = 0; q < nd; ++q) to[q] = s[q * step];
+        }
+    };
+    if (n * per * sizeof(double) <= kMoveMapped) {
+        CK(c->hmove.alloc(kMoveMapped / sizeof(double)));
         // [n][n3] positions, [n][3] displacements, [n][row] inverse, n particles, then the ratios
         double *hx = c->hmove.p, *hd = hx + n * n3, *hr = hd + 3 * n, *hi = hr + n * row, *out = hi + n;
-        std::memcpy(hx, x + w0 * n3, n * n3 * sizeof(double));
-        std::memcpy(hd, d + 3 * (size_t)w0, 3 * n * sizeof(double));
-        std::memcpy(hi, ipart + w0, n * sizeof(int));
-        for (size_t w = 0; w < n && smati; ++w) {
-            // up particle i: the inverse's column i (contiguous in smati); down: its row
-            const int i = ipart[w0 + w] - 1, nup = c->P.nup;
-            const double* s = smati + (w0 + w) * nd * nd + (i < nup ? (size_t)i * nd : (size_t)(i - nup));
-            const size_t step = i < nup ? 1 : nd;
-            for (size_t q = 0; q < nd; ++q) hr[w * nd + q] = s[q * step];
-        }
-        const int* ip = reinterpret_cast<const int*>(hi);
-        if (smati)
-            CK(launch_bcsone(c->P, c->kv.p, c->tud.p, c->phi.p, c->tpoly.p, c->phi_sym, hx, hr, ip, hd, out, (int)n,
-                             c->stream));
-        else
-            CK(launch_getphione(c->P, c->tpoly.p, c->tud.p, c->tss.p, hx, ip, hd, out, (int)n, c->stream));
-        ++c->launches;
+        std::memcpy(hx, x, n * n3 * sizeof(double));
+        std::memcpy(hd, d, 3 * n * sizeof(double));
+        std::memcpy(hi, ipart, n * sizeof(int));
+        if (smati) gather(0, n, hr);
+        CK(launch_move(c, smati != nullptr, hx, hr, reinterpret_cast<const int*>(hi), hd, out, nw));
         CK(cudaStreamSynchronize(c->stream));
-        std::memcpy(ratio + w0, out, n * sizeof(double));
+        std::memcpy(ratio, out, n * sizeof(double));
+        return DMC_OK;
     }
+    CK(c->sx.alloc(n * n3));
+    CK(c->sip.alloc(n));
+    CK(c->sdr.alloc(3 * n));
+    CK(c->sratio.alloc(n));
+    CK(cudaMemcpyAsync(c->sx.p, x, n * n3 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->sip.p, ipart, n * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->sdr.p, d, 3 * n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    if (smati) {
+        // in parts, which bounds the page-locked memory that a context keeps
+        const size_t part = std::min(n, std::max<size_t>(1, kMoveBytes / (nd * sizeof(double))));
+        CK(c->hmove.alloc(std::max(part * nd, kMoveMapped / sizeof(double))));
+        CK(c->ssinv.alloc(n * nd));
+        for (size_t w0 = 0; w0 < n; w0 += part) {
+            const size_t w1 = std::min(n, w0 + part);
+            if (w0 > 0) CK(cudaStreamSynchronize(c->stream));   // the last part has left the buffer
+            gather(w0, w1, c->hmove.p);
+            CK(cudaMemcpyAsync(c->ssinv.p + w0 * nd, c->hmove.p, (w1 - w0) * nd * sizeof(double), cudaMemcpyHostToDevice,
+                               c->stream));
+        }
+    }
+    CK(launch_move(c, smati != nullptr, c->sx.p, c->ssinv.p, c->sip.p, c->sdr.p, c->sratio.p, nw));
+    CK(cudaMemcpyAsync(ratio, c->sratio.p, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
     return DMC_OK;
 }
 
