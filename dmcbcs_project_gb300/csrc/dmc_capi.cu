@@ -59,6 +59,12 @@ struct DevBuf {
     }
 };
 
+// A part of another allocation.
+template <class T>
+struct DevPtr {
+    T* p = nullptr;
+};
+
 // Page-locked host memory the device addresses, grown on demand.
 struct PinBuf {
     double* p = nullptr;
@@ -157,15 +163,16 @@ struct dmc_ctx {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double last_ms = 0.0;
     // tables
-    DevBuf<KVecDev> kv;
+    DevBuf<unsigned char> shells;   // what the amplitudes decide, one copy per change: kv, kv_mp, phi, phi_oct
+    DevPtr<KVecDev> kv;
     DevBuf<TabUD> tud;
     DevBuf<TabSS> tss;
-    DevBuf<KVecMP> kv_mp;
+    DevPtr<KVecMP> kv_mp;
     DevBuf<TabUDmp> tud_mp;
     DevBuf<TabSSmp> tss_mp;
     DevBuf<TabPoly> tpoly;          // FP64 walker path: tables by grid interval
-    DevBuf<PhiFix> phi;             // and the pair function's fixed-point coefficients
-    DevBuf<long long> phi_oct;
+    DevPtr<PhiFix> phi;             // and the pair function's fixed-point coefficients
+    DevPtr<long long> phi_oct;
     bool phi_sym = false;           // in the symmetric form
     int precision = DMC_PREC_FP64;
     DevBuf<unsigned long long> jumpA, jumpC;
@@ -216,7 +223,9 @@ struct dmc_ctx {
     PinBuf hmove;                                               // single-particle moves: inputs and ratios
     DevBuf<double> pg_dpsi, pg_dphi, pg_dlog, pg_del, pg_scr;   // adjoint parameter gradients
     DevBuf<PgPoly> pg_btab;                                     // d beta / d b, d beta / d d by grid interval
+    bool pg_btab_ok = false;                                    // made with the present b and d
     DevBuf<PgPoly> pg_ktab;                                     // Jastrow knot basis by grid interval
+    DevBuf<double> pg_raw;                                      // the values on the grid that both are made from
     DevBuf<double> pg_slice;                                    // per-CTA slices of the adjoint kernel
     // particle-by-particle sweeps: FP32 inverses carried between calls, the
     // cos/sin tables, accepted moves per walker
@@ -351,7 +360,7 @@ void fill_params(dmc_ctx* c)
 // magnitudes, so that no partial sum leaves the fixed-point range (phi and the
 // gradient each in their own: A(0) takes no bits from the gradient).  A sum
 // that is not finite (an amplitude that is not) makes the units NaN.
-int upload_phi(dmc_ctx* c)
+void make_phi(const dmc_ctx* c, PhiFix& F, std::vector<long long>& oct)
 {
     const Setup& S = c->S;
     int n2max = 0, M = 0;
@@ -382,13 +391,12 @@ int upload_phi(dmc_ctx* c)
     const double sc = unit(sum), sg = sumg > 0.0 ? std::min(unit(sumg), sc) : sc, sl = unit(suml), one = 4611686018427387904.0;   // 2^62
     const bool fin = std::isfinite(sum) && std::isfinite(suml);
     auto fix = [&](double v, double u) { return fin ? (long long)std::llrint(v / u * one) : 0ll; };
-    PhiFix F;
     std::memset(&F, 0, sizeof F);
     F.M = M;
     while ((1 << F.kM) < M) ++F.kM;
     F.fast = n2max <= 6;
     const double kap = 2.0 * 3.14159265358979323846 / S.el;
-    std::vector<long long> oct(1, 0);
+    oct.assign(1, 0);
     if (F.fast) {
         double b[7] = {0, 0, 0, 0, 0, 0, 0};
         for (int m = 0; m <= n2max; ++m) b[m] = a[m];
@@ -415,12 +423,6 @@ int upload_phi(dmc_ctx* c)
     F.sphi = bad * sc / one;
     F.sgrad = bad * -kap * sg / one * (F.fast ? 4.0 : (double)(1 << F.kM));
     F.slap = bad * -kap * kap * sl / one;
-    c->phi_sym = F.fast != 0;
-    CK(c->phi.alloc(1));
-    CK(cudaMemcpy(c->phi.p, &F, sizeof F, cudaMemcpyHostToDevice));
-    CK(c->phi_oct.alloc(oct.size()));
-    CK(cudaMemcpy(c->phi_oct.p, oct.data(), oct.size() * sizeof(long long), cudaMemcpyHostToDevice));
-    return DMC_OK;
 }
 
 int upload_kv(dmc_ctx* c)
@@ -438,8 +440,6 @@ int upload_kv(dmc_ctx* c)
         d.v = q == 0 ? c->S.vorb[0] : 2.0 * c->S.vorb[K.shell - 1];
         d.shell = q == 0 ? 1 : K.shell;
     }
-    CK(c->kv.alloc(kv.size()));
-    CK(cudaMemcpy(c->kv.p, kv.data(), kv.size() * sizeof(KVecDev), cudaMemcpyHostToDevice));
     std::vector<KVecMP> km(kv.size());
     for (size_t q = 0; q < kv.size(); ++q) {
         std::memset(&km[q], 0, sizeof(KVecMP));
@@ -450,22 +450,27 @@ int upload_kv(dmc_ctx* c)
         km[q].k2 = from_double(kv[q].k2);
         km[q].v = from_double(kv[q].v);
     }
-    CK(c->kv_mp.alloc(km.size()));
-    CK(cudaMemcpy(c->kv_mp.p, km.data(), km.size() * sizeof(KVecMP), cudaMemcpyHostToDevice));
+    PhiFix F;
+    std::vector<long long> oct;
+    make_phi(c, F, oct);
+    c->phi_sym = F.fast != 0;
+    // set_vorb at seven shells: 31 us with a copy for each of the four
+    const size_t okm = kv.size() * sizeof(KVecDev), ophi = okm + km.size() * sizeof(KVecMP);
+    const size_t ooct = ophi + (sizeof F + 15) / 16 * 16, total = ooct + oct.size() * sizeof(long long);
+    std::vector<unsigned char> h(total);
+    std::memcpy(h.data(), kv.data(), okm);
+    std::memcpy(h.data() + okm, km.data(), ophi - okm);
+    std::memcpy(h.data() + ophi, &F, sizeof F);
+    std::memcpy(h.data() + ooct, oct.data(), total - ooct);
+    CK(c->shells.alloc(total));
+    unsigned char* d = c->shells.p;
+    c->kv.p = reinterpret_cast<KVecDev*>(d);
+    c->kv_mp.p = reinterpret_cast<KVecMP*>(d + okm);
+    c->phi.p = reinterpret_cast<PhiFix*>(d + ophi);
+    c->phi_oct.p = reinterpret_cast<long long*>(d + ooct);
+    CK(cudaMemcpy(d, h.data(), total, cudaMemcpyHostToDevice));
     c->P.vorb1 = c->S.vorb[0];
-    return upload_phi(c);
-}
-
-// the cubic through four grid points T[0..3] in t = position - 1, from
-// differences (an interval's own points give no cancellation)
-void interval_cubic(const double* T, double* c)
-{
-    const double d1 = T[2] - T[1];
-    const double a3 = ((T[3] - T[0]) - 3.0 * d1) / 6.0, a2 = ((T[0] - T[1]) + d1) / 2.0;
-    c[0] = T[1];
-    c[1] = (d1 - a2) - a3;
-    c[2] = a2;
-    c[3] = a3;
+    return DMC_OK;
 }
 
 int upload_tables(dmc_ctx* c)
@@ -482,13 +487,8 @@ int upload_tables(dmc_ctx* c)
     CK(c->tss.alloc(nt));
     CK(cudaMemcpy(c->tud.p, ud.data(), nt * sizeof(TabUD), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c->tss.p, ss.data(), nt * sizeof(TabSS), cudaMemcpyHostToDevice));
-    std::vector<TabPoly> tp(nt);   // FP64 walker path
-    std::memset(tp.data(), 0, nt * sizeof(TabPoly));
-    const std::vector<double>* src[7] = {&S.btab, &S.dbtab, &S.d2btab, &S.vtab[0], &S.utab[0], &S.dutab[0], &S.d2utab[0]};
-    for (int i = 1; i + 2 < nt; ++i)
-        for (int k = 0; k < 7; ++k) interval_cubic(src[k]->data() + i - 1, tp[i].c[k]);
-    CK(c->tpoly.alloc(nt));
-    CK(cudaMemcpy(c->tpoly.p, tp.data(), nt * sizeof(TabPoly), cudaMemcpyHostToDevice));
+    CK(c->tpoly.alloc(nt));   // FP64 walker path
+    CK(launch_tab_poly(c->tud.p, c->tpoly.p, nt, nullptr));   // behind the copies, on their stream
     // mixed-precision copies in double-float
     std::vector<TabUDmp> udm(nt);
     std::vector<TabSSmp> ssm(nt);
@@ -511,19 +511,22 @@ int upload_tables(dmc_ctx* c)
         CK(c->jq.alloc(S.jq.size()));
         CK(cudaMemcpy(c->jq.p, S.jq.data(), S.jq.size() * sizeof(double), cudaMemcpyHostToDevice));
     }
-    // LCG jump tables for t = 0..nrand+1 steps of ran1
-    const int nj = c->P.nrand + 2;
-    std::vector<unsigned long long> A(nj), C(nj);
-    A[0] = 1;
-    C[0] = 0;
-    for (int t = 1; t < nj; ++t) {
-        A[t] = (A[t - 1] * kMult1) & kMask48;
-        C[t] = (C[t - 1] * kMult1 + kAdd1) & kMask48;
+    if (!c->jumpA.p) {
+        // LCG jump tables for t = 0..nrand+1 steps of ran1
+        const int nj = c->P.nrand + 2;
+        std::vector<unsigned long long> A(nj), C(nj);
+        A[0] = 1;
+        C[0] = 0;
+        for (int t = 1; t < nj; ++t) {
+            A[t] = (A[t - 1] * kMult1) & kMask48;
+            C[t] = (C[t - 1] * kMult1 + kAdd1) & kMask48;
+        }
+        CK(c->jumpA.alloc(nj));
+        CK(c->jumpC.alloc(nj));
+        CK(cudaMemcpy(c->jumpA.p, A.data(), nj * sizeof(unsigned long long), cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(c->jumpC.p, C.data(), nj * sizeof(unsigned long long), cudaMemcpyHostToDevice));
     }
-    CK(c->jumpA.alloc(nj));
-    CK(c->jumpC.alloc(nj));
-    CK(cudaMemcpy(c->jumpA.p, A.data(), nj * sizeof(unsigned long long), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(c->jumpC.p, C.data(), nj * sizeof(unsigned long long), cudaMemcpyHostToDevice));
+    CK(cudaStreamSynchronize(nullptr));
     return DMC_OK;
 }
 
@@ -708,7 +711,6 @@ static int apply_layout(dmc_ctx* c, const SmemLayout& L, int per_sm)
     cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, c->device);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
     const int st_on = std::max(0, walker_static_smem_bytes(c->rd.idmc == 10));
-    const int st_big = std::max(0, walker_big_static_smem_bytes());
     SmemLayout L64{};
     bool found = false;
     // (with one shell the mixed kernel's k vectors take less room than the pair
@@ -716,7 +718,7 @@ static int apply_layout(dmc_ctx* c, const SmemLayout& L, int per_sm)
     // fits once: half of the grid then waits its turn)
     for (int fit = per_sm; fit > 0 && !found; --fit)
         for (int level = 0; level < 3 && !found; ++level) {
-            const int st = level < 2 ? st_on : st_big;
+            const int st = level < 2 ? st_on : std::max(0, walker_big_static_smem_bytes());
             const int limit = std::min(smem_sm / fit - st - 1024, std::min(optin, 227 * 1024) - 64 - st);
             L64 = make_layout64(c->P, limit, level);
             found = (long long)L64.total * 8 <= (long long)limit;
@@ -821,8 +823,8 @@ int dmc_destroy(dmc_ctx* c)
 {
     if (!c) return DMC_OK;
     if (c->stream) cudaStreamSynchronize(c->stream);
-    c->kv.release(); c->tud.release(); c->tss.release(); c->kv_mp.release(); c->tud_mp.release();
-    c->tss_mp.release(); c->tpoly.release(); c->phi.release(); c->phi_oct.release(); c->jumpA.release(); c->jumpC.release(); c->jq.release();
+    c->shells.release(); c->tud.release(); c->tss.release(); c->tud_mp.release();
+    c->tss_mp.release(); c->tpoly.release(); c->jumpA.release(); c->jumpC.release(); c->jq.release();
     c->gscratch.release(); c->st[0].release(); c->st[1].release(); c->est.release(); c->counts.release();
     c->offs.release(); c->status.release(); c->wstat.release(); c->irn1.release(); c->wtisto.release(); c->vb.release();
     c->bx.release(); c->bpsil.release(); c->bdpsi.release();
@@ -1822,21 +1824,22 @@ static int pgrad_nbeta(const dmc_ctx* c) { return c->P.nobeta ? 0 : 3; }
 static int pgrad_nknot(const dmc_ctx* c) { return (int)c->S.jknots.size(); }
 static int pgrad_np(const dmc_ctx* c) { return c->S.norb + pgrad_nbeta(c) + pgrad_nknot(c); }
 
-// the b and d derivative tables of beta on the device (built once: b and d
-// do not change during a context's life)
+// the b and d derivative tables of beta on the device, made anew for new b and d
 static int pgrad_btab(dmc_ctx* c)
 {
-    if (c->P.nobeta || c->pg_btab.p) return DMC_OK;
+    if (c->P.nobeta || c->pg_btab_ok) return DMC_OK;
     std::vector<double> t[2][3];
     c->S.beta_param_tables(t);
     const size_t nt = (size_t)c->S.ntabb + 1;
-    std::vector<PgPoly> h(2 * nt);
-    std::memset(h.data(), 0, h.size() * sizeof(PgPoly));
-    for (size_t i = 1; i + 2 < nt; ++i)
-        for (int w = 0; w < 2; ++w)
-            for (int m = 0; m < 3; ++m) interval_cubic(t[w][m].data() + i - 1, h[2 * i + w].c[m]);
+    std::vector<double> h(6 * nt);   // [3][2][nt]
+    for (int m = 0; m < 3; ++m)
+        for (int w = 0; w < 2; ++w) std::copy(t[w][m].begin(), t[w][m].begin() + nt, h.begin() + (2 * m + w) * nt);
+    CK(c->pg_raw.alloc(h.size()));
     CK(c->pg_btab.alloc(2 * nt));
-    CK(cudaMemcpy(c->pg_btab.p, h.data(), 2 * nt * sizeof(PgPoly), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(c->pg_raw.p, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice));
+    CK(launch_pg_poly(c->pg_raw.p, c->pg_btab.p, 2, (int)nt, nullptr));
+    CK(cudaStreamSynchronize(nullptr));
+    c->pg_btab_ok = true;
     return DMC_OK;
 }
 
@@ -1848,13 +1851,15 @@ static int pgrad_ktab(dmc_ctx* c)
     std::vector<double> t[3];
     c->S.knot_basis_tables(t);
     const size_t nk = c->S.jknots.size(), nt = t[0].size() / nk;
-    std::vector<PgPoly> h(t[0].size());
-    std::memset(h.data(), 0, h.size() * sizeof(PgPoly));
-    for (size_t i = 1; i + 2 < nt; ++i)
-        for (size_t k = 0; k < nk; ++k)
-            for (int m = 0; m < 3; ++m) interval_cubic(t[m].data() + k * nt + i - 1, h[i * nk + k].c[m]);
-    CK(c->pg_ktab.alloc(h.size()));
-    CK(cudaMemcpy(c->pg_ktab.p, h.data(), h.size() * sizeof(PgPoly), cudaMemcpyHostToDevice));
+    CK(c->pg_raw.alloc(3 * nk * nt));   // [3][16][nt]
+    for (int m = 0; m < 3; ++m)
+        CK(cudaMemcpy(c->pg_raw.p + m * nk * nt, t[m].data(), nk * nt * sizeof(double), cudaMemcpyHostToDevice));
+    DevBuf<PgPoly> tab;
+    CK(tab.alloc(nk * nt));
+    CK(launch_pg_poly(c->pg_raw.p, tab.p, (int)nk, (int)nt, nullptr));
+    CK(cudaStreamSynchronize(nullptr));
+    std::swap(c->pg_ktab.p, tab.p);
+    std::swap(c->pg_ktab.n, tab.n);
     return DMC_OK;
 }
 
@@ -1933,7 +1938,7 @@ int dmc_set_beta(dmc_ctx* c, double b, double d, double bfact)
     c->sd.bbeta = b;
     c->sd.dbeta = d;
     c->sd.bfact = bfact;
-    c->pg_btab.release();   // the b and d derivative tables follow on the next gradient
+    c->pg_btab_ok = false;   // the b and d derivative tables follow on the next gradient
     return upload_tables(c);
 }
 

@@ -91,6 +91,11 @@ constexpr int kPgradMax = DMC_MAX_SHELLS + 3 + 16;
 struct __align__(16) PgPoly {
     double c[3][4];
 };
+// The cubics through each grid interval's four points, zero where there are
+// none (the last two intervals and the first): of the up-down tables, and of n
+// functions given with their derivatives as raw[3][n][nt], to out[nt][n].
+cudaError_t launch_tab_poly(const TabUD* tud, TabPoly* out, int nt, cudaStream_t st);
+cudaError_t launch_pg_poly(const double* raw, PgPoly* out, int n, int nt, cudaStream_t st);
 // adjoint parameter gradients (dmc_single.cu): doubles of one CTA's core
 // (on chip when it fits in smem_limit bytes, else in gscr: grid x that) and
 // of its global slice (slices: grid x that, always); the grid that keeps

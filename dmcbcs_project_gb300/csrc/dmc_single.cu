@@ -821,6 +821,55 @@ __global__ void __launch_bounds__(128) sr_sums_kernel(const double* __restrict__
 
 }  // namespace
 
+// The cubic through four grid points in t = position - 1, from differences (an
+// interval's own points give no cancellation).
+__device__ __forceinline__ void interval_cubic(double t0, double t1, double t2, double t3, double* c)
+{
+    const double d1 = t2 - t1;
+    const double a3 = fma(-3.0, d1, t3 - t0) / 6.0, a2 = ((t0 - t1) + d1) * 0.5;
+    c[0] = t1;
+    c[1] = (d1 - a2) - a3;
+    c[2] = a2;
+    c[3] = a3;
+}
+
+// One thread per cubic.  Made on the host and copied, they cost set_beta 0.18 ms
+// (716 -> 541 us) and the gradient after it as much again.
+__global__ void tab_poly_kernel(const TabUD* __restrict__ tud, TabPoly* __restrict__ out, int nt)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, i = t / 7, k = t - 7 * i;
+    if (i >= nt) return;
+    double c[4] = {0.0, 0.0, 0.0, 0.0};
+    if (i >= 1 && i + 2 < nt) {
+        constexpr int field[7] = {4, 5, 6, 0, 1, 2, 3};   // beta, beta', lap beta, v, u, u', u'' in a TabUD
+        const double* T = reinterpret_cast<const double*>(tud + i - 1) + field[k];
+        constexpr int ld = sizeof(TabUD) / 8;
+        interval_cubic(T[0], T[ld], T[2 * ld], T[3 * ld], c);
+    }
+    for (int m = 0; m < 4; ++m) out[i].c[k][m] = c[m];
+}
+__global__ void pg_poly_kernel(const double* __restrict__ raw, PgPoly* __restrict__ out, int n, int nt)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, i = t / (3 * n), f = (t - 3 * n * i) / 3, m = t % 3;
+    if (i >= nt) return;
+    double c[4] = {0.0, 0.0, 0.0, 0.0};
+    const double* T = raw + ((size_t)m * n + f) * nt + i - 1;
+    if (i >= 1 && i + 2 < nt) interval_cubic(T[0], T[1], T[2], T[3], c);
+    for (int q = 0; q < 4; ++q) out[(size_t)i * n + f].c[m][q] = c[q];
+}
+
+cudaError_t launch_tab_poly(const TabUD* tud, TabPoly* out, int nt, cudaStream_t st)
+{
+    static_assert(sizeof(TabUD) == 64, "fields by number");
+    tab_poly_kernel<<<(7 * nt + 255) / 256, 256, 0, st>>>(tud, out, nt);
+    return cudaGetLastError();
+}
+cudaError_t launch_pg_poly(const double* raw, PgPoly* out, int n, int nt, cudaStream_t st)
+{
+    pg_poly_kernel<<<(3 * n * nt + 255) / 256, 256, 0, st>>>(raw, out, n, nt);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_bcsone(const DevParams& p, const KVecDev* kv, const TabUD* tud, const PhiFix* phi,
                           const TabPoly* tpoly, bool sym, const double* x, const double* inv, const int* ipart,
                           const double* dr, double* ratio, int nw, cudaStream_t st)
