@@ -590,7 +590,7 @@ matinv_kernel(const double* a, double* inv, double* detl, int* is, int n, DevPar
     Ctx<double> ctx{p, dummy, L, sm, nullptr};
     double logdet;
     int sg;
-    const bool ok = walker::inverse_stage<double>(ctx, logdet, sg);
+    const bool ok = walker::inverse_stage<double, true>(ctx, logdet, sg);
     for (int t = threadIdx.x; t < n * n; t += kThreads) {
         const int r = t % n, cc = t / n;
         inv[b * n2 + t] = sm[L.S + r * p.ldS + cc];

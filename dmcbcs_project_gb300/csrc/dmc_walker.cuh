@@ -1145,10 +1145,9 @@ __device__ __forceinline__ df pivot_rcp(df p) { return rcp(p); }
 // through xch (2 PW (B + 2) values, by the column's parity).  Records piv[k],
 // pvals[k] and rowpos[piv[k]] = k.  Returns false on a zero pivot.
 // Bound: the column's serial chain, whose FP64 instructions take 64 cycles each
-// however few rows a warp holds; so a warp has one row a lane where that leaves
-// enough warps for the update.  us per generation, one panel warp with all
-// rows and a division per pivot before: FP64 n = 33, 4096 walkers 1733 -> 1700;
-// n = 19, 1024 walkers 304 -> 288; n = 66, 1024 walkers 2048 -> 2030.
+// however few rows a warp holds; inverse_stage chooses the warps.  A division per
+// pivot instead of pivot_rcp: FP64, 1024 walkers, n = 33 497 -> 502 us per
+// generation, n = 19 293 -> 296.
 template <class R, int RPL, int B, int PW>
 __device__ __forceinline__ bool gj_panel(R* A, int ld, int n, int k0, int bw, int* piv, R* pvals, int* rowpos, R* xch)
 {
@@ -1576,24 +1575,33 @@ __device__ bool inverse_unblocked(const Ctx<R, NT, BIG>& c, double& logdet, int&
     return !sing;
 }
 
-template <class R, int NT, bool BIG>
+template <class R, bool ALONE = false, int NT, bool BIG>
 __device__ bool inverse_stage(const Ctx<R, NT, BIG>& c, double& logdet, int& sgn)
 {
     const int n = c.p.nd;
     if (c.L.S2 >= 0) {
-        // double-float instructions do not hold the pipe as FP64's do: below 65
-        // rows and above 96 the exchange costs more than the second row (us per
-        // generation with it and without: n = 33, 4096 walkers 1560 and 1531;
-        // n = 100, 512 walkers 3442 and 3295; n = 66, 1024 walkers 1459 and 1524)
+        // A panel's chain is shorter with a row a lane on more warps, the update
+        // beside it longer.  Three panel warps pay with sixteen warps (mixed), not
+        // with eight (us per generation of 1024 walkers, three panel warps / one:
+        // mixed n = 66, 512 threads, 1473 / 1534, at three shells n = 80 1875 / 1924;
+        // 256 threads, n = 76 2441 / 2304, n = 90 4742 / 4310; FP64, always 256, n =
+        // 66 2023 / 2030, n = 76 2227 / 2130, n = 90 4108 / 3880).  FP64
+        // instructions hold their pipe whatever the rows, so there the second warp
+        // pays while it is not full (n = 40 826 / 856, n = 48 1061 / 1073, n = 56 1487
+        // / 1455, n = 64 1793 / 1730) and for four rows, where one lane's do not fit
+        // the walker kernel's registers (n = 112 6986 / 7552; ALONE, the batched
+        // inverse, has them all: 64 matrices of n = 120 2057 / 1905), in double-float
+        // not at all (n = 33, 4096 walkers 1560 / 1531; n = 100 no difference).
         if constexpr (is_df<R>::value) {
             if (n <= 64) return inverse_blocked<R, 2, 6, 1>(c, logdet, sgn);
-            if (n <= 96) return inverse_blocked<R, 1, 8, 3>(c, logdet, sgn);
+            if (n <= 96) return inverse_blocked<R, (NT > kThreads ? 1 : 3), 8, (NT > kThreads ? 3 : 1)>(c, logdet, sgn);
             if (n <= 128) return inverse_blocked<R, 4, 8, 1>(c, logdet, sgn);
         } else {
             if (n <= 32) return inverse_blocked<R, 1, 6, 1>(c, logdet, sgn);
-            if (n <= 64) return inverse_blocked<R, 1, 6, 2>(c, logdet, sgn);
-            if (n <= 96) return inverse_blocked<R, 1, 8, 3>(c, logdet, sgn);
-            if (n <= 128) return inverse_blocked<R, 2, 8, 2>(c, logdet, sgn);
+            if (n <= 52) return inverse_blocked<R, 1, 6, 2>(c, logdet, sgn);
+            if (n <= 64) return inverse_blocked<R, 2, 6, 1>(c, logdet, sgn);
+            if (n <= 96) return inverse_blocked<R, 3, 8, 1>(c, logdet, sgn);
+            if (n <= 128) return inverse_blocked<R, (ALONE ? 4 : 2), 8, (ALONE ? 1 : 2)>(c, logdet, sgn);
         }
     }
     return inverse_unblocked<R>(c, logdet, sgn);
