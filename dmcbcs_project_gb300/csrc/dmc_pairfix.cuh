@@ -157,7 +157,9 @@ __device__ __forceinline__ void phi_sym(const PhiFix* F, const long long* tr, in
 }
 
 // Octant form for any shells: c_m, s_m by the recurrence x_{m+1} = 2 c_1 x_m
-// - x_{m-1}, the z sum innermost.
+// - x_{m-1}, the z sum innermost.  o.f is left without n = 0 and in the gradient's
+// units: phi_value (here it would hold F's registers through the loops, which
+// cost the walker kernel 1 %).
 static __device__ __noinline__ void phi_octant(const PhiFix* F, const long long* oct, const long long* tr, int P, int i, int j,
                                         PhiPair& o)
 {
@@ -205,12 +207,14 @@ static __device__ __noinline__ void phi_octant(const PhiFix* F, const long long*
         cx = cn;
         sx = sn;
     }
-    o.f = fadd(F->f[0], f >> F->kphi);
+    o.f = f;
     o.g[0] = gx;
     o.g[1] = gy;
     o.g[2] = gz;
     o.l = l;
 }
+
+__device__ __forceinline__ long long phi_value(const PhiFix* F, long long f) { return fadd(F->f[0], f >> F->kphi); }
 
 // ---- FP64 ------------------------------------------------------------------
 

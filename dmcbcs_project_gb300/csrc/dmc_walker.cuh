@@ -668,23 +668,25 @@ __device__ bool pair_stage64(const Ctx<double, NT, BIG>& c, int mode, double (&j
                 // the integer part first: its temporaries are dead before the distances
                 PhiPair o;
                 if (det) {
-                    if (F->fast)
+                    if (F->fast) {
                         phi_sym(F, tr, P, i, pj, grad, o);
-                    else
+                    } else {
                         phi_octant(F, c.a.phi_oct, tr, P, i, pj, o);
+                        o.f = phi_value(F, o.f);
+                    }
                 }
                 const bool nan = (nf[i] | nf[pj]) != 0;
                 double d[3], r, ri;
                 pair_dist(p, x, xf, i, pj, unit, nan, d, r, ri);
-                const long long rb = __double_as_longlong(r);
+                const long long rb = nan ? 0 : __double_as_longlong(r);   // NaN takes the near branches
                 double t;
                 const int ic = grid_split(r * tscale, p.ntab, t);
                 const TabPoly* T = c.a.tpoly + ic;
                 if (jas) {
                     double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-                    if (rb < half || nan) {   // r < L/2 (false for NaN)
+                    if (rb < half) {   // r < L/2
                         if (list) {
-                            near = ic - 1 <= p.ntab0 || nan;
+                            near = ic - 1 <= p.ntab0;   // (the interval of NaN is the first)
                             if (!near) tv += poly3(T->c[3], t);
                         } else {
                             pair_jastrow(c.a.tpoly, T, t, r, ri, tscale, r_min, two_iu, p.ntab, tu, tv, td, g0);
@@ -700,7 +702,7 @@ __device__ bool pair_stage64(const Ctx<double, NT, BIG>& c, int mode, double (&j
                     }
                 }
                 if (det) {
-                    const bool in_b = !p.nobeta && (rb <= half || nan);
+                    const bool in_b = !p.nobeta && rb <= half;
                     double f = in_b ? poly3(T->c[0], t) : 0.0;
                     if (nan) f = r;
                     S[i * ldS + j] = fma((double)o.f, F->sphi, f);
