@@ -337,6 +337,7 @@ void fill_params(dmc_ctx* c)
         p.sigma[s] = S.sigma[s];
         p.dcut[s] = S.dcut[s];
     }
+    p.imu_ud = 1.0 / (S.mass[0] * S.mass[1] / (S.mass[0] + S.mass[1]));
     p.hbar = S.hbar; p.a2 = S.a2; p.dt = c->rd.dt; p.etrial = S.etrial; p.wtcut = c->rd.wtcut; p.nfac = S.nfac;
     for (int k = 0; k < 3; ++k) p.qex[k] = S.qex[k];
     p.v0ex = S.v0ex; p.v0exjas = S.v0exjas; p.vorb1 = S.vorb[0];

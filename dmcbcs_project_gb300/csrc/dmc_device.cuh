@@ -103,7 +103,7 @@ struct DevParams {
     double jbeta, jgamma; // its parameters
     int ldS, ldU;
     double el, eli, range, scale, rangeb, scaleb;
-    double mass[2], sqm[2], imass[2], isqm[2];
+    double mass[2], sqm[2], imass[2], isqm[2], imu_ud;   // imu_ud: over the reduced mass of an up-down pair
     double hbar, a2, dt, etrial, wtcut, nfac;
     double sigma[2], dcut[2];
     double qex[3], v0ex, v0exjas, vorb1;

@@ -537,12 +537,12 @@ __device__ void same_spin_stage(const Ctx<R, NT, BIG>& c, double (&ss)[3])
 
 // ---------------------------------------------------------------------------
 // FP64 path, before the pairs: positions as 64-bit fractions of the box
-// (differences then wrap to the minimum image by themselves), the axis
-// angles' cos and sin, and a flag per particle with a coordinate that is not
+// (differences then wrap to the minimum image by themselves), with the
+// determinant the axis angles' cos and sin, and a flag per particle with a coordinate that is not
 // finite (such a particle's pairs get NaN, as its distances would).
 // ---------------------------------------------------------------------------
 template <int NT, bool BIG>
-__device__ void fix_positions(const Ctx<double, NT, BIG>& c)
+__device__ void fix_positions(const Ctx<double, NT, BIG>& c, bool det)
 {
     const DevParams& p = c.p;
     double* sm = c.sm;
@@ -554,7 +554,7 @@ __device__ void fix_positions(const Ctx<double, NT, BIG>& c)
         const int pt = t / 3, a = t - 3 * pt;
         const long long f = box_fraction(x[t], p.el, p.eli);
         xf[t] = f;
-        fix_sincos(f, tr[(2 * a) * p.npart + pt], tr[(2 * a + 1) * p.npart + pt]);
+        if (det) fix_sincos(f, tr[(2 * a) * p.npart + pt], tr[(2 * a + 1) * p.npart + pt]);
         if (a == 0) nf[pt] = !(isfinite(x[t]) && isfinite(x[t + 1]) && isfinite(x[t + 2]));
     }
     __syncthreads();
@@ -642,9 +642,9 @@ __device__ bool pair_stage64(const Ctx<double, NT, BIG>& c, int mode, double (&j
     const bool jas = mode != MODE_BCS, det = mode != MODE_GETPHI, grad = det && !(mode == MODE_BCS && c.a.inv_only);
     const double unit = p.el * 5.421010862427522e-20;    // L 2^-64: distances below are in this unit, L/2 = 2^63
     const double tscale = (double)p.ntab * 1.0842021724855044e-19;   // grid points per unit: ntab / 2^63
-    const double r_min = 1.0e-14 / unit, two_iu = 2.0 / unit;
+    // 2 / unit and 1e-14 / unit (no division here: one takes 1300 cycles of every walker's time)
+    const double two_iu = 3.6893488147419103e19 * p.eli, r_min = 0.5e-14 * two_iu;
     const long long half = 0x43E0000000000000ll;         // 2^63 as a double's bits
-    const double imu_ud = 1.0 / (p.mass[0] * p.mass[1] / (p.mass[0] + p.mass[1]));
     double tu = 0.0, tv = 0.0, td = 0.0;
     bool bad = false;
     if (jas)
@@ -806,7 +806,7 @@ __device__ bool pair_stage64(const Ctx<double, NT, BIG>& c, int mode, double (&j
     }
     jt[0] = tu;
     jt[1] = tv;
-    jt[2] = td * imu_ud;
+    jt[2] = td * p.imu_ud;
     return bad;
 }
 
@@ -2367,7 +2367,7 @@ __device__ HRes hpsi_eval(const Ctx<R, NT, BIG>& c, int mode)
         pair_stage<R>(c, jt);
         if (p.ieq) same_spin_stage(c, ss);
     } else {
-        fix_positions(c);
+        fix_positions(c, mode != MODE_GETPHI);
         bad = pair_stage64(c, mode, jt);
         if (p.ieq && mode != MODE_BCS) same_spin_stage(c, ss);
     }
