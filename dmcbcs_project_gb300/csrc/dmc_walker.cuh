@@ -600,13 +600,16 @@ __device__ __forceinline__ void pair_jastrow(const TabPoly* tpoly, const TabPoly
 // pairs inside the healing distance (grid points up to ntab0 differ from zero)
 // rather than with each pair.  A pair beyond it costs 16 FP64 instructions for
 // nothing, and one pair inside keeps its whole warp there; a listed pair's
-// distance is taken twice (16 again) and the list costs two barriers.  So: at
-// least two pairs a thread, and a healing sphere of at most a sixteenth of the
-// box, (pi/6) (ntab0 / ntab)^3.  A generation of 4096 walkers at N = 66: 1.88 ->
-// 1.73 ms; 1024 at N = 90: 1.08 -> 1.01 ms.
+// distance is taken twice (16 again), the list costs two barriers, and every
+// particle's thread walks it.  So: at least two pairs a thread, and a healing
+// distance of at most L/6.  A generation of 4096 walkers at N = 66 (L/11): 1.88 ->
+// 1.73 ms; 1024 at N = 90: 1.08 -> 1.01 ms.  getphi of 1500 walkers, us with the
+// list / without: at 0.16 L 33/33 317 / 365, 66/66 790 / 923, 100/100 1609 / 1940;
+// at 0.2 L 330 / 363, 886 / 927, 1956 / 1939; at 0.25 L 354 / 364, 1081 / 929,
+// 2673 / 1939.
 __device__ __forceinline__ bool jastrow_list(const DevParams& p, int nt)
 {
-    return p.nup * p.ndn >= 2 * nt && 2 * p.ntab0 <= p.ntab;
+    return p.nup * p.ndn >= 2 * nt && 3 * p.ntab0 <= p.ntab;
 }
 
 // ---------------------------------------------------------------------------
