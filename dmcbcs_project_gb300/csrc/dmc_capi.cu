@@ -558,7 +558,7 @@ int grid_for(dmc_ctx* c, int nw) { return std::max(1, std::min(nw, c->grid)); }
 
 int run_eval(dmc_ctx* c, int mode, int nw, const double* dx, double* psil, int* is, double* dpsi, double* d2psi,
              double* v, double* vext, double* psigl, double* dpsig, double* d2psig, double* sinv, cudaStream_t st,
-             double* dphi = nullptr, bool inv_only = false)
+             double* dphi = nullptr)
 {
     if (nw <= 0) return DMC_OK;
     KernelArgs a = base_args(c);
@@ -1795,7 +1795,7 @@ static int derbcs_device(dmc_ctx* c, int nw, const double* dx, double* dder, int
     const int prec = c->precision;
     c->precision = DMC_PREC_FP64;
     int rc = run_eval(c, MODE_BCS, nw, dx, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                      nullptr, c->ssinv.p, c->stream, nullptr, true);
+                      nullptr, c->ssinv.p, c->stream);
     c->precision = prec;
     if (rc) return rc;
     ++c->launches;
@@ -1992,7 +1992,7 @@ int dmc_sm_sweeps(dmc_ctx* c, int nsweeps, int recompute_every, int64_t* accepte
             const int prec = c->precision;
             c->precision = DMC_PREC_FP64;
             rc = run_eval(c, MODE_BCS, n, s.x.p, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                          nullptr, nullptr, c->ssinv.p, c->stream, nullptr, true);
+                          nullptr, nullptr, c->ssinv.p, c->stream);
             c->precision = prec;
             if (rc) return rc;
             ++c->launches;
@@ -2211,7 +2211,7 @@ int dmc_add_operators(dmc_ctx* c)
             const int prec = c->precision;
             c->precision = DMC_PREC_FP64;
             int rc = run_eval(c, MODE_BCS, n, s.x.p, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                              nullptr, nullptr, c->ssinv.p, c->stream, nullptr, true);
+                              nullptr, nullptr, c->ssinv.p, c->stream);
             c->precision = prec;
             if (rc) return rc;
             ++c->launches;

@@ -156,8 +156,7 @@ struct KernelArgs {
     const TabSS* tss;            // [ntab+1]
     const TabPoly* tpoly;        // FP64 path: the up-down tables by grid interval, [ntab+1]
     const PhiFix* phi;           // FP64 path: the pair function's coefficients
-    const long long* phi_oct;    // its octant tables, 2 (M+1)^3 (nullptr in the symmetric form)
-    int inv_only;                // MODE_BCS: the caller reads the inverse alone (no drift, no Laplacian)
+    const long long* phi_oct;    // its octant tables, 2 (M+1)^3 (one unused entry in the symmetric form)
     const KVecMP* kv_mp;         // mixed-precision copies of kv, tud, tss
     const TabUDmp* tud_mp;
     const TabSSmp* tss_mp;

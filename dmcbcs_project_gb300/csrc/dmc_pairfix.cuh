@@ -134,15 +134,14 @@ __device__ __forceinline__ long long sym_dot(const long long* f, const long long
     return fshl(fadd(fadd(fadd(fmh(f[0], e[0]), fmh(f[1], e[1])), fadd(fmh(f[2], e[2]), fmh(f[3], e[3]))),
                      fadd(fmh(f[4], e[4]), fmh(f[5], e[5]))), 2);
 }
-__device__ __forceinline__ void phi_sym(const PhiFix* F, const long long* tr, int P, int i, int j, bool all, PhiPair& o)
+__device__ __forceinline__ void phi_sym(const PhiFix* F, const long long* tr, int P, int i, int j, PhiPair& o)
 {
     long long c[3], s[3];
     SymTerms q;
-    pair_axes(tr, P, i, j, c, s, all);
+    pair_axes(tr, P, i, j, c, s, true);
     sym_terms(c, q);
     const long long* f = F->f;
     o.f = fadd(f[0], sym_dot(f + 1, q.e));
-    if (!all) return;
     o.l = sym_dot(f + 7, q.e);
 #pragma unroll
     for (int a = 0; a < 3; ++a) {

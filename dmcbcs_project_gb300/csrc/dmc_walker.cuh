@@ -619,16 +619,15 @@ __device__ __forceinline__ bool jastrow_list(const DevParams& p, int nt)
 // so the plane-wave sum of an entry and of its derivatives is a short
 // polynomial in the cosines of the pair's three axis angles (dmc_pairfix.cuh):
 // no orbitals, no products over k.  Writes S[i][j], the entry's gradient with
-// respect to x_i and its Laplacian to pb ([4][nup ndn]; inv_only: S alone)
-// and the Jastrow gradients' sums to acc.  jt[] gets the per-thread sums of
-// u, v and the pair Laplacian part; returns whether a pair at distance zero
-// left the derivatives not finite (inv_only, which does not form them).
+// respect to x_i and its Laplacian to pb ([4][nup ndn]) and the Jastrow
+// gradients' sums to acc.  jt[] gets the per-thread sums of u, v and the pair
+// Laplacian part.
 // Bound: the FP64 pipe, 59 of its instructions a pair (43 where the Jastrow
 // terms come from the list); the 64 high products run beside it on the integer
 // pipe.
 // ---------------------------------------------------------------------------
 template <int NT, bool BIG>
-__device__ bool pair_stage64(const Ctx<double, NT, BIG>& c, int mode, double (&jt)[3])
+__device__ void pair_stage64(const Ctx<double, NT, BIG>& c, int mode, double (&jt)[3])
 {
     const DevParams& p = c.p;
     double* sm = c.sm;
@@ -642,14 +641,13 @@ __device__ bool pair_stage64(const Ctx<double, NT, BIG>& c, int mode, double (&j
     double* du = sm + c.L.acc + 4 * p.npart;
     const int nup = p.nup, ndn = p.ndn, ldS = p.ldS, P = p.npart, pairs = nup * ndn;
     double* w0 = c.pb;
-    const bool jas = mode != MODE_BCS, det = mode != MODE_GETPHI, grad = det && !(mode == MODE_BCS && c.a.inv_only);
+    const bool jas = mode != MODE_BCS, det = mode != MODE_GETPHI;
     const double unit = p.el * 5.421010862427522e-20;    // L 2^-64: distances below are in this unit, L/2 = 2^63
     const double tscale = (double)p.ntab * 1.0842021724855044e-19;   // grid points per unit: ntab / 2^63
     // 2 / unit and 1e-14 / unit (no division here: one takes 1300 cycles of every walker's time)
     const double two_iu = 3.6893488147419103e19 * p.eli, r_min = 0.5e-14 * two_iu;
     const long long half = 0x43E0000000000000ll;         // 2^63 as a double's bits
     double tu = 0.0, tv = 0.0, td = 0.0;
-    bool bad = false;
     if (jas)
         for (int i = threadIdx.x; i < 3 * P; i += NT) du[i] = 0.0;
     __syncthreads();
@@ -672,7 +670,7 @@ __device__ bool pair_stage64(const Ctx<double, NT, BIG>& c, int mode, double (&j
                 PhiPair o;
                 if (det) {
                     if (F->fast) {
-                        phi_sym(F, tr, P, i, pj, grad, o);
+                        phi_sym(F, tr, P, i, pj, o);
                     } else {
                         phi_octant(F, c.a.phi_oct, tr, P, i, pj, o);
                         o.f = phi_value(F, o.f);
@@ -709,21 +707,17 @@ __device__ bool pair_stage64(const Ctx<double, NT, BIG>& c, int mode, double (&j
                     double f = in_b ? poly3(T->c[0], t) : 0.0;
                     if (nan) f = r;
                     S[i * ldS + j] = fma((double)o.f, F->sphi, f);
-                    if (grad) {
-                        double gr = 0.0, lp = 0.0;
-                        if (in_b) {
-                            gr = poly3(T->c[1], t) * ri;
-                            lp = poly3(T->c[2], t);
-                        }
-                        if (nan) gr = lp = r;
-                        double* w = w0 + i * ndn + j;
-                        w[0] = fma((double)o.g[0], F->sgrad, gr * d[0]);
-                        w[pairs] = fma((double)o.g[1], F->sgrad, gr * d[1]);
-                        w[2 * pairs] = fma((double)o.g[2], F->sgrad, gr * d[2]);
-                        w[3 * pairs] = fma((double)o.l, F->slap, lp);
-                    } else if (in_b && !isfinite(ri)) {
-                        bad = true;   // the drift would not be finite
+                    double gr = 0.0, lp = 0.0;
+                    if (in_b) {
+                        gr = poly3(T->c[1], t) * ri;
+                        lp = poly3(T->c[2], t);
                     }
+                    if (nan) gr = lp = r;
+                    double* w = w0 + i * ndn + j;
+                    w[0] = fma((double)o.g[0], F->sgrad, gr * d[0]);
+                    w[pairs] = fma((double)o.g[1], F->sgrad, gr * d[1]);
+                    w[2 * pairs] = fma((double)o.g[2], F->sgrad, gr * d[2]);
+                    w[3 * pairs] = fma((double)o.l, F->slap, lp);
                 }
             }
             if (list) {
@@ -810,7 +804,6 @@ __device__ bool pair_stage64(const Ctx<double, NT, BIG>& c, int mode, double (&j
     jt[0] = tu;
     jt[1] = tv;
     jt[2] = td * p.imu_ud;
-    return bad;
 }
 
 // ---------------------------------------------------------------------------
@@ -2339,7 +2332,6 @@ struct HRes {
     double psil, d2psi, v, vext, psigl, d2psig, u, d2u, logdet, d2phi;
     int is;
     bool singular;
-    bool bad;   // this thread met a pair whose drift terms (not formed: inv_only) are not finite
 };
 
 // ---------------------------------------------------------------------------
@@ -2360,7 +2352,6 @@ __device__ HRes hpsi_eval(const Ctx<R, NT, BIG>& c, int mode)
     using J = typename Prec<R>::J;
     J jt[3] = {rzero<J>(), rzero<J>(), rzero<J>()};
     double ss[3] = {0.0, 0.0, 0.0};
-    bool bad = false;
     // the pair stage also forms S (FP64) or its beta part (mixed), which
     // MODE_BCS needs too
     if constexpr (is_df<R>::value) {
@@ -2371,7 +2362,7 @@ __device__ HRes hpsi_eval(const Ctx<R, NT, BIG>& c, int mode)
         if (p.ieq) same_spin_stage(c, ss);
     } else {
         fix_positions(c, mode != MODE_GETPHI);
-        bad = pair_stage64(c, mode, jt);
+        pair_stage64(c, mode, jt);
         if (p.ieq && mode != MODE_BCS) same_spin_stage(c, ss);
     }
     double su = 0.0, sv = 0.0, sd2 = 0.0;
@@ -2411,8 +2402,7 @@ __device__ HRes hpsi_eval(const Ctx<R, NT, BIG>& c, int mode)
             __syncthreads();
         }
         ok = inverse_stage<R>(c, logdet, sgn);
-        // (the mixed path always forms the derivatives)
-        if (ok && (is_df<R>::value || !(mode == MODE_BCS && c.a.inv_only))) {
+        if (ok) {
             if constexpr (is_df<R>::value) {
                 drift_stage<R>(c);
                 beta_drift_stage<R>(c);
@@ -2517,7 +2507,6 @@ __device__ HRes hpsi_eval(const Ctx<R, NT, BIG>& c, int mode)
     }
     __syncthreads();
     h = s_h;
-    h.bad = bad;
     if (p.a2 == 0.0 || (mode != MODE_HPSI && mode != MODE_STEP)) {
         h.psigl = h.psil;
         h.d2psig = h.d2psi;

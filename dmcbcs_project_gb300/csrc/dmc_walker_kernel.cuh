@@ -337,16 +337,6 @@ walker_kernel(const __grid_constant__ DevParams p, const __grid_constant__ Kerne
         // with a barrier, after which the evaluation's shared data may change.
         auto flag_walker = [&](const HRes& hh) {
             int bad = 0;
-            if constexpr (!walker::is_df<R>::value) {
-                bad = hh.bad;
-                if (a.mode == MODE_BCS && a.inv_only && !hh.singular) {
-                    // no drift to look at: it is finite when the inverse is
-                    const R* Si = walker::at<R>(sm, L.S);
-                    const int nd = p.nd;
-                    for (int e = threadIdx.x; e < nd * nd; e += NT)
-                        if (!isfinite(Si[(e / nd) * p.ldS + e % nd])) bad = 1;
-                }
-            }
             for (int e = threadIdx.x; e < n3; e += NT) {
                 const double val = a.mode == MODE_GETPHI ? sm[L.acc + 4 * P + e] : dpsi[e];
                 if (!isfinite(val)) bad = 1;
