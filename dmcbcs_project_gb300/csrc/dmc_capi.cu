@@ -165,12 +165,13 @@ struct dmc_ctx {
     // tables
     DevBuf<unsigned char> shells;   // what the amplitudes decide, one copy per change: kv, kv_mp, phi, phi_oct
     DevPtr<KVecDev> kv;
-    DevBuf<TabUD> tud;
-    DevBuf<TabSS> tss;
     DevPtr<KVecMP> kv_mp;
-    DevBuf<TabUDmp> tud_mp;
-    DevBuf<TabSSmp> tss_mp;
-    DevBuf<TabPoly> tpoly;          // FP64 walker path: tables by grid interval
+    DevBuf<unsigned char> tables;   // the radial tables: tud, tss, tud_mp, tss_mp, tpoly
+    DevPtr<TabUD> tud;
+    DevPtr<TabSS> tss;
+    DevPtr<TabUDmp> tud_mp;
+    DevPtr<TabSSmp> tss_mp;
+    DevPtr<TabPoly> tpoly;          // FP64 walker path: tables by grid interval
     DevPtr<PhiFix> phi;             // and the pair function's fixed-point coefficients
     DevPtr<long long> phi_oct;
     bool phi_sym = false;           // in the symmetric form
@@ -478,23 +479,18 @@ int upload_tables(dmc_ctx* c)
 {
     const Setup& S = c->S;
     const int nt = S.ntab + 1;
-    std::vector<TabUD> ud(nt);
-    std::vector<TabSS> ss(nt);
+    // one buffer, one copy: FP64 tables, their mixed-precision copies in
+    // double-float, then (made on the device) the FP64 walker path's cubics
+    const size_t oss = nt * sizeof(TabUD), oudm = oss + nt * sizeof(TabSS), ossm = oudm + nt * sizeof(TabUDmp);
+    const size_t opoly = (ossm + nt * sizeof(TabSSmp) + 255) / 256 * 256;
+    std::vector<unsigned char> h(opoly);
+    TabUD* ud = reinterpret_cast<TabUD*>(h.data());
+    TabSS* ss = reinterpret_cast<TabSS*>(h.data() + oss);
+    TabUDmp* udm = reinterpret_cast<TabUDmp*>(h.data() + oudm);
+    TabSSmp* ssm = reinterpret_cast<TabSSmp*>(h.data() + ossm);
     for (int i = 0; i < nt; ++i) {
         ud[i] = TabUD{S.vtab[0][i], S.utab[0][i], S.dutab[0][i], S.d2utab[0][i], S.btab[i], S.dbtab[i], S.d2btab[i], 0.0};
         ss[i] = TabSS{S.vtab[1][i], S.utab[1][i], S.dutab[1][i], S.d2utab[1][i]};
-    }
-    CK(c->tud.alloc(nt));
-    CK(c->tss.alloc(nt));
-    CK(cudaMemcpy(c->tud.p, ud.data(), nt * sizeof(TabUD), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(c->tss.p, ss.data(), nt * sizeof(TabSS), cudaMemcpyHostToDevice));
-    CK(c->tpoly.alloc(nt));   // FP64 walker path
-    CK(launch_tab_poly(c->tud.p, c->tpoly.p, nt, nullptr));   // behind the copies, on their stream
-    // mixed-precision copies in double-float
-    std::vector<TabUDmp> udm(nt);
-    std::vector<TabSSmp> ssm(nt);
-    for (int i = 0; i < nt; ++i) {
-        std::memset(&udm[i], 0, sizeof(TabUDmp));
         udm[i].v = from_double(S.vtab[0][i]);
         udm[i].u = from_double(S.utab[0][i]);
         udm[i].du = from_double(S.dutab[0][i]);
@@ -504,10 +500,15 @@ int upload_tables(dmc_ctx* c)
         udm[i].d2b = from_double(S.d2btab[i]);
         ssm[i] = TabSSmp{(float)S.vtab[1][i], (float)S.utab[1][i], (float)S.dutab[1][i], (float)S.d2utab[1][i]};
     }
-    CK(c->tud_mp.alloc(nt));
-    CK(c->tss_mp.alloc(nt));
-    CK(cudaMemcpy(c->tud_mp.p, udm.data(), nt * sizeof(TabUDmp), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(c->tss_mp.p, ssm.data(), nt * sizeof(TabSSmp), cudaMemcpyHostToDevice));
+    CK(c->tables.alloc(opoly + nt * sizeof(TabPoly)));
+    unsigned char* d = c->tables.p;
+    c->tud.p = reinterpret_cast<TabUD*>(d);
+    c->tss.p = reinterpret_cast<TabSS*>(d + oss);
+    c->tud_mp.p = reinterpret_cast<TabUDmp*>(d + oudm);
+    c->tss_mp.p = reinterpret_cast<TabSSmp*>(d + ossm);
+    c->tpoly.p = reinterpret_cast<TabPoly*>(d + opoly);
+    CK(cudaMemcpy(d, h.data(), h.size(), cudaMemcpyHostToDevice));
+    CK(launch_tab_poly(c->tud.p, c->tpoly.p, nt, nullptr));   // behind the copy, on its stream
     if (S.nql > 0) {
         CK(c->jq.alloc(S.jq.size()));
         CK(cudaMemcpy(c->jq.p, S.jq.data(), S.jq.size() * sizeof(double), cudaMemcpyHostToDevice));
@@ -824,8 +825,7 @@ int dmc_destroy(dmc_ctx* c)
 {
     if (!c) return DMC_OK;
     if (c->stream) cudaStreamSynchronize(c->stream);
-    c->shells.release(); c->tud.release(); c->tss.release(); c->tud_mp.release();
-    c->tss_mp.release(); c->tpoly.release(); c->jumpA.release(); c->jumpC.release(); c->jq.release();
+    c->shells.release(); c->tables.release(); c->jumpA.release(); c->jumpC.release(); c->jq.release();
     c->gscratch.release(); c->st[0].release(); c->st[1].release(); c->est.release(); c->counts.release();
     c->offs.release(); c->status.release(); c->wstat.release(); c->irn1.release(); c->wtisto.release(); c->vb.release();
     c->bx.release(); c->bpsil.release(); c->bdpsi.release();

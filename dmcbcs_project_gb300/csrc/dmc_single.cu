@@ -834,7 +834,7 @@ __device__ __forceinline__ void interval_cubic(double t0, double t1, double t2, 
 }
 
 // One thread per cubic.  Made on the host and copied, they cost set_beta 0.18 ms
-// (716 -> 541 us) and the gradient after it as much again.
+// (716 -> 480 us with one copy of the tables) and the gradient after it as much.
 __global__ void tab_poly_kernel(const TabUD* __restrict__ tud, TabPoly* __restrict__ out, int nt)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x, i = t / 7, k = t - 7 * i;
