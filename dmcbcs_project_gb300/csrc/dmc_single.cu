@@ -306,19 +306,6 @@ __device__ void block_sum_n(double (&v)[N], double* red, double* outa, double* o
     __syncthreads();
 }
 
-__device__ double block_sum1(double v, double* red)
-{
-    red[threadIdx.x] = v;
-    __syncthreads();
-    for (int h = kThreads / 2; h > 0; h >>= 1) {
-        if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
-        __syncthreads();
-    }
-    const double t = red[0];
-    __syncthreads();
-    return t;
-}
-
 // Adjoint parameter gradients, one walker per CTA (FP64).
 //
 // The determinant's share of the kinetic term of E_L = -hbar d2psi + v is

@@ -162,21 +162,13 @@ struct Prec;
 template <>
 struct Prec<double> {
     using J = double;   // Jastrow / potential arithmetic
-    using Tab = TabUD;
-    using TabS = TabSS;
-    using KV = KVecDev;
-    static __device__ const Tab* tud(const KernelArgs& a) { return a.tud; }
-    static __device__ const TabS* tss(const KernelArgs& a) { return a.tss; }
-    static __device__ const KV* kv(const KernelArgs& a) { return a.kv; }
 };
 template <>
 struct Prec<df> {
     using J = df;
     using Tab = TabUDmp;
-    using TabS = TabSSmp;
     using KV = KVecMP;
     static __device__ const Tab* tud(const KernelArgs& a) { return a.tud_mp; }
-    static __device__ const TabS* tss(const KernelArgs& a) { return a.tss_mp; }
     static __device__ const KV* kv(const KernelArgs& a) { return a.kv_mp; }
 };
 
@@ -304,12 +296,6 @@ struct Ctx {
 };
 
 // two consecutive values (16-byte aligned) with one shared-memory load
-__device__ __forceinline__ void ld2(const double* p, double& a, double& b)
-{
-    const double2 v = *reinterpret_cast<const double2*>(p);
-    a = v.x;
-    b = v.y;
-}
 __device__ __forceinline__ void ld2(const df* p, df& a, df& b)
 {
     const float4 v = *reinterpret_cast<const float4*>(p);
@@ -846,20 +832,9 @@ __device__ void pair_drift64(const Ctx<double, NT, BIG>& c)
     __syncthreads();
 }
 
-// complex product in the arithmetic type
-__device__ __forceinline__ void cmul(double ar, double ai, double br, double bi, double& cr, double& ci)
-{
-    cr = ar * br - ai * bi;
-    ci = ar * bi + ai * br;
-}
 // product of two unit-modulus complex numbers (|a|, |b| <= 1 up to rounding):
 // every partial product is below 1 in magnitude, so the bounded accumulator
 // with sigma = 4 applies (6 instead of 12 FP32 instructions per term)
-__device__ __forceinline__ void cmul_unit(double ar, double ai, double br, double bi, double& cr, double& ci)
-{
-    cr = ar * br - ai * bi;
-    ci = ar * bi + ai * br;
-}
 __device__ __forceinline__ void cmul_unit(df ar, df ai, df br, df bi, df& cr, df& ci)
 {
     bacc r, i;
@@ -872,19 +847,6 @@ __device__ __forceinline__ void cmul_unit(df ar, df ai, df br, df bi, df& cr, df
     cr = bacc_value(r, 4.0f);
     ci = bacc_value(i, 4.0f);
 }
-__device__ __forceinline__ void cmul(df ar, df ai, df br, df bi, df& cr, df& ci)
-{
-    dfacc r, i;
-    acc_init(r);
-    acc_init(i);
-    acc_madd(r, ar, br);
-    acc_madd(r, -ai, bi);
-    acc_madd(i, ar, bi);
-    acc_madd(i, ai, br);
-    cr = acc_value(r);
-    ci = acc_value(i);
-}
-
 // Unpaired plane waves in S (psislaterbcs.f90:171-206): up columns ndn..,
 // down rows nup.., zero corner.
 template <class R, int NT, bool BIG>
@@ -1665,18 +1627,7 @@ __device__ __forceinline__ DriftSplit drift_split(int nup, int ndn, int ng)
 }
 
 // one accumulator per (k vector, cos|sin) of a task
-template <class R>
 struct DriftAcc {
-    typename AccOf<R>::type a[2 * kQT];
-    __device__ __forceinline__ void init(const float*) {
-#pragma unroll
-        for (int m = 0; m < 2 * kQT; ++m) acc_init(a[m]);
-    }
-    __device__ __forceinline__ void madd(int m, R x, R y) { acc_madd(a[m], x, y); }
-    __device__ __forceinline__ R value(int m, const float*) const { return acc_value(a[m]); }
-};
-template <>
-struct DriftAcc<df> {
     bacc a[2 * kQT];
     __device__ __forceinline__ void init(const float* sig) {
 #pragma unroll
@@ -1703,7 +1654,6 @@ constexpr int kTR = 2, kTS = 5, kTA = 4, kTB = 8;
 static_assert(kTA * kTB == 32, "one warp per tile");
 
 __device__ __forceinline__ float abs_hi(df v) { return fabsf(v.hi); }
-__device__ __forceinline__ float abs_hi(double v) { return (float)fabs(v); }
 
 // partial contraction of one (particle, k vector) item over the terms
 // k0, k0 + kstep, ...: G (up particle) or H (down particle) for the cos and
@@ -1721,37 +1671,21 @@ __device__ __forceinline__ void drift_dots(const Ctx<R, NT, BIG>& c, const float
     const int nk = p.nk, ld = p.ldS, ldU = p.ldU, qc = 2 * q - 2;
     const bool up = pt < p.nup;
     const int j = pt - p.nup;
-    typename AccOf<R>::type ac, as;
     bacc bc, bs;
-    float sig = 0.0f;
-    if constexpr (is_df<R>::value) {
-        sig = up ? pow2_ceil(4.0f * bound[pt]) : pow2_ceil(4.0f * fabsf(ks[4 * nk + q].hi) * 1.001f * bound[p.nd + j]);
-        bacc_init(bc, sig);
-        bacc_init(bs, sig);
-    } else {
-        acc_init(ac);
-        acc_init(as);
-    }
+    const float sig =
+        up ? pow2_ceil(4.0f * bound[pt]) : pow2_ceil(4.0f * fabsf(ks[4 * nk + q].hi) * 1.001f * bound[p.nd + j]);
+    bacc_init(bc, sig);
+    bacc_init(bs, sig);
     const int nK = up ? p.ndn : p.nup;
     for (int kk = k0; kk < nK; kk += kstep) {
         const R sv = up ? Si[kk * ld + pt] : Si[j * ld + kk];
         R bcv, bsv;
         ld2((up ? D : U) + kk * ldU + qc, bcv, bsv);
-        if constexpr (is_df<R>::value) {
-            bacc_madd(bc, bcv, sv);
-            bacc_madd(bs, bsv, sv);
-        } else {
-            acc_madd(ac, bcv, sv);
-            acc_madd(as, bsv, sv);
-        }
+        bacc_madd(bc, bcv, sv);
+        bacc_madd(bs, bsv, sv);
     }
-    if constexpr (is_df<R>::value) {
-        vc = bacc_value(bc, sig);
-        vs = bacc_value(bs, sig);
-    } else {
-        vc = acc_value(ac);
-        vs = acc_value(as);
-    }
+    vc = bacc_value(bc, sig);
+    vs = bacc_value(bs, sig);
 }
 
 // the 4 terms (3 drift components, Laplacian) of k vector q (1-based) for
@@ -1816,20 +1750,14 @@ __device__ __forceinline__ void drift_tile(const Ctx<R, NT, BIG>& c, const float
         return down ? pow2_ceil(4.0f * abs_hi(ks[4 * nk + qo[m] / 2 + 1]) * 1.001f * bound[p.nd + pi[k]])
                     : pow2_ceil(4.0f * bound[pi[k]]);
     };
-    typename AccOf<R>::type a64[kTR][kTS][2];
     bacc adf[kTR][kTS][2];
 #pragma unroll
     for (int k = 0; k < kTR; ++k)
 #pragma unroll
         for (int m = 0; m < kTS; ++m) {
-            if constexpr (is_df<R>::value) {
-                const float sg = sigma(k, m);
-                bacc_init(adf[k][m][0], sg);
-                bacc_init(adf[k][m][1], sg);
-            } else {
-                acc_init(a64[k][m][0]);
-                acc_init(a64[k][m][1]);
-            }
+            const float sg = sigma(k, m);
+            bacc_init(adf[k][m][0], sg);
+            bacc_init(adf[k][m][1], sg);
         }
     // up: G[i][q] = sum_j Si[j][i] D[j][q];  down: H[j][q] = sum_i Si[j][i] U[i][q]
     // Sinv element (particle pi[k], term kk) at s0 + kk * sstep + k * kTA * pstep
@@ -1846,13 +1774,8 @@ __device__ __forceinline__ void drift_tile(const Ctx<R, NT, BIG>& c, const float
             ld2(brow + qo[m], bc, bs);
 #pragma unroll
             for (int k = 0; k < kTR; ++k) {
-                if constexpr (is_df<R>::value) {
-                    bacc_madd(adf[k][m][0], bc, sv[k]);
-                    bacc_madd(adf[k][m][1], bs, sv[k]);
-                } else {
-                    acc_madd(a64[k][m][0], bc, sv[k]);
-                    acc_madd(a64[k][m][1], bs, sv[k]);
-                }
+                bacc_madd(adf[k][m][0], bc, sv[k]);
+                bacc_madd(adf[k][m][1], bs, sv[k]);
             }
         }
     }
@@ -1868,45 +1791,23 @@ __device__ __forceinline__ void drift_tile(const Ctx<R, NT, BIG>& c, const float
         const R* own = O + pi[k] * ldU;
 #pragma unroll
         for (int m = 0; m < kTS; ++m) {
-            R vc, vs;
-            if constexpr (is_df<R>::value) {
-                const float sg = sigma(k, m);
-                vc = bacc_value(adf[k][m][0], sg);
-                vs = bacc_value(adf[k][m][1], sg);
-            } else {
-                vc = acc_value(a64[k][m][0]);
-                vs = acc_value(a64[k][m][1]);
-            }
+            const float sk = sigma(k, m);
+            const R vc = bacc_value(adf[k][m][0], sk), vs = bacc_value(adf[k][m][1], sk);
             if (!okq[m]) continue;
             R oc, os;
             ld2(own + qo[m], oc, os);
-            R t, l;
-            if constexpr (is_df<R>::value) {
-                // |t|, |l| <= |own (cos, sin)| |(vc, vs)|: up |v_q| * colsum,
-                // down 1 * |v_q| * rowsum
-                const float vq = abs_hi(ks[4 * nk + qo[m] / 2 + 1]) * 1.001f;
-                const float sg = down ? sigma(k, m)
-                                      : pow2_ceil(4.0f * fmaxf(1.0f, vq) * bound[pi[k]]);
-                bacc at_, al_;
-                bacc_init(at_, sg);
-                bacc_init(al_, sg);
-                bacc_madd(at_, oc, vs);
-                bacc_madd(at_, -os, vc);
-                bacc_madd(al_, oc, vc);
-                bacc_madd(al_, os, vs);
-                t = bacc_value(at_, sg);
-                l = bacc_value(al_, sg);
-            } else {
-                typename AccOf<R>::type at_, al_;
-                acc_init(at_);
-                acc_init(al_);
-                acc_madd(at_, oc, vs);
-                acc_madd(at_, -os, vc);
-                acc_madd(al_, oc, vc);
-                acc_madd(al_, os, vs);
-                t = acc_value(at_);
-                l = acc_value(al_);
-            }
+            // |t|, |l| <= |own (cos, sin)| |(vc, vs)|: up |v_q| * colsum,
+            // down 1 * |v_q| * rowsum
+            const float vq = abs_hi(ks[4 * nk + qo[m] / 2 + 1]) * 1.001f;
+            const float sg = down ? sk : pow2_ceil(4.0f * fmaxf(1.0f, vq) * bound[pi[k]]);
+            bacc at_, al_;
+            bacc_init(at_, sg);
+            bacc_init(al_, sg);
+            bacc_madd(at_, oc, vs);
+            bacc_madd(at_, -os, vc);
+            bacc_madd(al_, oc, vc);
+            bacc_madd(al_, os, vs);
+            const R t = bacc_value(at_, sg), l = bacc_value(al_, sg);
             const int q1 = qo[m] / 2 + 1;
             acc_madd(sx, ks[q1], t);
             acc_madd(sy, ks[nk + q1], t);
@@ -1999,7 +1900,6 @@ __device__ bool drift_tiled(const Ctx<R, NT, BIG>& c, const float* bound)
 template <class R, int NT, bool BIG>
 __device__ void drift_stage(const Ctx<R, NT, BIG>& c)
 {
-    using KV = typename Prec<R>::KV;
     const DevParams& p = c.p;
     double* sm = c.sm;
     const R* U = c.template uat<R>(c.L.U);
@@ -2011,20 +1911,18 @@ __device__ void drift_stage(const Ctx<R, NT, BIG>& c)
     const int nq = p.nk - 1, nk = p.nk, P = p.npart, ld = p.ldS, ldU = p.ldU;
     const int ng = (nq + kQT - 1) / kQT;    // tasks per particle
     const DriftSplit sp = drift_split<NT>(p.nup, p.ndn, ng);
-    // double-float path: abs column sums (bound[i], for G) and row sums
-    // (bound[nd + j], for H) of the inverse bound the dot products
+    // abs column sums (bound[i], for G) and row sums (bound[nd + j], for H) of
+    // the inverse bound the dot products
     float* bound = reinterpret_cast<float*>(sm + c.L.colk);
-    if constexpr (is_df<R>::value) {
-        for (int t = threadIdx.x; t < 2 * p.nd; t += NT) {
-            float sacc = 0.0f;
-            if (t < p.nd)
-                for (int j = 0; j < p.nd; ++j) sacc += fabsf(Si[j * ld + t].hi);
-            else
-                for (int i = 0; i < p.nd; ++i) sacc += fabsf(Si[(t - p.nd) * ld + i].hi);
-            bound[t] = sacc * 1.001f;
-        }
-        __syncthreads();
+    for (int t = threadIdx.x; t < 2 * p.nd; t += NT) {
+        float sacc = 0.0f;
+        if (t < p.nd)
+            for (int j = 0; j < p.nd; ++j) sacc += fabsf(Si[j * ld + t].hi);
+        else
+            for (int i = 0; i < p.nd; ++i) sacc += fabsf(Si[(t - p.nd) * ld + i].hi);
+        bound[t] = sacc * 1.001f;
     }
+    __syncthreads();
     if (drift_tiled<R>(c, bound)) return;
     const int h = (int)threadIdx.x >= sp.tbeg[1] ? 1 : 0;
     const int lt = (int)threadIdx.x - sp.tbeg[h];
@@ -2047,15 +1945,13 @@ __device__ void drift_stage(const Ctx<R, NT, BIG>& c)
         }
         R vc[kQT], vs[kQT];   // G or H of each k vector
         float sig[kQT] = {};
-        DriftAcc<R> A;
+        DriftAcc A;
         const bool up = pt < p.nup;
         if (up) {
             const int i = pt;
-            if constexpr (is_df<R>::value) {
-                const float sg = pow2_ceil(4.0f * bound[i]);   // |D| <= 1
+            const float sg = pow2_ceil(4.0f * bound[i]);   // |D| <= 1
 #pragma unroll
-                for (int m = 0; m < kQT; ++m) sig[m] = sg;
-            }
+            for (int m = 0; m < kQT; ++m) sig[m] = sg;
             A.init(sig);
             const R* sc = Si + i;
             for (int j = 0; j < p.ndn; ++j) {
@@ -2071,11 +1967,9 @@ __device__ void drift_stage(const Ctx<R, NT, BIG>& c)
             }
         } else {
             const int j = pt - p.nup;
-            if constexpr (is_df<R>::value) {
 #pragma unroll
-                for (int m = 0; m < kQT; ++m)   // |U[i][q]| <= |v_q|
-                    sig[m] = pow2_ceil(4.0f * fabsf(ks[4 * nk + qv[m]].hi) * 1.001f * bound[p.nd + j]);
-            }
+            for (int m = 0; m < kQT; ++m)   // |U[i][q]| <= |v_q|
+                sig[m] = pow2_ceil(4.0f * fabsf(ks[4 * nk + qv[m]].hi) * 1.001f * bound[p.nd + j]);
             A.init(sig);
             const R* srow = Si + j * ld;
             for (int i = 0; i < p.nup; ++i) {
@@ -2220,7 +2114,6 @@ __device__ void beta_drift_stage(const Ctx<R, NT, BIG>& c)
     const DevParams& p = c.p;
     double* sm = c.sm;
     const R* xr = at<R>(sm, c.L.xr);
-    const double* x = sm + c.L.x;
     const R* Si = at<R>(sm, c.L.S);
     R* pv = c.template uat<R>(c.L.R);
     const R* pb = reinterpret_cast<const R*>(c.pb);
