@@ -217,8 +217,8 @@ __device__ __forceinline__ long long phi_value(const PhiFix* F, long long f) { r
 
 // ---- FP64 ------------------------------------------------------------------
 
-// r = sqrt(r2) and 1/r for r2 in [1, 2^128): a single-precision reciprocal
-// square root (converted by shifting exponents, on the integer pipe) refined
+// r = sqrt(r2) and 1/r for r2 in [2^-126, 2^128), FP32's normal numbers: a
+// single-precision reciprocal square root (converted by shifting exponents, on the integer pipe) refined
 // by one step of Householder's third-order iteration, y <- y (1 + e/2 + 3 e^2/8)
 // with e = 1 - r2 y^2, then one Newton correction of r = r2 y.  Eight FP64
 // instructions where sqrt and a division take fourteen.

@@ -1082,9 +1082,12 @@ template <int PW>
 __device__ __forceinline__ void bar2_sync() { asm volatile("bar.sync 2, %0;" ::"n"(32 * PW) : "memory"); }
 
 // 1 / p of a pivot: a single-precision reciprocal (converted by shifting
-// exponents, on the integer pipe), then one step of the third-order iteration
-// y <- y + y (e + e^2), e = 1 - p y; three FP64 instructions.  Outside FP32's
-// range the division.
+// exponents, on the integer pipe), then one step of the hyperpower iteration of
+// order three, y <- y (1 + e + e^2) with e = 1 - p y (the geometric series of
+// 1/p = y / (1 - e) cut after e^2; e is below 2^-21, so that is 2^-63 off before
+// rounding); three FP64 instructions.  Outside 2^-111 .. 2^109, where the
+// single-precision reciprocal would not be a normal number or nearly so, the
+// division.
 __device__ __forceinline__ double pivot_rcp(double p)
 {
     const unsigned hi = (unsigned)__double2hiint(p), lo = (unsigned)__double2loint(p), mag = hi & 0x7fffffffu;
