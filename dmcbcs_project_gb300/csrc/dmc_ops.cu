@@ -101,7 +101,10 @@ __global__ void __launch_bounds__(kThreads) ops_walker_kernel(const __grid_const
                 double r = unit * fix_dist(walker::fsub(xf[3 * i], xf[3 * j]), walker::fsub(xf[3 * i + 1], xf[3 * j + 1]),
                                            walker::fsub(xf[3 * i + 2], xf[3 * j + 2]));
                 double pos = o.scaleg * r;
-                const float at = (float)pos;   // FP32 looks first: 2^-22 of the range
+                // FP32 looks first, 2^-22 of the range, at pos cut to 24 bits by shifting (an FP64
+                // conversion was 3 % of g(r); below 2^-126 the value is none, but the bin is 0 in either form)
+                const unsigned hi = (unsigned)__double2hiint(pos), lo = (unsigned)__double2loint(pos);
+                const float at = __uint_as_float(((hi - 0x38000000u) << 3) | (lo >> 29));
                 if (wide || fabsf(at - rintf(at)) <= 2.3841858e-7f * o.ntabg) {
                     r = edge_dist(r, pos, xw + 3 * i, xw + 3 * j, o.el, o.ntabg, wide);
                     pos = o.scaleg * r;
