@@ -7,13 +7,16 @@
 // One CTA of 256 threads owns one walker at a time (persistent grid over
 // the population).  The whole wavefunction evaluation of a walker stays on
 // chip: positions, k-vector records, the nd x nd pair matrix and its
-// inverse, the pair-orbital matrices U (up x K) and D (down x K), the beta
-// pair terms and the reduction scratch.  Global memory is touched only to
+// inverse, the pair-orbital matrices U (up x K) and D (down x K) and the beta
+// pair terms (mixed) or the pairs' gradients and Laplacians (FP64), and the
+// reduction scratch.  Global memory is touched only to
 // read the walker, the tables (L2-resident) and to write the results.
 //
 // The reference computes the determinant drift and Laplacian from five
 // GEMMs (psislaterbcs.f90:278-281) and the contractions with the inverse
-// (:211-223).  Here the same quantities come from three products:
+// (:211-223).  The FP64 path takes an entry and its derivatives from
+// polynomials in the pair's axis cosines (dmc_pairfix.cuh) and contracts those;
+// on the mixed path the same quantities come from three products:
 //   S = U D^T (+ beta),  G = D^T-rows . S^-1 (up drift/Laplacian),
 //   H = S^-1 . U (down drift/Laplacian),
 // using that the orbital derivatives are the orbitals of the partner column
